@@ -24,6 +24,7 @@ struct KGeom {
     int fwd_chunk;   // tiled forward projector: subset angles per CTA (1..128)
     int ms_chunk = 0;  // slice-interleaved forward projector: subset angles per CTA (1..128);
                        // 0 = off (groups of eight slices then use the per-slice kernel)
+    int fwd_direct = 1;  // small problems take the kernels of xct_direct.cu (0: a tile chosen by hand)
 };
 
 // One slice of a batched launch (device-side descriptor).
@@ -143,6 +144,14 @@ int launch_fwd_finalize(const KGeom &g, const float *meas, float *out, double *a
 // Tiled OSEM2 backprojection + update, in place (same contract as the plain one).
 int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const float *ratio, int dN, int sub,
                            cudaStream_t st);
+// The small-problem kernels (xct_direct.cu): the contracts of launch_fwd_tiled (without an
+// accumulator) and launch_bp_update_tiled, and whether a launch of dN slices takes them.
+bool fwd_is_direct(const KGeom &g, int dN, int nrows);
+bool bp_is_direct(const KGeom &g, int dN);
+int launch_fwd_direct(const KGeom &g, const float2 *trig, const float *img, const float *meas, float *out, int dN, int sub,
+                      int step, int nrows, cudaStream_t st);
+int launch_bp_update_direct(const KGeom &g, const float2 *trig, float *img, const float *ratio, int dN, int sub,
+                            cudaStream_t st);
 // Batched launches (xct_tiled.cu): work units of one slice, persistent grid sizes, and one
 // subset step (forward, finalize, backprojection) over all slices; bases is [3][n+1]
 // prefix sums of the units of each kernel, queues 3 zeroed counters.

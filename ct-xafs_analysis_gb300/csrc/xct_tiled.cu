@@ -1879,6 +1879,7 @@ int launch_fwd_finalize(const KGeom &g, const float *meas, float *out, double *a
 int launch_fwd_tiled(const KGeom &g, const float2 *trig, const float *img, const float *meas, float *out,
                      double *acc, int dN, int sub, int step, int nrows, cudaStream_t st)
 {
+    if (fwd_is_direct(g, dN, nrows)) return launch_fwd_direct(g, trig, img, meas, out, dN, sub, step, nrows, st);
     int rc = launch_fwd_tiled_main(g, trig, img, acc, dN, sub, step, nrows, st);
     if (rc) return rc;
     return launch_fwd_finalize(g, meas, out, acc, dN, sub, step, nrows, st);
@@ -1986,6 +1987,7 @@ int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const
                            cudaStream_t st)
 {
     if (dN <= 0) return XCT_OK;
+    if (bp_is_direct(g, dN)) return launch_bp_update_direct(g, trig, img, ratio, dN, sub, st);
     const int nang = (g.pa - sub + g.ss - 1) / g.ss;  // OSEM2's angle loop (OSEM.cl:93)
     // with the slice-interleaved kernels on, whole groups of eight slices go through the
     // eight-slice backprojector, pairs of the rest through its two-slice form, and a last

@@ -209,6 +209,7 @@ int xct_plan_set_tuning(xct_plan *p, int fwd_tile, int ang_chunk)
         return xct_fail(XCT_E_INVALID, "ang_chunk must be in 1..128");
     p->kg.fwd_T = fwd_tile;
     p->kg.fwd_chunk = ang_chunk;
+    p->kg.fwd_direct = 0;  // tiles chosen by hand are used whatever the size
     return XCT_OK;
 }
 
