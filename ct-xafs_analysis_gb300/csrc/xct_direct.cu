@@ -13,6 +13,7 @@
 // overlap by programmatic stream serialization) against 37.4 us with the tiled kernels' three.
 #include "xct_device.cuh"
 #include "xct_launch.cuh"
+#include "xct_ray.cuh"
 
 namespace {
 
@@ -28,30 +29,6 @@ constexpr int kDirWarps = 8;                // warps sharing the samples of the 
 // of 512^2 x 36 angles 4 against 14 us a launch, 1024^2 x 72 angles 46 against 31.
 constexpr long long kDirectTaps = 4500000;  // image texels x subset angles x slices
 constexpr long long kDirectPixels = 600000; // image pixels x slices
-
-__device__ __forceinline__ float ray_coord(int Y, float hd, float sl, float a) { return fmaf((float)Y - hd, sl, a); }
-
-// First Y in [0, D] with the monotone predicate (sl > 0: u >= b; sl < 0: u < b), u the sample's
-// coordinate; the forward tile kernel's search (an estimate checked by exact evaluations, else bisection).
-__device__ __forceinline__ int first_true(float b, float a, float sl, float hd, int D)
-{
-    const bool up = sl > 0.0f;
-    float e = fmaf(b - a, 1.0f / sl, hd);
-    e = fminf(fmaxf(e, -1.0f), (float)D + 1.0f);
-    int Y = min(max((int)ceilf(e), 0), D);
-    const float ul = ray_coord(Y - 1, hd, sl, a), uh = ray_coord(Y, hd, sl, a);
-    const bool pl = Y > 0 && (up ? ul >= b : ul < b);
-    const bool ph = Y >= D || (up ? uh >= b : uh < b);
-    if (!pl && ph) return Y;
-    int lo = 0, hi = D;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const float u = ray_coord(mid, hd, sl, a);
-        if (up ? u >= b : u < b) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo;
-}
 
 // grid: (ceil(px / 8), nrows, dN), kDirWarps warps.  meas != nullptr: OSEM1 ratio; else raw ray sums.
 __global__ void __launch_bounds__(kDirWarps * 32) fwd_direct_kernel(const float *img, const float *meas, float *out,
@@ -76,7 +53,7 @@ __global__ void __launch_bounds__(kDirWarps * 32) fwd_direct_kernel(const float 
     if (X < g.px) {
         const float a = bound_x ? ax : ay, sl = bound_x ? s : c;
         const float hi = bound_x ? (float)g.nx : (float)g.ny;
-        if (sl != 0.0f) v = first_true(((sl > 0.0f) != upper) ? -1.0f : hi, a, sl, g.hd, D);
+        if (sl != 0.0f) v = first_true(((sl > 0.0f) != upper) ? -1.0f : hi, a, sl, 1.0f / sl, g.hd, D);
         else v = upper ? ((a >= -1.0f && a < hi) ? D : 0) : 0;
     }
     const int w = __shfl_xor_sync(0xffffffffu, v, 2);

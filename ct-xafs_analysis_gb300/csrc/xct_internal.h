@@ -22,8 +22,9 @@ struct KGeom {
     int fetch;       // XCT_FETCH_*
     int fwd_T;       // tiled forward projector: tile side (44, 60, 76, 92)
     int fwd_chunk;   // tiled forward projector: subset angles per CTA (1..128)
-    int ms_chunk = 0;  // slice-interleaved forward projector: subset angles per CTA (1..128);
-                       // 0 = off (groups of eight slices then use the per-slice kernel)
+    int ms_chunk = 0;  // slice-interleaved kernels: most subset angles per forward CTA (1..128);
+                       // 0 = off (the backprojectors and the adjoint then work slice by slice)
+    int fwd_group = 1;   // forward projection of several slices per CTA (0: one, by hand)
     int fwd_direct = 1;  // small problems take the kernels of xct_direct.cu (0: a tile chosen by hand)
 };
 
@@ -133,12 +134,10 @@ int launch_fwd_tiled(const KGeom &g, const float2 *trig, const float *img, const
 // The two halves of launch_fwd_tiled (timed separately by xct_osem_profile).
 int launch_fwd_tiled_main(const KGeom &g, const float2 *trig, const float *img, double *acc, int dN, int sub, int step,
                           int nrows, cudaStream_t st);
-// The slice-interleaved forward projector alone over groups x 8 slices (part of
-// launch_fwd_tiled_main when g.ms_chunk > 0); its slice group size and tile side.
-int launch_fwd_ms(const KGeom &g, const float2 *trig, const float *img, double *acc, int groups, int sub, int step,
-                  int nrows, int chunk, cudaStream_t st);
+// Modelled time of a forward launch (see its definition), for the choice of tiles and chunks.
+double xct_fwd_cost(int nx, int ny, int S, int T, int nrows, int chunk, int groups, int sms);
+// Slices per group of the slice-interleaved backprojectors.
 int fwd_ms_slices();
-int fwd_ms_tile();
 int launch_fwd_finalize(const KGeom &g, const float *meas, float *out, double *acc, int dN, int sub, int step,
                         int nrows, cudaStream_t st);
 // Tiled OSEM2 backprojection + update, in place (same contract as the plain one).

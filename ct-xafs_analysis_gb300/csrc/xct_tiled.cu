@@ -2,18 +2,18 @@
 //
 // Forward projector (OSEM1 / projection, OSEM.cl:38-68, reconstShare.cl:213-241),
 // tile-stationary:
-//   * one CTA owns an image tile: the samples whose base texel (floor(x), floor(y)) lies in
-//     [x0, x0+T) x [y0, y0+T), with x0 = -1 + bx*T (base texel -1 still reaches texel 0).
-//     It stages the tile ONCE per subset in shared memory as (t, t[x+1] - t) pairs, so
+//   * one CTA owns an image tile of up to five slices: the samples whose base texel (floor(x),
+//     floor(y)) lies in [x0, x0+T) x [y0, y0+T), with x0 = -1 + bx*T (base texel -1 still reaches
+//     texel 0).  It stages the tile ONCE per subset in shared memory as (t, t[x+1] - t) pairs, so
 //     the x-lerp of a bilinear sample is one FMA and its 2x2 footprint is two 64-bit
 //     loads, and serves every angle of its angle chunk from there;
 //   * a warp takes one angle and 8 consecutive rays, 4 lanes per ray; the exact interval of
 //     sample indices Y whose base texel lies in the tile (the coordinates are monotone in Y)
 //     comes from four boundary searches, one per lane of the ray's group; the 4 lanes then
-//     take every 4th sample of the interval, with packed f32x2 coordinate/floor/fraction
-//     arithmetic, and their partial sums are combined with two shuffles;
+//     take every 4th sample, all rays in step from the warp's first sample on, with packed f32x2
+//     coordinate/floor/fraction arithmetic over two samples;
 //   * per-tile partial ray sums go into a double-precision accumulator with one atomic per
-//     ray and tile.
+//     ray, slice and tile.
 // A finalize kernel turns the accumulator into the OSEM1 ratio (or the raw projection)
 // and clears it for the next subset.
 //
@@ -29,6 +29,7 @@
 //   * the multiplicative update is fused.
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 
@@ -36,34 +37,17 @@
 #include "xct_check.cuh"
 #include "xct_device.cuh"
 #include "xct_f32x2.cuh"
+#include "xct_launch.cuh"
+#include "xct_ray.cuh"
 
 namespace {
 
 constexpr int kThreads = 256;
-// forward projector: 12 warps per CTA so that 3 CTAs (3 x 69 KB of shared memory) give 36
-// resident warps per SM to hide the shared-memory load latency
-constexpr int kFwdThreads = 384;
-constexpr int kFwdWarps = kFwdThreads / 32;
 constexpr int kAngChunk = 128;  // most subset angles one forward-projector CTA serves
 
 // A warp works on 8 consecutive rays of one angle with 4 lanes per ray, the 4 lanes taking
-// every 4th sample (lane k: samples ya+k, ya+k+4, ...).  A half-warp then reads a compact
-// 4x4 patch of footprints, and with an element pitch of 4 (mod 8) most such patches fall in
-// distinct 64-bit bank pairs; 8 neighbouring rays also have similar lengths inside a tile,
-// so few lanes idle.  (A CPU model of the access pattern: 0.232 shared wavefronts and 90 %
-// active lanes per sample, against 0.293 and 73 % for one lane per ray with an odd pitch.)
-// Tile side T (owned base texels per side) is a template parameter chosen per plan by the
-// autotuner from {44, 60, 76, 92}; every candidate has an element pitch of T = 4 (mod 8).
-template <int T>
-struct FwdTile {
-    static_assert(T % 8 == 4, "tile pitch must be 4 (mod 8)");
-    static constexpr int P = T;         // element pitch
-    static constexpr int Rows = T + 1;  // a base row r reads element rows r and r+1
-    static constexpr size_t Smem = (size_t)P * Rows * sizeof(float2) + kAngChunk * sizeof(float2);
-    // CTAs per SM: 4 (48 warps, <= 40 registers, no spills) where four tiles fit in the
-    // 227 KB of shared memory (T <= 76), else 3 (56 registers)
-    static constexpr int MinBlocks = Smem * 4 <= 227u * 1024u ? 4 : 3;
-};
+// every 4th sample (lane k: samples ya+k, ya+k+4, ...); 8 neighbouring rays have similar
+// lengths inside a tile, so few lanes idle.
 constexpr int kLanesPerRay = 4;
 constexpr int kRaysPerWarp = 32 / kLanesPerRay;
 
@@ -81,52 +65,9 @@ constexpr int kBpChunk = 64;           // angles per staging pass of the backpro
 
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 
-// ---------------------------------------------------------------------- ray intervals
-__device__ __forceinline__ float ray_coord(int Y, float hd, float sl, float a)
-{
-    return fmaf((float)Y - hd, sl, a);
-}
-
-// First Y in [0, D] where the monotone predicate P holds (D if none), with the sentinels
-// P(-1) = false, P(D) = true:  sl > 0: P(Y) = u(Y) >= b;  sl < 0: P(Y) = u(Y) < b,
-// u(Y) = fma(Y - hd, sl, a).  The estimate from the real crossing point is checked with
-// two exact evaluations; a binary search settles the rare cases it misses.
-__device__ __noinline__ int first_true_search(float b, float a, float sl, float hd, int D)
-{
-    const bool up = sl > 0.0f;
-    int lo = 0, hi = D;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const float u = ray_coord(mid, hd, sl, a);
-        if (up ? (u >= b) : (u < b)) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ int first_true(float b, float a, float sl, float inv_sl, float hd, int D)
-{
-    const bool up = sl > 0.0f;
-    float e = fmaf(b - a, inv_sl, hd);
-    e = fminf(fmaxf(e, -1.0f), (float)D + 1.0f);  // also maps +-inf; NaN -> -1
-    int Y = (int)ceilf(e);
-    Y = min(max(Y, 0), D);
-    const float ul = ray_coord(Y - 1, hd, sl, a);
-    const float uh = ray_coord(Y, hd, sl, a);
-    const bool pl = (Y > 0) && (up ? (ul >= b) : (ul < b));
-    const bool ph = (Y >= D) || (up ? (uh >= b) : (uh < b));
-    if (!pl && ph) return Y;
-    return first_true_search(b, a, sl, hd, D);
-}
-
 __device__ __forceinline__ void lds_f2(unsigned addr, float &a, float &b)
 {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(addr));
-}
-template <int P>
-__device__ __forceinline__ void lds_f2_next_row(unsigned addr, float &a, float &b)
-{
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2+%3];" : "=f"(a), "=f"(b) : "r"(addr), "n"(P * 8));
 }
 __device__ __forceinline__ float lds_f1(unsigned addr)
 {
@@ -136,434 +77,317 @@ __device__ __forceinline__ float lds_f1(unsigned addr)
 }
 
 // ----------------------------------------------------------------- forward projector
-// One bilinear sample at Yc (both halves of yc2): coordinates (fma(Yc,s,ax), fma(Yc,c,ay)),
-// floor as a round-down add of 1.5*2^23 (the low mantissa bits), fraction = coordinate -
-// floor, the footprint as two 64-bit loads of (t, t[x+1] - t), three FMA lerps.  [alo, ahi]:
-// the byte addresses the first load may take (checked in the bounds-checked build only).
-template <int P>
-__device__ __forceinline__ float fwd_sample(f2x yc2, f2x sc, f2x axy, f2x MM, unsigned base2, unsigned alo,
-                                            unsigned ahi)
-{
-    const f2x xy = f2_fma(yc2, sc, axy);
-    const f2x tb = f2_add_rd(xy, MM);
-    const f2x fr = f2_sub(xy, f2_sub(tb, MM));
-    int ixb, iyb;
-    f2_unpack_bits(tb, ixb, iyb);
-    float fx, fy;
-    f2_unpack(fr, fx, fy);
-    const unsigned addr = (unsigned)iyb * (unsigned)(P * 8) + (unsigned)ixb * 8u + base2;
-    if (!XCT_IN(addr, alo, ahi, XCT_SITE_FWD_TAP)) return 0.0f;
-    float t00, d0, t01, d1;
-    lds_f2(addr, t00, d0);
-    lds_f2_next_row<P>(addr, t01, d1);
-    const float r0 = fmaf(fx, d0, t00);
-    const float r1 = fmaf(fx, d1, t01);
-    return fmaf(fy, r1 - r0, r0);
-}
-
-// The work of one CTA: tile (bx, by) of one slice (image im, accumulator acc [nrows][px])
-// for the subset angles k0 .. k0+chunk-1 (chunk <= kAngChunk).  Starts and ends with all
-// threads in step.
-template <int T>
-__device__ __forceinline__ void fwd_tile(const KGeom &g, const float *__restrict__ im, double *__restrict__ acc,
-                                         const float2 *__restrict__ trig, int sub, int step, int nrows, int bx,
-                                         int by, int k0, int chunk, unsigned char *smem_raw)
-{
-    constexpr int kFwdT = T, kFwdP = FwdTile<T>::P, kFwdRows = FwdTile<T>::Rows;
-    float2 *tile = reinterpret_cast<float2 *>(smem_raw);
-    float2 *scs = reinterpret_cast<float2 *>(smem_raw + (size_t)kFwdP * kFwdRows * sizeof(float2));
-    const int kn = min(chunk, nrows - k0);
-    if (kn <= 0) return;
-    const int x0 = -1 + bx * kFwdT, y0 = -1 + by * kFwdT;
-
-    // element (c, r) = (t(x0+c, y0+r), t(x0+c+1, y0+r) - t(x0+c, y0+r)), zero border
-    for (int i = threadIdx.x; i < kFwdT * kFwdRows; i += kFwdThreads) {
-        const int r = i / kFwdT, c = i - r * kFwdT;
-        const int gx = x0 + c, gy = y0 + r;
-        float t0 = 0.0f, t1 = 0.0f;
-        if ((unsigned)gy < (unsigned)g.ny) {
-            const float *row = im + (size_t)gy * g.nx;
-            if ((unsigned)gx < (unsigned)g.nx) t0 = __ldg(row + gx);
-            if ((unsigned)(gx + 1) < (unsigned)g.nx) t1 = __ldg(row + gx + 1);
-        }
-        tile[r * kFwdP + c] = make_float2(t0, t1 - t0);
-    }
-    for (int k = threadIdx.x; k < kn; k += kFwdThreads) scs[k] = trig[sub + (k0 + k) * step];
-    __syncthreads();
-
-    // owned base-texel ranges (the union over tiles is [-1, n-1])
-    const float xlo = (float)x0, xhi = (float)min(x0 + kFwdT, g.nx);
-    const float ylo = (float)y0, yhi = (float)min(y0 + kFwdT, g.ny);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int D = g.depth;
-    // shared address of element (col, row) from the floor bits (col + BIAS + x0, ...):
-    // base2 + iy_bits * 8P + ix_bits * 8, with the biases folded into base2 (mod 2^32)
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(tile);
-    const unsigned bias = (unsigned)XCT_FLOOR_BIAS;
-    const unsigned base2 = sbase - (((bias + (unsigned)y0) * (unsigned)kFwdP + bias + (unsigned)x0) * 8u);
-    const f2x MM = f2_pack(kMagic, kMagic);
-    const f2x step2 = f2_pack((float)kLanesPerRay, (float)kLanesPerRay);
-    // a footprint's first element may be any but the last row's (the second load reads the row below)
-    const unsigned alo = sbase, ahi = sbase + (unsigned)((kFwdP * (kFwdRows - 1) - 1) * 8);
-    const int ray = lane / kLanesPerRay;  // ray within the warp's 8
-    const int ph = lane % kLanesPerRay;   // sample phase of this lane
-    const int grp = lane & ~(kLanesPerRay - 1);
-    // lane phase 0/1 bound the x coordinate, 2/3 the y coordinate (lower / upper Y limit)
-    const bool bound_x = ph < 2;
-    const bool upper = (ph & 1) != 0;
-
-    for (int k = warp; k < kn; k += kFwdWarps) {
-        const float c = scs[k].x, s = scs[k].y;
-        const float inv_s = 1.0f / s, inv_c = 1.0f / c;
-        // rays that can reach the tile: project the (expanded) tile corners on the
-        // detector axis, X = (x - nx/2) c - (y - ny/2) s + cx
-        float pmin = 3.0e38f, pmax = -3.0e38f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float px_ = (q & 1) ? xhi + 2.0f : xlo - 2.0f;
-            const float py_ = (q & 2) ? yhi + 2.0f : ylo - 2.0f;
-            const float p = (px_ - g.hx) * c - (py_ - g.hy) * s + g.cx;
-            pmin = fminf(pmin, p);
-            pmax = fmaxf(pmax, p);
-        }
-        const int Xlo = max(0, (int)floorf(pmin) - 1);
-        const int Xhi = min(g.px - 1, (int)ceilf(pmax) + 1);
-        const f2x sc = f2_pack(s, c);
-        for (int base = Xlo; base <= Xhi; base += kRaysPerWarp) {
-            const int X = base + ray;
-            const bool live = X <= Xhi;
-            const float Xc = (float)X - g.cx;
-            const float ax = fmaf(Xc, c, g.hx);
-            const float ay = fmaf(Xc, -s, g.hy);
-            // the four interval limits of this ray, one per lane of its group: the lower (even
-            // phase) or upper (odd phase) Y limit from the x (phase 0/1) or y (2/3) coordinate
-            int v = 0;
-            if (live) {
-                const float a = bound_x ? ax : ay, sl = bound_x ? s : c, isl = bound_x ? inv_s : inv_c;
-                const float lo = bound_x ? xlo : ylo, hi = bound_x ? xhi : yhi;
-                if (sl != 0.0f) {
-                    // sl > 0: [first(u >= lo), first(u >= hi)); sl < 0: [first(u < hi), first(u < lo))
-                    const float b = ((sl > 0.0f) != upper) ? lo : hi;
-                    v = first_true(b, a, sl, isl, g.hd, D);
-                } else {  // constant coordinate: all samples or none
-                    v = upper ? ((a >= lo && a < hi) ? D : 0) : 0;
-                }
-            }
-            const int v0 = __shfl_sync(0xffffffffu, v, grp + 0), v1 = __shfl_sync(0xffffffffu, v, grp + 1);
-            const int v2 = __shfl_sync(0xffffffffu, v, grp + 2), v3 = __shfl_sync(0xffffffffu, v, grp + 3);
-            const int ya = max(v0, v2), yb = min(v1, v3);
-            const int n = yb - ya > ph ? (yb - ya - ph + kLanesPerRay - 1) / kLanesPerRay : 0;
-            const float yc0 = (float)(ya + ph) - g.hd;
-            f2x yc2 = f2_pack(yc0, yc0);
-            const f2x axy = f2_pack(ax, ay);
-            // two samples per iteration into two accumulators (independent load/FMA chains)
-            float sum = 0.0f, sum_b = 0.0f;
-            int i = 0;
-            for (; i + 1 < n; i += 2) {
-                const f2x yb2 = f2_add(yc2, step2);
-                sum += fwd_sample<kFwdP>(yc2, sc, axy, MM, base2, alo, ahi);
-                sum_b += fwd_sample<kFwdP>(yb2, sc, axy, MM, base2, alo, ahi);
-                yc2 = f2_add(yb2, step2);
-            }
-            if (i < n) sum += fwd_sample<kFwdP>(yc2, sc, axy, MM, base2, alo, ahi);
-            sum += sum_b;
-            // the ray's partial sum over this tile: the 4 phases, then one atomic
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            if (ph == 0 && live && yb > ya &&
-                XCT_IN((long long)(k0 + k) * g.px + X, 0, (long long)nrows * g.px - 1, XCT_SITE_FWD_ACC))
-                atomicAdd(acc + (size_t)(k0 + k) * g.px + X, (double)sum);
-        }
-    }
-}
-
-// grid: (ntx*nty tiles, angle chunks, dN).  acc: [dN][nrows][px] doubles.
-template <int T>
-__global__ void __launch_bounds__(kFwdThreads, FwdTile<T>::MinBlocks) fwd_tiled_kernel(const float *__restrict__ img,
-                                                                   double *__restrict__ acc,
-                                                                   const float2 *__restrict__ trig, KGeom g, int sub,
-                                                                   int step, int nrows, int ntx)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int z = blockIdx.z;
-    fwd_tile<T>(g, img + (size_t)z * g.nx * g.ny, acc + (size_t)z * nrows * g.px, trig, sub, step, nrows,
-                (int)blockIdx.x % ntx, (int)blockIdx.x / ntx, (int)blockIdx.y * g.fwd_chunk, g.fwd_chunk, smem_raw);
-}
-
-// ------------------------------------------- forward projector, eight slices per tile
-// For a batch of slices of one geometry (the reference's dN image-array layers, OSEM1 over
-// global size (px, pa/ss, dN)), eight slices share every sample position.  A CTA of 28 warps
-// (the most whose registers fit one SM: 71 a thread; the tile fills shared memory, one CTA
-// per SM; 28 warps hide the shared-memory latency better than 16: 2.08 against 2.24 ms per
-// launch of 8 slices x 100 angles of 2048^2) owns a T x T tile of base texels of eight
-// slices; shared memory holds, per base texel, one
-// 16-byte element per slice -- (t00, t10 - t00, t01 - t00, (t11 - t01) - (t10 - t00)), the
-// whole 2x2 footprint -- and a texel's eight elements are one 128-byte record.  A warp takes
-// eight rays of one angle, a quarter-warp (eight lanes) per pair of consecutive rays: lanes
-// 0-3 of the quarter walk the first ray's samples in the tile, lanes 4-7 the second's, lane j
-// of a ray taking its samples j, j + 4, ...  For each sample a lane finds the coordinates,
-// floor and record once and then reads the eight slices' elements starting at slot p (its
-// lane in the quarter) and wrapping, so at every load the quarter's eight lanes read eight
-// different 16-byte bank groups: no load has a bank conflict whatever the geometry, the
-// coordinate work is spread over eight slice-samples, and a quarter whose rays are done
-// costs no shared-memory wavefronts.  The bilinear value of one slice,
-// t00 + fy dy + fx (dx + fy dxy), is two packed-pair FMAs: (t00, dx) + fy (dy, dxy), then
-// added into the slot's pair of partial sums with weights (1, fx).  Slot r of lane p
-// accumulates slice (r + p) mod 8; eight shuffles give lane p the quarter's totals for slice
-// p of both rays, which it adds to the double accumulator with one atomic per ray.  Work
-// items (angle, eight rays) are taken from a shared counter, so warps finish within one item
-// of each other.
-constexpr int kMsSlices = 8;
-constexpr int kMsThreads = 896;
-constexpr int kMsRays = 2 * 32 / kMsSlices;  // rays per warp (a pair per quarter-warp)
-constexpr int kMsLanesPerRay = kMsSlices / 2;
-constexpr int kMsTile = 42;              // base texels per tile side: 42^2 x 128 B = 221 KB
-constexpr int kMsStageRows = 6;          // element rows per staging strip
-
-template <int T>
-struct FwdMsTile {
-    static constexpr size_t TileBytes = (size_t)T * T * kMsSlices * sizeof(float4);
-    // per chunk angle: (c, s), (1/c, 1/s), first and last ray, ray-group prefix; then the
-    // group total and the work counter
-    static constexpr size_t Smem = TileBytes + (size_t)kAngChunk * (2 * sizeof(float2) + 3 * sizeof(int)) + 16;
-    static_assert(Smem <= 227u * 1024u, "eight-slice tile exceeds shared memory");
+// A CTA owns the samples whose base texel lies in a T x T tile of S slices (the slices of one call
+// share their geometry, so a sample's coordinates, addresses and weights serve all S).  Shared
+// memory holds one plane per slice of the elements (t(x), t(x+1) - t(x)), so a sample takes, per
+// slice, two 64-bit loads (its two rows), two x-lerps and two weighted sums.
+//
+// Bound: the shared-memory data path, 16 B per sample and slice.  A 64-bit load is served a
+// half-warp (4 rays x 4 samples here) at a time; with the rows loaded in image order the rotated
+// lattice of a half-warp's samples collides in the banks whatever the pitch (a CPU model: 0.212
+// wavefronts per sample at best, 0.125 ideal).  Loading the EVEN row of every sample's two first
+// and the odd row second -- lanes whose base row is odd start with the row below -- halves the
+// rows one load touches, and neighbouring samples then mostly share their elements: 0.127 with a
+// pitch of 3 or 5 (mod 8).  The weight of the odd row is the distance |y - (even row)|.
+//
+// S up to 5 and T: two CTAs of 512 threads per SM fill shared memory (one stages while the other
+// computes); with S = 1 the tile side is the plan's choice (44, 60, 76 or 92).
+template <int S, int T>
+struct FwdTile {
+    // element pitch: the smallest of 3 or 5 (mod 8) that holds a row
+    static constexpr int P = T % 8 <= 3 ? T - T % 8 + 3 : T % 8 <= 5 ? T - T % 8 + 5 : T - T % 8 + 11;
+    static constexpr int Rows = T + 1;  // a base row r reads element rows r and r+1
+    static constexpr unsigned Plane = (unsigned)(P * Rows * 8);
+    // per chunk angle: (c, s, 1/c, 1/s) and (first ray, last ray, first item, end item)
+    static constexpr size_t TableOff = ((size_t)S * Plane + 15) & ~(size_t)15;
+    static constexpr size_t Smem = TableOff + (size_t)kAngChunk * 32;
+    // S = 1: 12 warps per CTA, 4 CTAs per SM where four tiles fit (T <= 76), else 3
+    static constexpr int Threads = S == 1 ? 384 : 512;
+    static constexpr int MinBlocks = S > 1 ? 2 : (Smem + 1024) * 4 <= 228u * 1024u ? 4 : 3;
+    static_assert((P % 8 == 3 || P % 8 == 5) && P >= T, "tile pitch");
+    static_assert((Smem + 1024) * MinBlocks <= 228u * 1024u, "tiles exceed shared memory");
+};
+// tile side of the grouped forms (S = 2 .. 5): the largest that two CTAs per SM hold
+template <int S>
+struct FwdGroup {
+    static constexpr int T = S == 2 ? 83 : S == 3 ? 67 : S == 4 ? 58 : 51;
 };
 
-// float -> double for the accumulator without the FP64 pipe (GB300 runs FP64 at a small
-// fraction of the FP32 rate): normal numbers and zero by re-biasing the exponent in integer
-// arithmetic, the rare others through the conversion instruction.
-__device__ __forceinline__ double f32_to_f64(float v)
+template <int kOff>
+__device__ __forceinline__ void lds_f2_off(unsigned addr, float &a, float &b)
 {
-    const unsigned u = __float_as_uint(v);
-    const unsigned e = (u >> 23) & 0xffu;
-    if (e - 1u < 254u) {
-        const unsigned hi = (u & 0x80000000u) | ((e + (1023u - 127u)) << 20) | ((u >> 3) & 0xfffffu);
-        return __hiloint2double((int)hi, (int)(u << 29));
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2+%3];" : "=f"(a), "=f"(b) : "r"(addr), "n"(kOff));
+}
+
+// Slices Z .. S-1 of one sample: its odd row's elements at B + kRow, its even row's at A + 2 kRow.
+template <int S, unsigned kRow, unsigned Plane, int Z = 0>
+__device__ __forceinline__ void fwd_tap(unsigned A, unsigned B, float fx, float wa, float wb, float (&sum)[S])
+{
+    if constexpr (Z < S) {
+        float ta, da, tb, db;
+        lds_f2_off<(int)(Z * Plane + 2 * kRow)>(A, ta, da);
+        lds_f2_off<(int)(Z * Plane + kRow)>(B, tb, db);
+        sum[Z] = fmaf(wa, fmaf(fx, da, ta), sum[Z]);
+        sum[Z] = fmaf(wb, fmaf(fx, db, tb), sum[Z]);
+        fwd_tap<S, kRow, Plane, Z + 1>(A, B, fx, wa, wb, sum);
     }
-    if ((u & 0x7fffffffu) == 0u) return __hiloint2double((int)(u & 0x80000000u), 0);
-    return (double)v;
 }
 
-// One slice element (t00, dx | dy, dxy) of a record as two packed pairs.
-__device__ __forceinline__ void lds_2f2(unsigned addr, f2x &lo, f2x &hi)
+// Two samples of one ray at once, Yc = the halves of yc2 (f32x2 arithmetic, lane for lane the scalar
+// one): coordinates x = fma(Yc, s, ax), y = fma(Yc, c, ay); floor(x) as a round-down add of 1.5*2^23;
+// 2 floor(y/2) -- the even row at or above y -- as a round-down add of 1.5*2^24 (spacing 2).  With e =
+// y - (that row + 1) in [-1, 1): the odd row is that row + 1, weight 1 - |e|; the even one is that row
+// (e < 0) or the row below the odd one (e >= 0), weight |e|.  Pred: only where on0 / on1 are set.
+// [alo, ahi]: the byte addresses a load may take (checked in the bounds-checked build only).
+template <int S, int T, bool Pred>
+__device__ __forceinline__ void fwd_pair(f2x yc2, f2x s2, f2x c2, f2x ax2, f2x ay2, f2x M23, f2x M24, f2x one2,
+                                         unsigned base2, bool on0, bool on1, unsigned alo, unsigned ahi, float (&sum)[S])
 {
-    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(addr));
-}
-
-// The eight slices' elements of the record at byte address rec, slot r from offset off[r],
-// added to the slots' partial sums: part[r] += (1, fx) * ((t00, dx) + fy * (dy, dxy)).
-__device__ __forceinline__ void ms_tap(unsigned rec, const unsigned (&off)[kMsSlices], unsigned alo, unsigned ahi,
-                                       float fx, float fy, f2x (&part)[kMsSlices])
-{
-    if (!XCT_IN(rec, alo, ahi, XCT_SITE_FWD_MS_TAP)) return;
-    f2x lo[kMsSlices], hi[kMsSlices];
+    constexpr unsigned kRow = FwdTile<S, T>::P * 8, Plane = FwdTile<S, T>::Plane;
+    const f2x x2 = f2_fma(yc2, s2, ax2), y2 = f2_fma(yc2, c2, ay2);
+    const f2x tx = f2_add_rd(x2, M23), ty = f2_add_rd(y2, M24);
+    const f2x fx2 = f2_sub(x2, f2_sub(tx, M23));
+    const f2x e2 = f2_sub(y2, f2_add(f2_sub(ty, M24), one2));  // from the odd row: exact where the weight is small
+    int ix[2], jy[2];
+    float fx[2], e[2];
+    f2_unpack_bits(tx, ix[0], ix[1]);
+    f2_unpack_bits(ty, jy[0], jy[1]);
+    f2_unpack(fx2, fx[0], fx[1]);
+    f2_unpack(e2, e[0], e[1]);
 #pragma unroll
-    for (int r = 0; r < kMsSlices; ++r) lds_2f2(rec + off[r], lo[r], hi[r]);
-    const f2x fy2 = f2_pack(fy, fy), wx = f2_pack(1.0f, fx);
-#pragma unroll
-    for (int r = 0; r < kMsSlices; ++r) part[r] = f2_fma(wx, f2_fma(fy2, hi[r], lo[r]), part[r]);
+    for (int q = 0; q < 2; ++q) {
+        if (Pred && !(q ? on1 : on0)) continue;
+        const unsigned B = (unsigned)jy[q] * (2u * kRow) + ((unsigned)ix[q] * 8u + base2);
+        const unsigned A = B + (unsigned)(__float_as_int(e[q]) >> 31) * (2u * kRow);
+        if (!XCT_IN(A + 2 * kRow, alo, ahi, XCT_SITE_FWD_TAP) || !XCT_IN(B + kRow, alo, ahi, XCT_SITE_FWD_TAP)) continue;
+        const float wa = fabsf(e[q]);
+        fwd_tap<S, kRow, Plane>(A, B, fx[q], wa, 1.0f - wa, sum);
+    }
 }
 
-// grid: (ntx*nty tiles, angle chunks, dN / 8 slice groups); acc [dN][nrows][px] doubles.
-template <int T>
-__global__ void __launch_bounds__(kMsThreads, 1) fwd_ms_kernel(const float *__restrict__ img,
-                                                               double *__restrict__ acc,
-                                                               const float2 *__restrict__ trig, KGeom g, int sub,
-                                                               int step, int nrows, int ntx, int chunk)
+// The sums of a ray's four lanes: lane ph of the four ends with slice ph's (S = 1: lane 0's; S = 5:
+// lane 0 also has slice 4's in `fifth`).
+template <int S>
+__device__ __forceinline__ float fwd_reduce(const float (&sum)[S], int ph, float &fifth)
 {
-    // 128-byte records, read with 128-bit loads
-    extern __shared__ __align__(128) unsigned char ms_smem[];
-    float4 *tile = reinterpret_cast<float4 *>(ms_smem);
-    float2 *scs = reinterpret_cast<float2 *>(ms_smem + FwdMsTile<T>::TileBytes);
-    float2 *inv_s = scs + kAngChunk;
-    int *xlo_s = reinterpret_cast<int *>(inv_s + kAngChunk);
-    int *xhi_s = xlo_s + kAngChunk;
-    int *gpre = xhi_s + kAngChunk;
-    int *tail = gpre + kAngChunk;  // [0] ray groups of the chunk, [1] work counter
-    const int k0 = (int)blockIdx.y * chunk;
+    float v;
+    if constexpr (S == 1) {
+        v = sum[0] + __shfl_xor_sync(0xffffffffu, sum[0], 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+    } else if constexpr (S == 2) {
+        const bool odd = ph & 1;
+        v = (odd ? sum[1] : sum[0]) + __shfl_xor_sync(0xffffffffu, odd ? sum[0] : sum[1], 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+    } else {
+        const bool hi = ph & 2, odd = ph & 1;
+        const float s3 = S > 3 ? sum[S > 3 ? 3 : 0] : 0.0f;
+        const float k0 = (hi ? sum[2] : sum[0]) + __shfl_xor_sync(0xffffffffu, hi ? sum[0] : sum[2], 2);
+        const float k1 = (hi ? s3 : sum[1]) + __shfl_xor_sync(0xffffffffu, hi ? sum[1] : s3, 2);
+        v = (odd ? k1 : k0) + __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 1);
+        if constexpr (S == 5) {
+            fifth = sum[4] + __shfl_xor_sync(0xffffffffu, sum[4], 1);
+            fifth += __shfl_xor_sync(0xffffffffu, fifth, 2);
+        }
+    }
+    return v;
+}
+
+// The work of one CTA: tile (bx, by) of S slices (images from im, accumulators from acc [S][nrows][px])
+// for the subset angles k0 .. k0+chunk-1 (chunk <= kAngChunk).  Starts and ends with all threads in
+// step.
+template <int S, int T>
+__device__ __forceinline__ void fwd_tile(const KGeom &g, const float *im, double *acc, const float2 *__restrict__ trig,
+                                         int sub, int step, int nrows, int bx, int by, int k0, int chunk,
+                                         unsigned char *smem_raw)
+{
+    typedef FwdTile<S, T> C;
+    constexpr int kThr = C::Threads;
+    float4 *s_cs = reinterpret_cast<float4 *>(smem_raw + C::TableOff);
+    int4 *s_ray = reinterpret_cast<int4 *>(s_cs + kAngChunk);
     const int kn = min(chunk, nrows - k0);
     if (kn <= 0) return;
-    const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
     const int x0 = -1 + bx * T, y0 = -1 + by * T;
-    const int z0 = (int)blockIdx.z * kMsSlices;
     const size_t nimg = (size_t)g.nx * g.ny;
-    const float *im0 = img + (size_t)z0 * nimg;
 
-    // element (c, r) of slice z at tile[(r*T + c)*8 + z]; texels outside the image are 0.
-    // A warp stages a strip of four columns x eight slices (lane 8*cl + z: column 4u + cl of
-    // slice z) over kMsStageRows element rows, walking down the texel rows: each texel is
-    // loaded once, its right neighbour comes from the next column's lane (the strip's last
-    // column loads it), and the quarter-warps store whole records (no bank conflict).
+    // element (c, r) = (t(x0+c, y0+r), t(x0+c+1, y0+r) - t(x0+c, y0+r)), zero border.  A warp stages
+    // rows of a slice: each texel is loaded once, its right neighbour comes from the next lane.
+    const int lane = threadIdx.x & 31;
     {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int cl = lane >> 3, z = lane & (kMsSlices - 1);
-        const float *im = im0 + (size_t)z * nimg;
-        constexpr int kStrips = (T + 3) / 4, kBands = (T + kMsStageRows - 1) / kMsStageRows;
-        for (int u = warp; u < kStrips * kBands; u += kMsThreads / 32) {
-            const int c = (u % kStrips) * 4 + cl, r0 = (u / kStrips) * kMsStageRows;
-            const int gx = x0 + c;
-            const bool c0 = (unsigned)gx < (unsigned)g.nx, c1 = (unsigned)(gx + 1) < (unsigned)g.nx;
-            float tp = 0.0f, trp = 0.0f;
+        constexpr int kCols = T / 32 + 1;  // lanes cover columns 0 .. T
+#pragma unroll 2
+        for (int q = threadIdx.x >> 5; q < S * C::Rows; q += kThr / 32) {
+            const int z = q / C::Rows, r = q - z * C::Rows;
+            const int gy = y0 + r;
+            const bool rv = (unsigned)gy < (unsigned)g.ny;
+            const float *row = im + (size_t)z * nimg + ((long long)gy * g.nx + x0);
+            float t[kCols + 1];
 #pragma unroll
-            for (int j = 0; j <= kMsStageRows; ++j) {
-                const int r = r0 + j, gy = y0 + r;
-                const bool rv = (unsigned)gy < (unsigned)g.ny && r <= T;
-                const long long o = (long long)gy * g.nx + gx;
-                const float t = (rv && c0) ? __ldg(im + o) : 0.0f;
-                float tr = __shfl_down_sync(0xffffffffu, t, 8);
-                if (cl == 3) tr = (rv && c1) ? __ldg(im + o + 1) : 0.0f;
-                if (j > 0 && c < T && r - 1 < T) {
-                    const float d0 = trp - tp, d1 = tr - t;
-                    tile[((r - 1) * T + c) * kMsSlices + z] = make_float4(tp, d0, t - tp, d1 - d0);
-                }
-                tp = t;
-                trp = tr;
+            for (int u = 0; u < kCols; ++u) {
+                const int c = lane + 32 * u;
+                t[u] = (rv && (unsigned)(x0 + c) < (unsigned)g.nx) ? row[c] : 0.0f;
+            }
+            t[kCols] = 0.0f;
+            unsigned char *dst = smem_raw + (size_t)z * C::Plane + (size_t)(r * C::P + lane) * 8;
+#pragma unroll
+            for (int u = 0; u < kCols; ++u) {
+                const float a = __shfl_down_sync(0xffffffffu, t[u], 1), b = __shfl_sync(0xffffffffu, t[u + 1], 0);
+                const float t1 = lane == 31 ? b : a;
+                if (lane + 32 * u < T) *reinterpret_cast<float2 *>(dst + 256 * u) = make_float2(t[u], t1 - t[u]);
             }
         }
     }
     // owned base-texel ranges (the union over tiles is [-1, n-1])
     const float xlo = (float)x0, xhi = (float)min(x0 + T, g.nx);
     const float ylo = (float)y0, yhi = (float)min(y0 + T, g.ny);
-    for (int k = threadIdx.x; k < kn; k += kMsThreads) {
+    for (int k = threadIdx.x; k < kn; k += kThr) {
         const float2 cs = trig[sub + (k0 + k) * step];
-        scs[k] = cs;
-        inv_s[k] = make_float2(1.0f / cs.x, 1.0f / cs.y);
-        // rays that can reach the tile: the (expanded) tile corners on the detector axis
+        s_cs[k] = make_float4(cs.x, cs.y, 1.0f / cs.x, 1.0f / cs.y);
+        // rays that can reach the tile: its corners on the detector axis, X = (x - nx/2) c -
+        // (y - ny/2) s + cx (rounding stays far below the 0.25 allowed on either side)
         float pmin = 3.0e38f, pmax = -3.0e38f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const float px_ = (q & 1) ? xhi + 2.0f : xlo - 2.0f;
-            const float py_ = (q & 2) ? yhi + 2.0f : ylo - 2.0f;
-            const float p = (px_ - g.hx) * cs.x - (py_ - g.hy) * cs.y + g.cx;
+            const float p = (((q & 1) ? xhi : xlo) - g.hx) * cs.x - (((q & 2) ? yhi : ylo) - g.hy) * cs.y + g.cx;
             pmin = fminf(pmin, p);
             pmax = fmaxf(pmax, p);
         }
-        xlo_s[k] = max(0, (int)floorf(pmin) - 1);
-        xhi_s[k] = min(g.px - 1, (int)ceilf(pmax) + 1);
+        const int xa = max(0, (int)ceilf(pmin - 0.25f)), xb = min(g.px - 1, (int)floorf(pmax + 0.25f));
+        s_ray[k] = make_int4(xa, xb, 0, xb < xa ? 0 : (xb - xa) / kRaysPerWarp + 1);
     }
     __syncthreads();
-    if (threadIdx.x < 32) {  // exclusive prefix of the ray groups per angle (warp 0)
-        const int lane = threadIdx.x;
+    if (threadIdx.x < 32) {  // the angles' item ranges: a running sum of their ray groups (warp 0)
         int carry = 0;
         for (int b = 0; b < kn; b += 32) {
             const int k = b + lane;
-            const int n = k < kn ? max(0, (xhi_s[k] - xlo_s[k] + kMsRays) / kMsRays) : 0;
+            const int n = k < kn ? s_ray[k].w : 0;
             int v = n;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int t = __shfl_up_sync(0xffffffffu, v, o);
                 if (lane >= o) v += t;
             }
-            if (k < kn) gpre[k] = carry + v - n;
+            if (k < kn) {
+                s_ray[k].z = carry + v - n;
+                s_ray[k].w = carry + v;
+            }
             carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) {
-            tail[0] = carry;
-            tail[1] = 0;
         }
     }
     __syncthreads();
 
-    const int total = tail[0];
-    const int lane = threadIdx.x & 31;
-    const int ph = lane & (kMsSlices - 1);    // lane of the quarter; also this lane's first slot
-    const int qb = lane & ~(kMsSlices - 1);   // first lane of the quarter
-    const int pair = lane >> 3;               // ray pair of the warp's four
-    const int half = ph / kMsLanesPerRay;     // 0: the pair's first ray, 1: its second
-    const int jr = ph % kMsLanesPerRay;       // this lane's phase in its ray's samples
     const int D = g.depth;
-    // byte address of the record of base texel (col, row) from the floor bits:
-    // (iy_bits * T + ix_bits) * 128 + base2, the biases folded into base2 (mod 2^32)
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(tile);
-    const unsigned bias = (unsigned)XCT_FLOOR_BIAS;
-    const unsigned base2 =
-        sbase - ((bias + (unsigned)y0) * (unsigned)T + bias + (unsigned)x0) * (unsigned)(kMsSlices * 16);
-    const unsigned alo = sbase, ahi = sbase + (unsigned)((T * T - 1) * kMsSlices * 16);
-    // slot r of this lane holds slice (r + ph) mod 8, read at byte offset 16 * that
-    unsigned off[kMsSlices];
-#pragma unroll
-    for (int r = 0; r < kMsSlices; ++r) off[r] = 16u * (unsigned)((r + ph) & (kMsSlices - 1));
-    const f2x MM = f2_pack(kMagic, kMagic);
-    // the four lanes of a ray find its four interval limits: the lower (even jr) or upper
-    // (odd jr) Y limit from the x (jr < 2) or the y coordinate
-    const bool bound_x = jr < 2;
-    const bool upper = (jr & 1) != 0;
-    int *counter = tail + 1;
-    int k = 0;  // the warp's current angle: items only grow, so the search runs forward
+    const int total = s_ray[kn - 1].w;
+    // shared address of element (col, row) from the round-down bits of the coordinates, the biases
+    // folded into base2 (mod 2^32): bits(1.5*2^24 + 2j) = kBias24 + j
+    const unsigned sbase = (unsigned)__cvta_generic_to_shared(smem_raw);
+    constexpr unsigned kRow = C::P * 8, kBias24 = 0x4BC00000u;
+    const unsigned base2 = sbase - kBias24 * (2u * kRow) - (unsigned)y0 * kRow - ((unsigned)XCT_FLOOR_BIAS + (unsigned)x0) * 8u;
+    const f2x M23 = f2_pack(kMagic, kMagic), M24 = f2_pack(2.0f * kMagic, 2.0f * kMagic), one2 = f2_pack(1.0f, 1.0f);
+    const f2x step2 = f2_pack(8.0f, 8.0f);
+    const unsigned alo = sbase, ahi = sbase + C::Plane - 8;
+    const int ray = lane / kLanesPerRay;  // ray within the warp's 8
+    const int ph = lane % kLanesPerRay;   // sample phase of this lane
+    // lane phase 0/1 bound the x coordinate, 2/3 the y coordinate (lower / upper Y limit)
+    const bool bound_x = ph < 2;
+    const bool upper = (ph & 1) != 0;
+    const float blo = bound_x ? xlo : ylo, bhi = bound_x ? xhi : yhi;
+    double *accl = acc + (S > 1 ? (size_t)(ph < S ? ph : 0) * nrows * g.px : 0);
 
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(counter, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= total) break;
-        while (k + 1 < kn && gpre[k + 1] <= item) ++k;  // the last k with gpre[k] <= item
-        const float c = scs[k].x, s = scs[k].y;
-        // the quarter's two consecutive rays XA and XA + 1; this lane's ray X
-        const int XA = xlo_s[k] + (item - gpre[k]) * kMsRays + 2 * pair;
-        const int X = XA + half;
+    // items (angle, 8 consecutive rays), strided over the warps
+    int k = 0;
+    for (int item = threadIdx.x >> 5; item < total; item += kThr / 32) {
+        int4 rr = s_ray[k];
+        while (item >= rr.w) rr = s_ray[++k];
+        const float4 cs = s_cs[k];
+        const float c = cs.x, s = cs.y;
+        const int X = rr.x + (item - rr.z) * kRaysPerWarp + ray;
         const float Xc = (float)X - g.cx;
         const float ax = fmaf(Xc, c, g.hx);
         const float ay = fmaf(Xc, -s, g.hy);
+        // the four interval limits of this ray, one per lane of its group: the lower (even
+        // phase) or upper (odd phase) Y limit from the x (phase 0/1) or y (2/3) coordinate
         int v = 0;
-        if (X <= xhi_s[k]) {
-            const float a = bound_x ? ax : ay, sl = bound_x ? s : c;
-            const float isl = bound_x ? inv_s[k].y : inv_s[k].x;
-            const float lo_ = bound_x ? xlo : ylo, hi_ = bound_x ? xhi : yhi;
+        if (X <= rr.y) {
+            const float a = bound_x ? ax : ay, sl = bound_x ? s : c, isl = bound_x ? cs.w : cs.z;
             if (sl != 0.0f) {
                 // sl > 0: [first(u >= lo), first(u >= hi)); sl < 0: [first(u < hi), first(u < lo))
-                const float b = ((sl > 0.0f) != upper) ? lo_ : hi_;
-                v = first_true(b, a, sl, isl, g.hd, D);
+                v = first_true(((sl > 0.0f) != upper) ? blo : bhi, a, sl, isl, g.hd, D);
             } else {  // constant coordinate: all samples or none
-                v = upper ? ((a >= lo_ && a < hi_) ? D : 0) : 0;
+                v = upper ? ((a >= blo && a < bhi) ? D : 0) : 0;
             }
         }
-        // the ray's limits: lower ones (even jr) max-combined, upper ones min-combined across
-        // the x and y limits (xor 2), then exchanged within the pair of lanes (xor 1)
+        // lower limits (even phases) max-combined, upper ones min-combined across x and y (xor 2),
+        // then exchanged within the pair of lanes (xor 1)
         const int w = __shfl_xor_sync(0xffffffffu, v, 2);
         const int m = upper ? min(v, w) : max(v, w);
         const int u = __shfl_xor_sync(0xffffffffu, m, 1);
-        const int ya = upper ? u : m, yb = upper ? m : u;
-        const int L = max(yb - ya, 0);
-        const int Lo = __shfl_xor_sync(0xffffffffu, L, kMsLanesPerRay);  // the other ray's
-        // samples ya + jr, ya + jr + 4, ... of this lane's ray; Yc = Y - hd is tracked as a
-        // float (exact small integers)
-        const int n = L > jr ? (L - jr + kMsLanesPerRay - 1) / kMsLanesPerRay : 0;
-        float yc = (float)(ya + jr) - g.hd;
-        const f2x sc = f2_pack(s, c);
-        const f2x axy = f2_pack(ax, ay);
-        f2x part[kMsSlices];
+        const int ya = upper ? u : m, len = max((upper ? m : u) - ya, 0);  // this ray's samples ya .. ya+len-1
+        const f2x s2 = f2_pack(s, s), c2 = f2_pack(c, c), ax2 = f2_pack(ax, ax), ay2 = f2_pack(ay, ay);
+        float sum[S];
 #pragma unroll
-        for (int r = 0; r < kMsSlices; ++r) part[r] = 0ull;
-        for (int i = 0; i < n; ++i, yc += (float)kMsLanesPerRay) {
-            const f2x xy = f2_fma(f2_pack(yc, yc), sc, axy);
-            const f2x tb = f2_add_rd(xy, MM);
-            const f2x fr = f2_sub(xy, f2_sub(tb, MM));
-            int ixb, iyb;
-            float fx, fy;
-            f2_unpack_bits(tb, ixb, iyb);
-            f2_unpack(fr, fx, fy);
-            ms_tap(((unsigned)iyb * (unsigned)T + (unsigned)ixb) * (unsigned)(kMsSlices * 16) + base2, off, alo, ahi,
-                   fx, fy, part);
+        for (int z = 0; z < S; ++z) sum[z] = 0.0f;
+        if constexpr (S == 1) {
+            // one slice is bound by issue, not by the data path: every ray starts at its own first
+            // sample (0.165 wavefronts per sample), which saves the warp-wide limits and the edge steps
+            const float yc0 = (float)(ya + ph) - g.hd;
+            f2x yc2 = f2_pack(yc0, yc0 + 4.0f);
+            int n = len - ph;  // samples ya + ph, + 4, + 8, ... while n > 0
+            for (; n > 4; n -= 8) {
+                fwd_pair<S, T, false>(yc2, s2, c2, ax2, ay2, M23, M24, one2, base2, true, true, alo, ahi, sum);
+                yc2 = f2_add(yc2, step2);
+            }
+            if (n > 0) fwd_pair<S, T, true>(yc2, s2, c2, ax2, ay2, M23, M24, one2, base2, true, false, alo, ahi, sum);
+        } else {
+            // all rays start at the warp's first sample, so that the 8 rays x 4 samples of a load stay a
+            // compact patch (0.14 wavefronts per sample): a ray's lane ph takes Y = y0w + ph, + 4, + 8, ...
+            // Steps of 8 samples; between the latest start and the earliest end every lane is inside its ray.
+            const int y0w = __reduce_min_sync(0xffffffffu, len > 0 ? ya : 0x3fffffff);
+            const int steps = (__reduce_max_sync(0xffffffffu, len > 0 ? ya + len : 0) - y0w + 7) >> 3;
+            const int p0 = min((__reduce_max_sync(0xffffffffu, len > 0 ? ya : 0x3fffffff) - y0w + 7) >> 3, steps);
+            const int p1 = max((__reduce_min_sync(0xffffffffu, len > 0 ? ya + len : 0) - y0w) >> 3, p0);
+            const float yc0 = (float)(y0w + ph) - g.hd;
+            f2x yc2 = f2_pack(yc0, yc0 + 4.0f);
+            int q = y0w + ph - ya;  // this lane's sample, counted from its ray's first
+            int p = 0;
+            auto edge = [&](int end) {
+                for (; p < end; ++p) {
+                    fwd_pair<S, T, true>(yc2, s2, c2, ax2, ay2, M23, M24, one2, base2, (unsigned)q < (unsigned)len,
+                                         (unsigned)(q + 4) < (unsigned)len, alo, ahi, sum);
+                    yc2 = f2_add(yc2, step2);
+                    q += 8;
+                }
+            };
+            edge(p0);
+            for (; p < p1; ++p) {
+                fwd_pair<S, T, false>(yc2, s2, c2, ax2, ay2, M23, M24, one2, base2, true, true, alo, ahi, sum);
+                yc2 = f2_add(yc2, step2);
+            }
+            q = y0w + ph - ya + 8 * p;
+            edge(steps);
         }
-        // lane p gathers slice p's partial sums from lanes (p - d) mod 8 of its quarter, slot
-        // d: lanes 0-3 hold the first ray's, lanes 4-7 the second's
-        float tot0 = 0.0f, tot1 = 0.0f;
-#pragma unroll
-        for (int d = 0; d < kMsSlices; ++d) {
-            const int sp = (ph - d) & (kMsSlices - 1);
-            float plo, phi;
-            f2_unpack(part[d], plo, phi);
-            const float pv = __shfl_sync(0xffffffffu, plo + phi, qb + sp);
-            if (sp < kMsLanesPerRay) tot0 += pv;
-            else tot1 += pv;
+        // the ray's partial sums over this tile: the 4 phases, then one atomic per slice
+        float fifth = 0.0f;
+        const float tot = fwd_reduce<S>(sum, ph, fifth);
+        if (len > 0 && XCT_IN((long long)(k0 + k) * g.px + X, 0, (long long)nrows * g.px - 1, XCT_SITE_FWD_ACC)) {
+            const size_t o = (size_t)(k0 + k) * g.px + X;
+            if (ph < S) atomicAdd(accl + o, (double)tot);
+            if (S == 5 && ph == 0) atomicAdd(acc + (size_t)4 * nrows * g.px + o, (double)fifth);
         }
-        const int L0 = half ? Lo : L, L1 = half ? L : Lo;
-        double *accz = acc + ((size_t)(z0 + ph) * nrows + k0 + k) * g.px;
-        if (L0 > 0 && XCT_IN((long long)k * g.px + XA, 0, (long long)(nrows - k0) * g.px - 1, XCT_SITE_FWD_ACC))
-            atomicAdd(accz + XA, f32_to_f64(tot0));
-        if (L1 > 0 && XCT_IN((long long)k * g.px + XA + 1, 0, (long long)(nrows - k0) * g.px - 1, XCT_SITE_FWD_ACC))
-            atomicAdd(accz + XA + 1, f32_to_f64(tot1));
     }
+}
+
+// grid: (ntx*nty tiles, angle chunks, groups of S slices).  acc: [groups * S][nrows][px] doubles.
+template <int S, int T>
+__global__ void __launch_bounds__(FwdTile<S, T>::Threads, FwdTile<S, T>::MinBlocks)
+    fwd_tiled_kernel(const float *img, double *acc, const float2 *__restrict__ trig, KGeom g, int sub, int step, int nrows,
+                     int ntx, int chunk)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    xct_grid_wait();
+    xct_grid_trigger();
+    const size_t z = (size_t)blockIdx.z * S;
+    fwd_tile<S, T>(g, img + z * g.nx * g.ny, acc + z * nrows * g.px, trig, sub, step, nrows, (int)blockIdx.x % ntx,
+                   (int)blockIdx.x / ntx, (int)blockIdx.y * chunk, chunk, smem_raw);
 }
 
 // ------------------------------------------------------------------- exact adjoint
@@ -1253,9 +1077,10 @@ static int launch_adj_gather(const KGeom &g, const float2 *trig, const float *si
 }
 
 // acc -> OSEM1 ratio (meas != nullptr) or raw projection, rows th = sub + k*step; clears acc.
-__global__ void fwd_finalize_kernel(double *__restrict__ acc, const float *__restrict__ meas,
-                                    float *__restrict__ out, KGeom g, int sub, int step, int nrows)
+__global__ void fwd_finalize_kernel(double *acc, const float *meas, float *out, KGeom g, int sub, int step, int nrows)
 {
+    xct_grid_wait();
+    xct_grid_trigger();
     const int X = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = blockIdx.y, z = blockIdx.z;
     if (X >= g.px) return;
@@ -1274,10 +1099,11 @@ __global__ void fwd_finalize_kernel(double *__restrict__ acc, const float *__res
 
 // The same for 4 consecutive bins per thread (px % 4 == 0, exact measured fetch, 16-byte
 // aligned sinograms): float4 / double2 accesses, each bin's arithmetic unchanged.
-__global__ void __launch_bounds__(256) fwd_finalize4_kernel(double *__restrict__ acc, const float *__restrict__ meas,
-                                                            float *__restrict__ out, KGeom g, int sub, int step,
-                                                            int nrows)
+__global__ void __launch_bounds__(256) fwd_finalize4_kernel(double *acc, const float *meas, float *out, KGeom g, int sub,
+                                                            int step, int nrows)
 {
+    xct_grid_wait();
+    xct_grid_trigger();
     const int X = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const int k = blockIdx.y, z = blockIdx.z;
     if (X >= g.px) return;
@@ -1290,7 +1116,7 @@ __global__ void __launch_bounds__(256) fwd_finalize4_kernel(double *__restrict__
     const size_t o = ((size_t)z * g.pa + th) * g.px + X;
     float4 r;
     if (meas != nullptr) {
-        const float4 y = __ldg(reinterpret_cast<const float4 *>(meas + o));
+        const float4 y = *reinterpret_cast<const float4 *>(meas + o);
         r = make_float4(xct_ratio(y.x, p0), xct_ratio(y.y, p1), xct_ratio(y.z, p2), xct_ratio(y.w, p3));
     } else {
         r = make_float4(p0, p1, p2, p3);
@@ -1370,7 +1196,7 @@ __device__ __forceinline__ void bp_tile(const KGeom &g, float *__restrict__ img,
             const int k = i / kBpW, j = i - k * kBpW;
             const int bin = slo[k] + j;
             const int th = sub + (k0 + k) * g.ss;
-            win[i] = ((unsigned)bin < (unsigned)g.px) ? __ldg(rt + (size_t)th * g.px + bin) : 0.0f;
+            win[i] = ((unsigned)bin < (unsigned)g.px) ? ld_global(rt + (size_t)th * g.px + bin) : 0.0f;
         }
         __syncthreads();
         const unsigned wlo = wbase, whi = wbase + 4u * (unsigned)(kn * kBpW - 1);
@@ -1424,13 +1250,14 @@ __device__ __forceinline__ void bp_tile(const KGeom &g, float *__restrict__ img,
 
 // grid: (ntx*nty tiles, 1, dN).
 template <int R>
-__global__ void __launch_bounds__(BpCfg<R>::Threads) bp_tiled_kernel(float *__restrict__ img,
-                                                            const float *__restrict__ ratio,
+__global__ void __launch_bounds__(BpCfg<R>::Threads) bp_tiled_kernel(float *img, const float *ratio,
                                                             const float2 *__restrict__ trig, KGeom g, int sub,
                                                             int nang, int ntx, float ssf, float paf)
 {
     __shared__ BpShared sh;
     const int z = blockIdx.z;
+    xct_grid_wait();
+    xct_grid_trigger();
     bp_tile<R>(g, img + (size_t)z * g.nx * g.ny, ratio + (size_t)z * g.pa * g.px, trig, sub, nang,
             (int)blockIdx.x % ntx, (int)blockIdx.x / ntx, ssf, paf, sh);
 }
@@ -1447,6 +1274,7 @@ __global__ void __launch_bounds__(BpCfg<R>::Threads) bp_tiled_kernel(float *__re
 // the literal bin expression of bp_tiled_kernel, one address, eight 4-byte loads at constant
 // offsets (one per slice), four packed adds -- in angle order, so each slice's sum is
 // bp_tiled_kernel's bit for bit -- and the update at the end.
+constexpr int kMsSlices = 8;  // slices per group of the slice-interleaved kernels
 constexpr int kBpMsT = 32;
 constexpr int kBpMsThreads = 256;
 constexpr int kBpMsW = 52;      // staged bins per angle and slice (>= 31|c| + 31|s| + 3 + 3 = 49.9)
@@ -1465,11 +1293,13 @@ struct BpMsShared {
 // grid: (ntx*nty tiles of 32 x 32, 1, dN / S slice groups), S = 8 or 2.  vec: 16-byte staging
 // copies (px a multiple of 4 and a 16-byte aligned ratio array).
 template <int S>
-__global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *__restrict__ img, const float *__restrict__ ratio,
+__global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const float *ratio,
                                                              const float2 *__restrict__ trig, KGeom g, int sub,
                                                              int nang, int ntx, float ssf, float paf, int vec)
 {
     __shared__ __align__(16) BpMsShared<S> sh;
+    xct_grid_wait();
+    xct_grid_trigger();
     const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
     const int z0 = (int)blockIdx.z * S;
     const size_t nimg = (size_t)g.nx * g.ny, nprj = (size_t)g.pa * g.px;
@@ -1632,7 +1462,7 @@ __device__ __forceinline__ int unit_item(const int *__restrict__ base, int n, in
 }
 
 template <int T>
-__global__ void __launch_bounds__(kFwdThreads, FwdTile<T>::MinBlocks) fwd_batched_kernel(const XctItemDev *__restrict__ items,
+__global__ void __launch_bounds__(FwdTile<1, T>::Threads, FwdTile<1, T>::MinBlocks) fwd_batched_kernel(const XctItemDev *__restrict__ items,
                                                                      const int *__restrict__ base, int n, int sub,
                                                                      int *queue)
 {
@@ -1649,7 +1479,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdTile<T>::MinBlocks) fwd_batche
         const int local = u - base[i];
         const int tiles = it.fwd_ntx * it.fwd_nty;
         const int t = local % tiles, ch = local / tiles;
-        fwd_tile<T>(g, it.img, it.acc, it.trig, sub, g.ss, nrows, t % it.fwd_ntx, t / it.fwd_ntx, ch * g.fwd_chunk,
+        fwd_tile<1, T>(g, it.img, it.acc, it.trig, sub, g.ss, nrows, t % it.fwd_ntx, t / it.fwd_ntx, ch * g.fwd_chunk,
                     g.fwd_chunk, smem_raw);
         __syncthreads();  // the tile in shared memory is restaged by the next unit
     }
@@ -1705,14 +1535,13 @@ bool xct_fwd_tile_valid(int T) { return T == 44 || T == 60 || T == 76 || T == 92
 // Raises a kernel's dynamic shared-memory limit once per device.  Host threads may race on
 // the first call of a device: the flags are atomic, and setting the attribute twice is
 // harmless.  Devices beyond the table set it on every call.
-template <int T>
-static int fwd_smem_attr(const void *fn, std::atomic<bool> *done)
+static int smem_attr(const void *fn, size_t smem, std::atomic<bool> *done)
 {
     int dev = 0;
     XCT_CUDA_TRY(cudaGetDevice(&dev));
     const bool cached = dev >= 0 && dev < 64;
     if (!cached || !done[dev].load(std::memory_order_acquire)) {
-        XCT_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FwdTile<T>::Smem));
+        XCT_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (cached) done[dev].store(true, std::memory_order_release);
     }
     return XCT_OK;
@@ -1750,10 +1579,10 @@ int xct_batched_grids(int device, int sm_count, int fwd_T, int grids[3])
     int rc = with_tile(fwd_T, [&](auto tc) -> int {
         constexpr int T = decltype(tc)::value;
         static std::atomic<bool> done[64];
-        int r = fwd_smem_attr<T>((const void *)fwd_batched_kernel<T>, done);
+        int r = smem_attr((const void *)fwd_batched_kernel<T>, FwdTile<1, T>::Smem, done);
         if (r) return r;
-        XCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fwd_batched_kernel<T>, kFwdThreads,
-                                                                   FwdTile<T>::Smem));
+        XCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fwd_batched_kernel<T>, FwdTile<1, T>::Threads,
+                                                                   FwdTile<1, T>::Smem));
         return XCT_OK;
     });
     if (rc) return rc;
@@ -1769,7 +1598,7 @@ int launch_osem_step_batched(const XctItemDev *items, const int *bases /*[3][n+1
 {
     int rc = with_tile(fwd_T, [&](auto tc) -> int {
         constexpr int T = decltype(tc)::value;
-        fwd_batched_kernel<T><<<grids[0], kFwdThreads, FwdTile<T>::Smem, st>>>(items, bases, n, sub, queues);
+        fwd_batched_kernel<T><<<grids[0], FwdTile<1, T>::Threads, FwdTile<1, T>::Smem, st>>>(items, bases, n, sub, queues);
         XCT_CUDA_TRY(cudaGetLastError());
         return XCT_OK;
     });
@@ -1789,7 +1618,7 @@ int launch_fwd_batched(const XctItemDev *items, const int *bases, int n, int sub
 {
     return with_tile(fwd_T, [&](auto tc) -> int {
         constexpr int T = decltype(tc)::value;
-        fwd_batched_kernel<T><<<grid, kFwdThreads, FwdTile<T>::Smem, st>>>(items, bases, n, sub, queue);
+        fwd_batched_kernel<T><<<grid, FwdTile<1, T>::Threads, FwdTile<1, T>::Smem, st>>>(items, bases, n, sub, queue);
         XCT_CUDA_TRY(cudaGetLastError());
         return XCT_OK;
     });
@@ -1798,63 +1627,85 @@ int launch_fwd_batched(const XctItemDev *items, const int *bases, int n, int sub
 int fwd_tiled_rows_cap() { return kAngChunk; }
 
 int fwd_ms_slices() { return kMsSlices; }
-int fwd_ms_tile() { return kMsTile; }
 
-// The slice-interleaved forward projector over groups*8 slices (slice-group g of the grid is
-// slices 8g .. 8g+7 of img / acc).
-int launch_fwd_ms(const KGeom &g, const float2 *trig, const float *img, double *acc, int groups, int sub, int step,
-                  int nrows, int chunk, cudaStream_t st)
+// One forward launch over groups * S slices.
+template <int S, int T>
+static int launch_fwd_group(const KGeom &g, const float2 *trig, const float *img, double *acc, int groups, int sub, int step,
+                            int nrows, int chunk, cudaStream_t st)
 {
-    if (nrows <= 0 || groups <= 0) return XCT_OK;
-    if (chunk <= 0 || chunk > kAngChunk) return xct_fail(XCT_E_INVALID, "slice-interleaved angle chunk out of range");
-    constexpr int T = kMsTile;
+    typedef FwdTile<S, T> C;
     static std::atomic<bool> done[64];
-    int dev = 0;
-    XCT_CUDA_TRY(cudaGetDevice(&dev));
-    const bool cached = dev >= 0 && dev < 64;
-    if (!cached || !done[dev].load(std::memory_order_acquire)) {
-        XCT_CUDA_TRY(cudaFuncSetAttribute((const void *)fwd_ms_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)FwdMsTile<T>::Smem));
-        if (cached) done[dev].store(true, std::memory_order_release);
-    }
-    const int ntx = (g.nx + 1 + T - 1) / T, nty = (g.ny + 1 + T - 1) / T;
-    const int nch = (nrows + chunk - 1) / chunk;
-    dim3 grid(ntx * nty, nch, groups);
-    fwd_ms_kernel<T><<<grid, kMsThreads, FwdMsTile<T>::Smem, st>>>(img, acc, trig, g, sub, step, nrows, ntx, chunk);
-    g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-    XCT_CUDA_TRY(cudaGetLastError());
-    return XCT_OK;
+    const int r = smem_attr((const void *)fwd_tiled_kernel<S, T>, C::Smem, done);
+    if (r) return r;
+    const int ntx = (g.nx + 1 + T - 1) / T, nty = (g.ny + 1 + T - 1) / T;  // base texels -1 .. n-1
+    return xct_launch(fwd_tiled_kernel<S, T>, dim3(ntx * nty, (nrows + chunk - 1) / chunk, groups), C::Threads, C::Smem, st,
+                      img, acc, trig, g, sub, step, nrows, ntx, chunk);
 }
 
-// The forward projection of dN slices into the accumulator: with the slice-interleaved
-// kernel enabled (g.ms_chunk > 0), its groups of eight slices first, then the rest with the
-// per-slice tiled kernel.
+// Modelled time (SM cycles) of a forward launch of `groups` groups of S slices with tile side T and
+// nrows angles in chunks: the work of all tiles over the SMs, plus half a CTA's own time for the
+// unevenness of the last wave.  A tile and angle take T^2 (0.15 + 0.085 S) + 7 T cycles and its
+// staging 0.2 S T^2 + 400 (fits of measured launches: 2600 cycles per angle for S = 1, T = 92; 2790 for
+// S = 2, T = 83; 2010 for S = 4, T = 58).
+double xct_fwd_cost(int nx, int ny, int S, int T, int nrows, int chunk, int groups, int sms)
+{
+    const double t2 = (double)T * T;
+    const double angle = t2 * (0.15 + 0.085 * S) + 7.0 * T, stage = 0.2 * S * t2 + 400.0;
+    const int blocks = S > 1 ? 2 : T <= 76 ? 4 : 3;
+    const double area = (nx + 1.0) * (ny + 1.0) / t2 * groups;
+    const double tiles = (double)((nx + T) / T) * ((ny + T) / T) * groups;
+    const int n = (nrows + chunk - 1) / chunk;
+    return (tiles * n * stage + area * nrows * angle) / sms + 0.5 * blocks * (stage + chunk * angle);
+}
+
+// Subset angles per CTA of the grouped forms: the even split with the least modelled time.
+static int fwd_group_chunk(const KGeom &g, int S, int T, int nrows, int groups, int most)
+{
+    int best = 0;
+    double cost = 0.0;
+    for (int n = (nrows + most - 1) / most; n <= nrows; n += std::max(1, n / 8)) {
+        const int chunk = (nrows + n - 1) / n;
+        const double c = xct_fwd_cost(g.nx, g.ny, S, T, nrows, chunk, groups, device_sm_count());
+        if (best == 0 || c < cost) {
+            best = chunk;
+            cost = c;
+        }
+    }
+    return best;
+}
+
+template <int S>
+static int launch_fwd_groups(const KGeom &g, const float2 *trig, const float *&img, double *&acc, int &dN, int groups,
+                             int sub, int step, int nrows, cudaStream_t st)
+{
+    constexpr int T = FwdGroup<S>::T;
+    if (groups <= 0) return XCT_OK;
+    const int chunk = fwd_group_chunk(g, S, T, nrows, groups, g.ms_chunk > 0 ? g.ms_chunk : kAngChunk);
+    const int rc = launch_fwd_group<S, T>(g, trig, img, acc, groups, sub, step, nrows, chunk, st);
+    img += (size_t)groups * S * g.nx * g.ny;
+    acc += (size_t)groups * S * nrows * g.px;
+    dN -= groups * S;
+    return rc;
+}
+
+// The forward projection of dN slices into the accumulator: groups of four slices, the rest as one
+// group of five, three or two; a single slice (or every slice, with grouping off) with the plan's
+// tile.
 int launch_fwd_tiled_main(const KGeom &g, const float2 *trig, const float *img, double *acc, int dN, int sub, int step,
                           int nrows, cudaStream_t st)
 {
     if (nrows <= 0 || dN <= 0) return XCT_OK;
-    const int ms = g.ms_chunk > 0 ? (dN / kMsSlices) * kMsSlices : 0;
-    if (ms > 0) {
-        const int rc = launch_fwd_ms(g, trig, img, acc, ms / kMsSlices, sub, step, nrows, g.ms_chunk, st);
-        if (rc || ms == dN) return rc;
-        img += (size_t)ms * g.nx * g.ny;
-        acc += (size_t)ms * nrows * g.px;
-        dN -= ms;
+    if (g.fwd_group && dN >= 2) {
+        const bool five = dN % 4 == 1;
+        int rc = launch_fwd_groups<4>(g, trig, img, acc, dN, five ? dN / 4 - 1 : dN / 4, sub, step, nrows, st);
+        if (!rc && five) rc = launch_fwd_groups<5>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
+        if (!rc && dN == 3) rc = launch_fwd_groups<3>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
+        if (!rc && dN == 2) rc = launch_fwd_groups<2>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
+        return rc;
     }
     if (g.fwd_chunk <= 0 || g.fwd_chunk > kAngChunk) return xct_fail(XCT_E_INVALID, "forward angle chunk out of range");
     return with_tile(g.fwd_T, [&](auto tc) -> int {
-        constexpr int T = decltype(tc)::value;
-        static std::atomic<bool> done[64];
-        int r = fwd_smem_attr<T>((const void *)fwd_tiled_kernel<T>, done);
-        if (r) return r;
-        const int ntx = (g.nx + 1 + T - 1) / T;  // base texels -1 .. nx-1
-        const int nty = (g.ny + 1 + T - 1) / T;
-        const int nch = (nrows + g.fwd_chunk - 1) / g.fwd_chunk;
-        dim3 grid(ntx * nty, nch, dN);
-        fwd_tiled_kernel<T><<<grid, kFwdThreads, FwdTile<T>::Smem, st>>>(img, acc, trig, g, sub, step, nrows, ntx);
-        g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-        XCT_CUDA_TRY(cudaGetLastError());
-        return XCT_OK;
+        return launch_fwd_group<1, decltype(tc)::value>(g, trig, img, acc, dN, sub, step, nrows, g.fwd_chunk, st);
     });
 }
 
@@ -1864,16 +1715,11 @@ int launch_fwd_finalize(const KGeom &g, const float *meas, float *out, double *a
     if (nrows <= 0 || dN <= 0) return XCT_OK;
     const bool vec = g.px % 4 == 0 && g.fetch == XCT_FETCH_EXACT && (((uintptr_t)meas | (uintptr_t)out) & 15u) == 0 &&
                      ((uintptr_t)acc & 15u) == 0;
-    if (vec) {
-        dim3 g4((g.px / 4 + 255) / 256, nrows, dN);
-        fwd_finalize4_kernel<<<g4, 256, 0, st>>>(acc, meas, out, g, sub, step, nrows);
-    } else {
-        dim3 g2((g.px + 127) / 128, nrows, dN);
-        fwd_finalize_kernel<<<g2, 128, 0, st>>>(acc, meas, out, g, sub, step, nrows);
-    }
-    g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-    XCT_CUDA_TRY(cudaGetLastError());
-    return XCT_OK;
+    if (vec)
+        return xct_launch(fwd_finalize4_kernel, dim3((g.px / 4 + 255) / 256, nrows, dN), 256, 0, st, acc, meas, out, g, sub,
+                          step, nrows);
+    return xct_launch(fwd_finalize_kernel, dim3((g.px + 127) / 128, nrows, dN), 128, 0, st, acc, meas, out, g, sub, step,
+                      nrows);
 }
 
 int launch_fwd_tiled(const KGeom &g, const float2 *trig, const float *img, const float *meas, float *out,
@@ -1996,38 +1842,31 @@ int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const
         const int mtx = (g.nx + kBpMsT - 1) / kBpMsT, mty = (g.ny + kBpMsT - 1) / kBpMsT;
         const int vec = g.px % 4 == 0 && ((uintptr_t)ratio & 15u) == 0;
         const int g8 = dN / kMsSlices, g2 = (dN - g8 * kMsSlices) / 2;
+        int rc = XCT_OK;
         if (g8 > 0) {
-            bp_ms_kernel<kMsSlices><<<dim3(mtx * mty, 1, g8), kBpMsThreads, 0, st>>>(
-                img, ratio, trig, g, sub, nang, mtx, (float)g.ss, (float)g.pa, vec);
-            g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-            XCT_CUDA_TRY(cudaGetLastError());
+            rc = xct_launch(bp_ms_kernel<kMsSlices>, dim3(mtx * mty, 1, g8), kBpMsThreads, 0, st, img, ratio, trig, g, sub,
+                            nang, mtx, (float)g.ss, (float)g.pa, vec);
             img += (size_t)g8 * kMsSlices * g.nx * g.ny;
             ratio += (size_t)g8 * kMsSlices * g.pa * g.px;
             dN -= g8 * kMsSlices;
         }
-        if (g2 > 0) {
-            bp_ms_kernel<2><<<dim3(mtx * mty, 1, g2), kBpMsThreads, 0, st>>>(img, ratio, trig, g, sub, nang, mtx,
-                                                                             (float)g.ss, (float)g.pa, vec);
-            g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-            XCT_CUDA_TRY(cudaGetLastError());
+        if (g2 > 0 && rc == XCT_OK) {
+            rc = xct_launch(bp_ms_kernel<2>, dim3(mtx * mty, 1, g2), kBpMsThreads, 0, st, img, ratio, trig, g, sub, nang, mtx,
+                            (float)g.ss, (float)g.pa, vec);
             img += (size_t)g2 * 2 * g.nx * g.ny;
             ratio += (size_t)g2 * 2 * g.pa * g.px;
             dN -= g2 * 2;
         }
-        if (dN == 0) return XCT_OK;
+        if (rc || dN == 0) return rc;
     }
     const int ntx = (g.nx + kBpTX - 1) / kBpTX, nty = (g.ny + kBpTY - 1) / kBpTY;
-    dim3 grid(ntx * nty, 1, dN);
+    const dim3 grid(ntx * nty, 1, dN);
     // four rows per thread once the grid gives three waves of its resident CTAs (6 per SM)
     if ((long long)ntx * nty * dN >= 3LL * 6 * device_sm_count())
-        bp_tiled_kernel<4><<<grid, BpCfg<4>::Threads, 0, st>>>(img, ratio, trig, g, sub, nang, ntx, (float)g.ss,
-                                                                (float)g.pa);
-    else
-        bp_tiled_kernel<2><<<grid, BpCfg<2>::Threads, 0, st>>>(img, ratio, trig, g, sub, nang, ntx, (float)g.ss,
-                                                                (float)g.pa);
-    g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-    XCT_CUDA_TRY(cudaGetLastError());
-    return XCT_OK;
+        return xct_launch(bp_tiled_kernel<4>, grid, BpCfg<4>::Threads, 0, st, img, ratio, trig, g, sub, nang, ntx, (float)g.ss,
+                          (float)g.pa);
+    return xct_launch(bp_tiled_kernel<2>, grid, BpCfg<2>::Threads, 0, st, img, ratio, trig, g, sub, nang, ntx, (float)g.ss,
+                      (float)g.pa);
 }
 
 XCT_CHECK_READER(xct_check_read_tiled)

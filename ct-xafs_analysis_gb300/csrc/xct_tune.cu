@@ -159,30 +159,43 @@ const char *xct_tune_env_path()
 }
 
 // ---------------------------------------------------------------- single-shape plans
-static long long plan_ctas(const xct_plan *p, int dN, int T, int c)
-{
-    const int rows = (p->g.pa + p->g.ss - 1) / p->g.ss;
-    return (long long)((p->g.nx + T) / T) * ((p->g.ny + T) / T) * ((rows + c - 1) / c) * dN;
-}
-
 // The slice-interleaved forward projector by default: on (all subset angles per CTA) when a
 // plan's full batch holds a group of eight slices whose tiles give at least two waves of
 // CTAs (one per SM); smaller problems keep the per-slice kernel, whose smaller CTAs fill
 // the SMs better.
 static int plan_default_ms_chunk(const xct_plan *p)
 {
-    const int G = fwd_ms_slices(), T = fwd_ms_tile();
+    const int G = fwd_ms_slices(), T = 42;
     if (p->g.kernels != XCT_KERNELS_TILED || p->g.max_batch < G) return 0;
     const long long tiles = (long long)((p->g.nx + T) / T) * ((p->g.ny + T) / T);
     return tiles * (p->g.max_batch / G) >= 2LL * p->ctx->sm_count ? fwd_tiled_rows_cap() : 0;
+}
+
+// The per-slice forward tiles of a plan that has no cached choice: the tile side and the even split
+// of the subset's angles with the least modelled time for one slice (several slices go through the
+// grouped forms, whose tiles are fixed).
+static TuneChoice plan_default_tiles(const xct_plan *p)
+{
+    const int rows = (p->g.pa + p->g.ss - 1) / p->g.ss, cap = fwd_tiled_rows_cap();
+    TuneChoice best{0, 0, 0.0f};
+    double cost = 0.0;
+    for (int T : kTiles)
+        for (int n = (rows + cap - 1) / cap; n <= rows; n += std::max(1, n / 8)) {
+            const int chunk = (rows + n - 1) / n;
+            const double c = xct_fwd_cost(p->g.nx, p->g.ny, 1, T, rows, chunk, 1, p->ctx->sm_count);
+            if (best.T == 0 || c < cost) {
+                best = TuneChoice{T, chunk, 0.0f};
+                cost = c;
+            }
+        }
+    return best;
 }
 
 void xct_plan_default_tuning(xct_plan *p)
 {
     TuneChoice c;
     const std::string key = xct_tune_key(p->ctx->name, p->g.nx, p->g.ny, p->g.px, p->g.pa, p->g.ss, p->g.max_batch);
-    if (!xct_tune_lookup(key, xct_tune_env_path(), c))
-        c = xct_tune_default(p->ctx->sm_count, [&](int T, int ch) { return plan_ctas(p, p->g.max_batch, T, ch); });
+    if (!xct_tune_lookup(key, xct_tune_env_path(), c)) c = plan_default_tiles(p);
     // the cache holds the per-slice kernel's tiles; the slice-interleaved kernels' switch
     // follows the plan's shape
     c.ms_chunk = plan_default_ms_chunk(p);
@@ -209,7 +222,8 @@ int xct_plan_set_tuning(xct_plan *p, int fwd_tile, int ang_chunk)
         return xct_fail(XCT_E_INVALID, "ang_chunk must be in 1..128");
     p->kg.fwd_T = fwd_tile;
     p->kg.fwd_chunk = ang_chunk;
-    p->kg.fwd_direct = 0;  // tiles chosen by hand are used whatever the size
+    p->kg.fwd_direct = 0;  // tiles chosen by hand are used whatever the size and the batch
+    p->kg.fwd_group = 0;
     return XCT_OK;
 }
 
@@ -228,6 +242,8 @@ int xct_plan_set_multislice(xct_plan *p, int ang_chunk)
     if (ang_chunk > 0 && p->g.kernels != XCT_KERNELS_TILED)
         return xct_fail(XCT_E_UNSUPPORTED, "xct_plan_set_multislice: the plain kernels have no slice-interleaved form");
     p->kg.ms_chunk = ang_chunk;
+    p->kg.fwd_group = ang_chunk > 0;
+    p->kg.fwd_direct = 0;  // a switch set by hand holds whatever the size
     return XCT_OK;
 }
 
@@ -264,7 +280,9 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
         for (int r = 0; r < 3 && rc == XCT_OK; ++r) {  // first run warms up
             cudaMemsetAsync(p->d_acc, 0, acc_bytes, st);
             cudaEventRecord(e0, st);
-            rc = launch_fwd_tiled_main(p->kg, p->d_trig, p->d_img, p->d_acc, dN, 0, p->g.ss, nrows, st);
+            KGeom k = p->kg;
+            k.fwd_group = 0;  // the choice is the per-slice kernel's
+            rc = launch_fwd_tiled_main(k, p->d_trig, p->d_img, p->d_acc, dN, 0, p->g.ss, nrows, st);
             cudaEventRecord(e1, st);
             cudaError_t e = cudaEventSynchronize(e1);
             if (rc == XCT_OK && e != cudaSuccess) rc = xct_cuda_fail(e, "xct_plan_autotune");
