@@ -256,6 +256,7 @@ enum {
 #ifdef XCT_CHECKED
 int xct_check_read_tiled(XctCheckWord *out, bool reset);
 int xct_check_read_fbp(XctCheckWord *out, bool reset);
+int xct_check_read_adj(XctCheckWord *out, bool reset);
 #endif
 
 // SM count of the current device (cached per device).

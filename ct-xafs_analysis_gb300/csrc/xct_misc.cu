@@ -67,7 +67,7 @@ extern "C" int xct_check_report(xct_ctx *ctx, long long *count, int *site, long 
 #ifdef XCT_CHECKED
     XCT_CUDA_TRY(cudaSetDevice(ctx->device));
     XCT_CUDA_TRY(cudaDeviceSynchronize());
-    int (*const readers[])(XctCheckWord *, bool) = {xct_check_read_tiled, xct_check_read_fbp};
+    int (*const readers[])(XctCheckWord *, bool) = {xct_check_read_tiled, xct_check_read_fbp, xct_check_read_adj};
     long long total = 0;
     XctCheckWord first = {};
     for (auto rd : readers) {

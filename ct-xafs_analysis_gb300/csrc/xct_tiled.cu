@@ -390,692 +390,6 @@ __global__ void __launch_bounds__(FwdTile<S, T>::Threads, FwdTile<S, T>::MinBloc
                    (int)blockIdx.x / ntx, (int)blockIdx.y * chunk, chunk, smem_raw);
 }
 
-// ------------------------------------------------------------------- exact adjoint
-// A^T of the forward projector: img[t] = sum over samples of w_t(sample) * sino[th][X], with
-// the bilinear weights w00 = (1-fx)(1-fy), w10 = fx(1-fy), w01 = (1-fx)fy, w11 = fx fy of the
-// sample's 2x2 footprint.  A CTA owns a T x T texel tile; it visits every sample whose base
-// texel lies in [x0-1, x0+T) x [y0-1, y0+T) (exactly those whose footprint touches the
-// tile), scatters its four weighted values into a shared (T+2)^2 accumulator with shared
-// atomics (fixed-point integers per window of angles, below), and writes its own T x T
-// texels once -- no global atomics, no overlap between tiles.  grid: (ntx*nty tiles, 1, dN).
-// tile side: 64, or 32 when a launch of 64-texel tiles would leave fewer than three CTAs per
-// SM (one slice of 1024^2 makes only 256 tiles of 64)
-constexpr int kAdjT = 64, kAdjTSmall = 32;
-constexpr int kAdjWarps = kThreads / 32;  // one angle per warp and window
-
-// Accumulation: the warps take one angle each per window of kAdjWarps angles; within a window
-// the contributions are scattered as 32-bit fixed-point integers (shared-memory integer atomics
-// run ~6x the rate of float ones on this GPU), with a power-of-two scale chosen from the
-// window's largest |ray value| vmax: every contribution is at most vmax * scale <= 2^22, so
-// it converts to an integer with one add of 1.5*2^23 (its low bits hold the rounded value --
-// no conversion instruction), and no texel can overflow: it receives at most six taps per
-// angle (the half-open 2x2 cell around it holds at most five samples of the rotated unit
-// lattice, one more allowed for coordinate rounding), 48 * 2^22 < 2^28 per window.  After the
-// window every thread adds its texels' integers, unscaled, to the float total in window order
-// -- so the result does not depend on the order of the atomics -- and clears them.  One
-// integer unit is at most 2^-21 of vmax, each contribution rounds by at most 2^-22 of it; only
-// rays with |value| >= vmax * 2^-6 take the integer path (so each of their contributions
-// rounds by at most 2^-16 of the ray's value, below the weight error of float32 sample
-// coordinates), smaller ones -- and every ray of a window with a non-finite value or one above
-// 1e30 -- scatter float atomics, which keep full relative precision.
-// The angles are th = sub + k*step for k < nang (all: 0, 1, pa); with base non-null the
-// output is base + scale * (A^T sino) (a gradient step).
-template <int T>
-__global__ void __launch_bounds__(kThreads) adj_tiled_kernel(const float *__restrict__ sino,
-                                                             float *__restrict__ img,
-                                                             const float2 *__restrict__ trig, KGeom g, int ntx,
-                                                             int sub, int step, int nang,
-                                                             const float *__restrict__ base, float scale)
-{
-    constexpr int kAdjT = T, kAdjP = T + 2;  // this launch's tile side and pitch
-    __shared__ float accs[kAdjP * kAdjP];
-    __shared__ int acci[kAdjP * kAdjP];
-    __shared__ float wmax[kAdjWarps];
-    const int bx = blockIdx.x % ntx, by = blockIdx.x / ntx;
-    const int z = blockIdx.z;
-    const int x0 = bx * kAdjT, y0 = by * kAdjT;  // owned texels [x0, x0+T) x [y0, y0+T)
-    for (int i = threadIdx.x; i < kAdjP * kAdjP; i += kThreads) {
-        accs[i] = 0.0f;
-        acci[i] = 0;
-    }
-    __syncthreads();
-    const float *sn = sino + (size_t)z * g.pa * g.px;
-    // base texels whose footprint touches the tile
-    const float xlo = (float)(x0 - 1), xhi = (float)min(x0 + kAdjT, g.nx);
-    const float ylo = (float)(y0 - 1), yhi = (float)min(y0 + kAdjT, g.ny);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int D = g.depth;
-    for (int w0 = 0; w0 < nang; w0 += kAdjWarps) {
-        const bool active = w0 + warp < nang;
-        const int th = active ? sub + (w0 + warp) * step : 0;
-        float c = 1.0f, s = 0.0f;
-        int Xlo = 0, Xhi = -1;
-        if (active) {
-            const float2 cs = trig[th];
-            c = cs.x;
-            s = cs.y;
-            float pmin = 3.0e38f, pmax = -3.0e38f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float px_ = (q & 1) ? xhi + 2.0f : xlo - 2.0f;
-                const float py_ = (q & 2) ? yhi + 2.0f : ylo - 2.0f;
-                const float p = (px_ - g.hx) * c - (py_ - g.hy) * s + g.cx;
-                pmin = fminf(pmin, p);
-                pmax = fmaxf(pmax, p);
-            }
-            Xlo = max(0, (int)floorf(pmin) - 1);
-            Xhi = min(g.px - 1, (int)ceilf(pmax) + 1);
-        }
-        // the window's largest |ray value| (NaN and inf make it non-finite)
-        float m = 0.0f;
-        for (int X = Xlo + lane; X <= Xhi; X += 32) {
-            const float v = fabsf(__ldg(sn + (size_t)th * g.px + X));
-            m = (v == v && m == m) ? fmaxf(m, v) : __int_as_float(0x7fc00000);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float t = __shfl_xor_sync(0xffffffffu, m, o);
-            m = (t == t && m == m) ? fmaxf(m, t) : __int_as_float(0x7fc00000);
-        }
-        if (lane == 0) wmax[warp] = m;
-        __syncthreads();
-        float vmax = 0.0f;
-#pragma unroll
-        for (int k = 0; k < kAdjWarps; ++k) {
-            const float t = wmax[k];
-            vmax = (t == t && vmax == vmax) ? fmaxf(vmax, t) : __int_as_float(0x7fc00000);
-        }
-        // false for NaN and inf, and for finite windows above 1e30: those scatter float atomics
-        const bool fixed = vmax < 1.0e30f;
-        // scale = 2^(22 - e) with vmax < 2^e: every contribution is below 2^22 in magnitude
-        float scale = 0.0f, inv = 0.0f;
-        if (fixed && vmax > 0.0f) {
-            int e;
-            frexpf(vmax, &e);  // vmax < 2^e
-            e = max(e, -78);   // keep the scale <= 2^100 (a finite float)
-            scale = ldexpf(1.0f, 22 - e);
-            inv = ldexpf(1.0f, e - 22);
-        }
-        if (active && (!fixed || vmax > 0.0f)) {
-            // the forward projector's lane mapping: 8 consecutive rays, 4 lanes per ray taking
-            // every 4th sample of the ray's interval in the tile, whose four limits come from
-            // one boundary search per lane -- the same samples the forward visits
-            const float inv_s = 1.0f / s, inv_c = 1.0f / c;
-            const int ray = lane / kLanesPerRay, ph = lane % kLanesPerRay, grp = lane & ~(kLanesPerRay - 1);
-            const bool bound_x = ph < 2, upper = (ph & 1) != 0;
-            for (int base = Xlo; base <= Xhi; base += kRaysPerWarp) {
-                const int X = base + ray;
-                const bool live = X <= Xhi;
-                const float v = live ? __ldg(sn + (size_t)th * g.px + X) : 0.0f;
-                const float Xc = (float)X - g.cx;
-                const float ax = fmaf(Xc, c, g.hx);
-                const float ay = fmaf(Xc, -s, g.hy);
-                int lim = 0;
-                if (live) {
-                    const float a = bound_x ? ax : ay, sl = bound_x ? s : c, isl = bound_x ? inv_s : inv_c;
-                    const float lo = bound_x ? xlo : ylo, hi = bound_x ? xhi : yhi;
-                    if (sl != 0.0f) {
-                        const float bnd = ((sl > 0.0f) != upper) ? lo : hi;
-                        lim = first_true(bnd, a, sl, isl, g.hd, D);
-                    } else {
-                        lim = upper ? ((a >= lo && a < hi) ? D : 0) : 0;
-                    }
-                }
-                const int l0 = __shfl_sync(0xffffffffu, lim, grp + 0), l1 = __shfl_sync(0xffffffffu, lim, grp + 1);
-                const int l2 = __shfl_sync(0xffffffffu, lim, grp + 2), l3 = __shfl_sync(0xffffffffu, lim, grp + 3);
-                const int ya = max(l0, l2);
-                const int yb = (live && v != 0.0f) ? min(l1, l3) : ya;  // a zero ray contributes nothing
-                const float vs = v * scale;
-                const bool as_int = fixed && fabsf(v) >= vmax * 0.015625f;  // |v| >= vmax * 2^-6
-                for (int Y = ya + ph; Y < yb; Y += kLanesPerRay) {
-                    const float Yc = (float)Y - g.hd;
-                    const float x = fmaf(Yc, s, ax), y = fmaf(Yc, c, ay);
-                    const float fi = floorf(x), fj = floorf(y);
-                    const float fx = x - fi, fy = y - fj;
-                    const int col = (int)fi - (x0 - 1), row = (int)fj - (y0 - 1);
-                    const float gx = 1.0f - fx, gy = 1.0f - fy;
-                    if (!XCT_IN(row * kAdjP + col, 0, kAdjP * kAdjP - kAdjP - 2, XCT_SITE_ADJ)) continue;
-                    const int o = row * kAdjP + col;
-                    if (as_int) {
-                        // round(x) for |x| < 2^22: the low bits of x + 1.5*2^23
-                        const float p0 = vs * gy, p1 = vs * fy;
-                        atomicAdd(acci + o, __float_as_int(gx * p0 + kMagic) - 0x4B400000);
-                        atomicAdd(acci + o + 1, __float_as_int(fx * p0 + kMagic) - 0x4B400000);
-                        atomicAdd(acci + o + kAdjP, __float_as_int(gx * p1 + kMagic) - 0x4B400000);
-                        atomicAdd(acci + o + kAdjP + 1, __float_as_int(fx * p1 + kMagic) - 0x4B400000);
-                    } else {
-                        atomicAdd(accs + o, gx * gy * v);
-                        atomicAdd(accs + o + 1, fx * gy * v);
-                        atomicAdd(accs + o + kAdjP, gx * fy * v);
-                        atomicAdd(accs + o + kAdjP + 1, fx * fy * v);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        if (fixed && vmax > 0.0f) {
-            for (int i = threadIdx.x; i < kAdjP * kAdjP; i += kThreads) {
-                const int q = acci[i];
-                if (q != 0) {
-                    accs[i] += (float)q * inv;
-                    acci[i] = 0;
-                }
-            }
-        }
-        __syncthreads();  // the integers are clear and wmax may be rewritten
-    }
-    float *im = img + (size_t)z * g.nx * g.ny;
-    const float *bz = base ? base + (size_t)z * g.nx * g.ny : nullptr;
-    for (int i = threadIdx.x; i < kAdjT * kAdjT; i += kThreads) {
-        const int r = i / kAdjT, cc = i - r * kAdjT;
-        const int X = x0 + cc, Y = y0 + r;
-        if (X < g.nx && Y < g.ny) {
-            const float a = accs[(r + 1) * kAdjP + cc + 1];
-            const size_t o = (size_t)Y * g.nx + X;
-            im[o] = bz ? fmaf(scale, a, __ldg(bz + o)) : a;
-        }
-    }
-}
-
-// The exact adjoint over S slices of one geometry at once: adj_tiled_kernel's samples,
-// windows, fixed-point scales (one per slice and window) and epilogue, with each sample's
-// coordinates, weights and accumulator offset found once for the S slices.  Tile 32 texels;
-// the (T+2)^2 accumulators of a slice are kept at a pitch of 37 (a CPU model of the 32 lanes'
-// footprints over all angles gives 2.0 bank wavefronts per atomic instruction at this pitch,
-// 3.0 at pitch 34).  grid: (ntx*nty tiles, 1, dN / S slice groups); dynamic shared memory
-// AdjMs<S>::Smem.
-constexpr int kAdjMsT = 32, kAdjMsP = 37, kAdjMsR = kAdjMsT + 2;
-constexpr int kAdjMsSlices = 4;  // slices per adjoint group
-constexpr int kAdjMsN = kAdjMsR * kAdjMsP;  // accumulator entries per slice
-template <int S>
-struct AdjMs {
-    static constexpr size_t Smem = (size_t)S * kAdjMsN * (sizeof(float) + sizeof(int)) + kAdjWarps * S * sizeof(float);
-};
-
-template <int S>
-__global__ void __launch_bounds__(kThreads) adj_ms_kernel(const float *__restrict__ sino, float *__restrict__ img,
-                                                          const float2 *__restrict__ trig, KGeom g, int ntx, int sub,
-                                                          int step, int nang, const float *__restrict__ base,
-                                                          float scale_out)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float *accs = reinterpret_cast<float *>(smem_raw);
-    int *acci = reinterpret_cast<int *>(accs + S * kAdjMsN);
-    float *wmax = reinterpret_cast<float *>(acci + S * kAdjMsN);
-    const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
-    const int z0 = (int)blockIdx.z * S;
-    const size_t nprj = (size_t)g.pa * g.px, nimg = (size_t)g.nx * g.ny;
-    const int x0 = bx * kAdjMsT, y0 = by * kAdjMsT;  // owned texels [x0, x0+T) x [y0, y0+T)
-    for (int i = threadIdx.x; i < S * kAdjMsN; i += kThreads) {
-        accs[i] = 0.0f;
-        acci[i] = 0;
-    }
-    __syncthreads();
-    const float *sn = sino + (size_t)z0 * nprj;
-    // base texels whose footprint touches the tile
-    const float xlo = (float)(x0 - 1), xhi = (float)min(x0 + kAdjMsT, g.nx);
-    const float ylo = (float)(y0 - 1), yhi = (float)min(y0 + kAdjMsT, g.ny);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int D = g.depth;
-    for (int w0 = 0; w0 < nang; w0 += kAdjWarps) {
-        const bool active = w0 + warp < nang;
-        const int th = active ? sub + (w0 + warp) * step : 0;
-        float c = 1.0f, s = 0.0f;
-        int Xlo = 0, Xhi = -1;
-        if (active) {
-            const float2 cs = trig[th];
-            c = cs.x;
-            s = cs.y;
-            float pmin = 3.0e38f, pmax = -3.0e38f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float px_ = (q & 1) ? xhi + 2.0f : xlo - 2.0f;
-                const float py_ = (q & 2) ? yhi + 2.0f : ylo - 2.0f;
-                const float p = (px_ - g.hx) * c - (py_ - g.hy) * s + g.cx;
-                pmin = fminf(pmin, p);
-                pmax = fmaxf(pmax, p);
-            }
-            Xlo = max(0, (int)floorf(pmin) - 1);
-            Xhi = min(g.px - 1, (int)ceilf(pmax) + 1);
-        }
-        const float *row = sn + (size_t)th * g.px;
-        // each slice's largest |ray value| over the window (NaN and inf make it non-finite)
-        float m[S];
-#pragma unroll
-        for (int z = 0; z < S; ++z) m[z] = 0.0f;
-        for (int X = Xlo + lane; X <= Xhi; X += 32) {
-#pragma unroll
-            for (int z = 0; z < S; ++z) {
-                const float v = fabsf(__ldg(row + (size_t)z * nprj + X));
-                m[z] = (v == v && m[z] == m[z]) ? fmaxf(m[z], v) : __int_as_float(0x7fc00000);
-            }
-        }
-#pragma unroll
-        for (int z = 0; z < S; ++z) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float t = __shfl_xor_sync(0xffffffffu, m[z], o);
-                m[z] = (t == t && m[z] == m[z]) ? fmaxf(m[z], t) : __int_as_float(0x7fc00000);
-            }
-        }
-        if (lane == 0) {
-#pragma unroll
-            for (int z = 0; z < S; ++z) wmax[warp * S + z] = m[z];
-        }
-        __syncthreads();
-        float vmax[S], sc[S], inv[S];
-        unsigned fixed = 0;  // bit z: slice z's window takes the fixed-point path
-#pragma unroll
-        for (int z = 0; z < S; ++z) {
-            float vm = 0.0f;
-#pragma unroll
-            for (int k = 0; k < kAdjWarps; ++k) {
-                const float t = wmax[k * S + z];
-                vm = (t == t && vm == vm) ? fmaxf(vm, t) : __int_as_float(0x7fc00000);
-            }
-            vmax[z] = vm;
-            sc[z] = 0.0f;
-            inv[z] = 0.0f;
-            // false for NaN and inf, and for finite windows above 1e30: those scatter float atomics
-            if (vm < 1.0e30f && vm > 0.0f) {
-                int e;
-                frexpf(vm, &e);  // vmax < 2^e
-                e = max(e, -78);  // keep the scale <= 2^100 (a finite float)
-                sc[z] = ldexpf(1.0f, 22 - e);
-                inv[z] = ldexpf(1.0f, e - 22);
-                fixed |= 1u << z;
-            }
-        }
-        if (active) {
-            // the forward projector's lane mapping: 8 consecutive rays, 4 lanes per ray
-            const float inv_s = 1.0f / s, inv_c = 1.0f / c;
-            const int ray = lane / kLanesPerRay, ph = lane % kLanesPerRay, grp = lane & ~(kLanesPerRay - 1);
-            const bool bound_x = ph < 2, upper = (ph & 1) != 0;
-            for (int b0 = Xlo; b0 <= Xhi; b0 += kRaysPerWarp) {
-                const int X = b0 + ray;
-                const bool live = X <= Xhi;
-                float v[S];
-                bool any = false;
-#pragma unroll
-                for (int z = 0; z < S; ++z) {
-                    v[z] = live ? __ldg(row + (size_t)z * nprj + X) : 0.0f;
-                    any |= v[z] != 0.0f;
-                }
-                const float Xc = (float)X - g.cx;
-                const float ax = fmaf(Xc, c, g.hx);
-                const float ay = fmaf(Xc, -s, g.hy);
-                int lim = 0;
-                if (live) {
-                    const float a = bound_x ? ax : ay, sl = bound_x ? s : c, isl = bound_x ? inv_s : inv_c;
-                    const float lo = bound_x ? xlo : ylo, hi = bound_x ? xhi : yhi;
-                    if (sl != 0.0f) {
-                        const float bnd = ((sl > 0.0f) != upper) ? lo : hi;
-                        lim = first_true(bnd, a, sl, isl, g.hd, D);
-                    } else {
-                        lim = upper ? ((a >= lo && a < hi) ? D : 0) : 0;
-                    }
-                }
-                const int l0 = __shfl_sync(0xffffffffu, lim, grp + 0), l1 = __shfl_sync(0xffffffffu, lim, grp + 1);
-                const int l2 = __shfl_sync(0xffffffffu, lim, grp + 2), l3 = __shfl_sync(0xffffffffu, lim, grp + 3);
-                const int ya = max(l0, l2);
-                const int yb = (live && any) ? min(l1, l3) : ya;  // a ray zero in every slice adds nothing
-                float vs[S];
-                unsigned as_int = 0;  // bit z: |v| >= vmax * 2^-6 in a fixed-point window
-#pragma unroll
-                for (int z = 0; z < S; ++z) {
-                    vs[z] = v[z] * sc[z];
-                    if (((fixed >> z) & 1u) && fabsf(v[z]) >= vmax[z] * 0.015625f) as_int |= 1u << z;
-                }
-                for (int Y = ya + ph; Y < yb; Y += kLanesPerRay) {
-                    const float Yc = (float)Y - g.hd;
-                    const float x = fmaf(Yc, s, ax), y = fmaf(Yc, c, ay);
-                    const float fi = floorf(x), fj = floorf(y);
-                    const float fx = x - fi, fy = y - fj;
-                    const int col = (int)fi - (x0 - 1), rr = (int)fj - (y0 - 1);
-                    const float gx = 1.0f - fx, gy = 1.0f - fy;
-                    if (!XCT_IN(rr * kAdjMsP + col, 0, (kAdjMsR - 2) * kAdjMsP + kAdjMsR - 2, XCT_SITE_ADJ)) continue;
-                    const int o = rr * kAdjMsP + col;
-#pragma unroll
-                    for (int z = 0; z < S; ++z) {
-                        int *ai = acci + z * kAdjMsN + o;
-                        float *af = accs + z * kAdjMsN + o;
-                        if ((as_int >> z) & 1u) {
-                            // round(x) for |x| < 2^22: the low bits of x + 1.5*2^23
-                            const float p0 = vs[z] * gy, p1 = vs[z] * fy;
-                            atomicAdd(ai, __float_as_int(gx * p0 + kMagic) - 0x4B400000);
-                            atomicAdd(ai + 1, __float_as_int(fx * p0 + kMagic) - 0x4B400000);
-                            atomicAdd(ai + kAdjMsP, __float_as_int(gx * p1 + kMagic) - 0x4B400000);
-                            atomicAdd(ai + kAdjMsP + 1, __float_as_int(fx * p1 + kMagic) - 0x4B400000);
-                        } else if (v[z] != 0.0f) {
-                            atomicAdd(af, gx * gy * v[z]);
-                            atomicAdd(af + 1, fx * gy * v[z]);
-                            atomicAdd(af + kAdjMsP, gx * fy * v[z]);
-                            atomicAdd(af + kAdjMsP + 1, fx * fy * v[z]);
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int z = 0; z < S; ++z) {
-            if ((fixed >> z) & 1u) {
-                for (int i = threadIdx.x; i < kAdjMsN; i += kThreads) {
-                    const int q = acci[z * kAdjMsN + i];
-                    if (q != 0) {
-                        accs[z * kAdjMsN + i] += (float)q * inv[z];
-                        acci[z * kAdjMsN + i] = 0;
-                    }
-                }
-            }
-        }
-        __syncthreads();  // the integers are clear and wmax may be rewritten
-    }
-    for (int z = 0; z < S; ++z) {
-        float *im = img + (size_t)(z0 + z) * nimg;
-        const float *bz = base ? base + (size_t)(z0 + z) * nimg : nullptr;
-        for (int i = threadIdx.x; i < kAdjMsT * kAdjMsT; i += kThreads) {
-            const int r = i / kAdjMsT, cc = i - r * kAdjMsT;
-            const int X = x0 + cc, Y = y0 + r;
-            if (X < g.nx && Y < g.ny) {
-                const float a = accs[z * kAdjMsN + (r + 1) * kAdjMsP + cc + 1];
-                const size_t o = (size_t)Y * g.nx + X;
-                im[o] = bz ? fmaf(scale_out, a, __ldg(bz + o)) : a;
-            }
-        }
-    }
-}
-
-// The exact adjoint over eight or ten slices as a gather, without atomics.  Every sample (ray X,
-// index Y) of the forward projector has one base texel (floor of its coordinates); its value
-// v goes to that base texel's four footprint texels with the weights gx gy, fx gy, gx fy,
-// fx fy.  A thread owns one base texel (i, j) and keeps four accumulators per slice -- the
-// parts its samples give to (i, j), (i+1, j), (i, j+1), (i+1, j+1) -- so each sample is
-// handled by exactly one thread.  Per angle the thread finds its samples: a half-open unit
-// square holds at most two points of the rotated unit sample lattice, which lie on the at
-// most two rays whose lattice coordinate is within 0.717 of the square's centre, each at
-// most two sample indices within 0.717 of the centre's projection on the ray; each of those
-// four candidates is evaluated with the forward projector's own arithmetic (fma
-// coordinates, round-down floor) and kept when its base texel is (i, j), the ray is on the
-// detector and the index within [0, D).  A CTA owns 32 x BY base texels (BY = 16 for eight
-// slices, 20 for ten) and writes the 31 x (BY - 1) texels whose four base texels it holds,
-// texel (i, j) = A00(i, j) + A10(i-1, j) + A01(i, j-1) + A11(i-1, j-1), after staging the
-// four parts in shared memory.
-// The rays' values of 16 angles at a time are staged by asynchronous copies into one of two
-// windows: the next chunk's copies run while this chunk is accumulated.  Most squares hold
-// one sample per angle, about 9 % two and 9 % none, so a warp whose lanes each added all
-// their samples at once would run two accumulation passes at almost every angle; with ten
-// slices a second sample instead waits in a four-slot queue per thread in shared memory
-// (window address and fractions) and the queues are emptied at the end of the chunk -- about
-// 1.2 passes per angle instead of 1.8.  Float sums in a fixed order given by the geometry:
-// deterministic, and no fixed-point rounding.
-constexpr int kAdjGBX = 32;                          // base texels per CTA row
-constexpr int kAdjGW = 44;  // staged rays per angle (a 32 x 20 block needs at most 43)
-constexpr int kAdjGChunk = 16;                       // angles per staging pass
-template <int S>
-struct AdjG {
-    // base texel rows per CTA (one thread per base texel): 16 at two CTAs per SM (eight
-    // slices, 64 registers), 20 at one (ten slices, 94 registers)
-    static constexpr int BY = S <= 8 ? 16 : 20;
-    static constexpr int Threads = kAdjGBX * BY;
-    static constexpr unsigned QStride = 16u * Threads;  // bytes between a queue's slots
-    // two windows: [slice pair][angle][ray] of float2, then the queues: [slot][thread] of
-    // (window address, fx, fy); later the parts: [corner][slice][thread]; three slots of
-    // (cos, sin) and first staged ray per angle
-    static constexpr unsigned PairBytes = (unsigned)(kAdjGChunk * kAdjGW * 8);
-    static constexpr unsigned WinBytes = (unsigned)(S / 2) * PairBytes;
-    static constexpr size_t CombBytes = (size_t)4 * S * Threads * 4;
-    // queued samples per thread: four where the registers allow (one CTA per SM); none at
-    // two CTAs per SM, whose 64 registers a thread would then exceed
-    static constexpr int Queue = S > 8 ? 4 : 0;
-    static constexpr size_t QueueBytes = (size_t)Queue * QStride;
-    static constexpr size_t SlotBytes = (size_t)3 * kAdjGChunk * 12;
-    static constexpr size_t Front = 2 * (size_t)WinBytes + QueueBytes;
-    static constexpr size_t Smem = (Front > CombBytes ? Front : CombBytes) + SlotBytes;
-};
-
-__device__ __forceinline__ f2x lds_f2x(unsigned addr)
-{
-    f2x v;
-    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr));
-    return v;
-}
-
-// A queued sample: window address and fractions (fx, fy) in one 16-byte slot.
-__device__ __forceinline__ void sts_q(unsigned addr, unsigned ad, f2x fr)
-{
-    asm volatile("{ .reg .b32 lo, hi; mov.b64 {lo, hi}, %2; st.shared.v4.b32 [%0], {%1, lo, hi, %1}; }"
-                 :: "r"(addr), "r"(ad), "l"(fr) : "memory");
-}
-__device__ __forceinline__ void lds_q(unsigned addr, unsigned &ad, f2x &fr)
-{
-    asm volatile("{ .reg .b32 lo, hi, pad; ld.shared.v4.b32 {%0, lo, hi, pad}, [%2]; mov.b64 %1, {lo, hi}; }"
-                 : "=r"(ad), "=l"(fr) : "r"(addr) : "memory");
-}
-
-// S (even) slices per CTA; the library launches S = 8 and S = 10 (one CTA per SM).
-template <int S>
-__global__ void __launch_bounds__(AdjG<S>::Threads, S <= 8 ? 2 : 1) adj_gather_kernel(const float *__restrict__ sino,
-                                                                     float *__restrict__ img,
-                                                                     const float2 *__restrict__ trig, KGeom g,
-                                                                     int ntx, int sub, int step, int nang,
-                                                                     const float *__restrict__ base, float scale_out)
-{
-    constexpr int P = S / 2;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float *part = reinterpret_cast<float *>(smem_raw);  // the window, later the parts
-    float2 *scs = reinterpret_cast<float2 *>(smem_raw + AdjG<S>::Smem - AdjG<S>::SlotBytes);
-    int *sxw = reinterpret_cast<int *>(scs + 3 * kAdjGChunk);
-    const int tx = threadIdx.x % kAdjGBX, ty = threadIdx.x / kAdjGBX;
-    const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
-    const int z0 = (int)blockIdx.z * S;
-    const size_t nprj = (size_t)g.pa * g.px, nimg = (size_t)g.nx * g.ny;
-    const float *sz = sino + (size_t)z0 * nprj;
-    // base texels [bi0, bi0 + 32) x [bj0, bj0 + 16); output texels from bi0 + 1, bj0 + 1
-    const int bi0 = bx * (kAdjGBX - 1) - 1, bj0 = by * (AdjG<S>::BY - 1) - 1;
-    const int i = bi0 + tx, j = bj0 + ty;
-    const int ibits = i + XCT_FLOOR_BIAS, jbits = j + XCT_FLOOR_BIAS;
-    const float ci = (float)i + 0.5f, cj = (float)j + 0.5f;  // the square's centre
-    const float di = ci - g.hx, dj = cj - g.hy;
-    const int D = g.depth;
-    const unsigned wbase = (unsigned)__cvta_generic_to_shared(part);
-    const f2x MM = f2_pack(kMagic, kMagic), one2 = f2_pack(1.0f, 1.0f);
-    const f2x hxy = f2_pack(g.hx, g.hy);
-    f2x acc[4][P];  // [corner 00, 10, 01, 11][slice pair]
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int h = 0; h < P; ++h) acc[q][h] = 0ull;
-
-    // one sample: fractions (fx, fy) of its base texel, window byte address ad of its ray;
-    // the four bilinear weights (gx gy, fx gy, gx fy, fx fy) times the slices' ray values
-    const f2x bxy = f2_pack(__int_as_float(ibits) - kMagic, __int_as_float(jbits) - kMagic);
-    auto add = [&](unsigned ad, f2x fr, unsigned wb) {
-        const f2x gr = f2_sub(one2, fr);
-        float fx, fy, gx, gy;
-        f2_unpack(fr, fx, fy);
-        f2_unpack(gr, gx, gy);
-        const float w[4] = {gx * gy, fx * gy, gx * fy, fx * fy};
-        if (!XCT_IN(ad, wb, wb + AdjG<S>::WinBytes - 8, XCT_SITE_ADJ)) return;
-        f2x v[P];
-#pragma unroll
-        for (int h = 0; h < P; ++h) v[h] = lds_f2x(ad + (unsigned)h * AdjG<S>::PairBytes);
-#pragma unroll
-        for (int cq = 0; cq < 4; ++cq) {
-            const f2x ww = f2_pack(w[cq], w[cq]);
-#pragma unroll
-            for (int h = 0; h < P; ++h) acc[cq][h] = f2_fma(ww, v[h], acc[cq][h]);
-        }
-    };
-    // this thread's queue of samples left for the end of the chunk: slot i at qb + i * stride
-    const unsigned qb = wbase + 2u * AdjG<S>::WinBytes + 16u * threadIdx.x;
-    int qn = 0;
-
-    // Software pipeline over chunks of 16 angles: the rays of chunk ch + 1 are copied into the
-    // other window while chunk ch is accumulated; the angles' (cos, sin) and first staged ray
-    // sit in three slots (chunks ch, ch + 1, ch + 2), the (cos, sin) of chunk ch + 3 in the
-    // registers of threads 0..15.
-    const int nch = (nang + kAdjGChunk - 1) / kAdjGChunk;
-    auto trig_of = [&](int ch) -> float2 {
-        const int a = ch * kAdjGChunk + (int)threadIdx.x;
-        return (ch < nch && (int)threadIdx.x < kAdjGChunk && a < nang) ? __ldg(trig + sub + a * step)
-                                                                        : make_float2(0.0f, 0.0f);
-    };
-    auto prep = [&](int ch, float2 cs) {
-        if (ch >= nch || (int)threadIdx.x >= kAdjGChunk) return;
-        const int at = (ch % 3) * kAdjGChunk + (int)threadIdx.x;
-        scs[at] = cs;
-        // rays whose lattice coordinate meets the block's base squares
-        float umin = 3.0e38f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float px_ = (float)(bi0 + ((q & 1) ? kAdjGBX : 0)) - g.hx;
-            const float py_ = (float)(bj0 + ((q & 2) ? AdjG<S>::BY : 0)) - g.hy;
-            umin = fminf(umin, px_ * cs.x - py_ * cs.y + g.cx);
-        }
-        sxw[at] = (int)floorf(umin) - 2;
-    };
-    // window (pair p, angle k, ray sxw + r) = (slice 2p, slice 2p + 1), 0 off the detector
-    auto stage = [&](int ch) {
-        if (ch >= nch) return;
-        const int k0 = ch * kAdjGChunk, kn = min(kAdjGChunk, nang - k0), sl = (ch % 3) * kAdjGChunk;
-        const unsigned wb = wbase + (unsigned)(ch & 1) * AdjG<S>::WinBytes;
-        for (int e = threadIdx.x; e < kn * S * kAdjGW; e += AdjG<S>::Threads) {
-            const int r = e % kAdjGW, t2 = e / kAdjGW;
-            const int z = t2 % S, k = t2 / S;
-            const int X = sxw[sl + k] + r;
-            const float *row = sz + (size_t)z * nprj + (size_t)(sub + (k0 + k) * step) * g.px;
-            const bool in = (unsigned)X < (unsigned)g.px;
-            const unsigned dst = wb + (unsigned)(z >> 1) * AdjG<S>::PairBytes + 8u * (unsigned)(k * kAdjGW + r) +
-                                 4u * (unsigned)(z & 1);
-            cp_async4(dst, in ? (const void *)(row + X) : (const void *)row, in ? 4u : 0u);
-        }
-    };
-    prep(0, trig_of(0));
-    prep(1, trig_of(1));
-    float2 csr = trig_of(2);
-    __syncthreads();
-    stage(0);
-    for (int ch = 0; ch < nch; ++ch) {
-        // this chunk's copies have landed; every thread is past chunk ch - 1, whose window
-        // and slot are reused below
-        cp_async_wait_all();
-        __syncthreads();
-        prep(ch + 2, csr);
-        csr = trig_of(ch + 3);
-        stage(ch + 1);
-        const int k0 = ch * kAdjGChunk, kn = min(kAdjGChunk, nang - k0), sl = (ch % 3) * kAdjGChunk;
-        const unsigned wb = wbase + (unsigned)(ch & 1) * AdjG<S>::WinBytes;
-        for (int k = 0; k < kn; ++k) {
-            const float c = scs[sl + k].x, s = scs[sl + k].y;
-            const f2x cs2 = f2_pack(c, -s), sc2 = f2_pack(s, c);
-            const unsigned wk = wb + 8u * (unsigned)(k * kAdjGW - sxw[sl + k]);
-            // the candidates: rays Xa, Xa + 1 (lattice coordinate of the cell centre u0 - 0.717
-            // and up); on each, indices Ya, Ya + 1 (the centre's coordinate along the rays, w0,
-            // is the same on every ray)
-            const float u0 = fmaf(di, c, fmaf(-dj, s, g.cx));
-            const float w0 = fmaf(di, s, dj * c) + g.hd;
-            const int Xa = (xct_floor_bits(u0 - 0.717f) - XCT_FLOOR_BIAS) + 1;
-            const int Ya = (xct_floor_bits(w0 - 0.717f) - XCT_FLOOR_BIAS) + 1;
-            // Y - hd is exact (hd is a multiple of 0.5), so the second index is the first + 1
-            const float Yc0 = (float)Ya - g.hd;
-            const f2x yy[2] = {f2_pack(Yc0, Yc0), f2_pack(Yc0 + 1.0f, Yc0 + 1.0f)};
-            const bool yin[2] = {(unsigned)Ya < (unsigned)D, (unsigned)(Ya + 1) < (unsigned)D};
-            f2x cxy[4];
-            unsigned valid = 0;
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
-                const int X = Xa + a;
-                const float Xc = (float)X - g.cx;
-                const f2x axy = f2_fma(f2_pack(Xc, Xc), cs2, hxy);  // (ax, ay) as the forward
-                const bool xin = (unsigned)X < (unsigned)g.px;
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const f2x xy = f2_fma(yy[b], sc2, axy);  // (x, y) as the forward
-                    int xb, yb;
-                    f2_unpack_bits(f2_add_rd(xy, MM), xb, yb);
-                    const int q = 2 * a + b;
-                    cxy[q] = xy;
-                    if (xb == ibits && yb == jbits && xin && yin[b]) valid |= 1u << q;
-                }
-            }
-            // a unit square holds at most two samples.  The first is added now; a second one
-            // (and, never seen but kept for float-rounded coordinates at the square's corners,
-            // any further) waits in the queue, or is added now when the queue is full
-            unsigned now = valid & (0u - valid), rest = valid ^ now;
-            while (rest != 0 && qn < AdjG<S>::Queue) {
-                const int q = __ffs(rest) - 1;
-                rest &= rest - 1;
-                const f2x xy = q == 1 ? cxy[1] : q == 2 ? cxy[2] : cxy[3];
-                const int X = Xa + (q >> 1);
-                sts_q(qb + (unsigned)qn * AdjG<S>::QStride, wk + 8u * (unsigned)X, f2_sub(xy, bxy));
-                ++qn;
-            }
-            now |= rest;
-            while (now != 0) {
-                const int q = __ffs(now) - 1;
-                now &= now - 1;
-                const f2x xy = q == 0 ? cxy[0] : q == 1 ? cxy[1] : q == 2 ? cxy[2] : cxy[3];
-                const int X = Xa + (q >> 1);
-                add(wk + 8u * (unsigned)X, f2_sub(xy, bxy), wb);
-            }
-        }
-        // the queued samples, while this chunk's window is still in place
-        for (int i = 0; i < qn; ++i) {
-            unsigned ad;
-            f2x fr;
-            lds_q(qb + (unsigned)i * AdjG<S>::QStride, ad, fr);
-            add(ad, fr, wb);
-        }
-        qn = 0;
-    }
-    // the parts: part[corner][slice][thread]
-    __syncthreads();
-#pragma unroll
-    for (int cq = 0; cq < 4; ++cq)
-#pragma unroll
-        for (int h = 0; h < P; ++h) {
-            float a0, a1;
-            f2_unpack(acc[cq][h], a0, a1);
-            part[(cq * S + 2 * h) * AdjG<S>::Threads + threadIdx.x] = a0;
-            part[(cq * S + 2 * h + 1) * AdjG<S>::Threads + threadIdx.x] = a1;
-        }
-    __syncthreads();
-    if (tx == 0 || ty == 0 || i >= g.nx || j >= g.ny) return;
-    const int t = threadIdx.x;
-#pragma unroll
-    for (int z = 0; z < S; ++z) {
-        const float a = part[(0 * S + z) * AdjG<S>::Threads + t] + part[(1 * S + z) * AdjG<S>::Threads + t - 1] +
-                        part[(2 * S + z) * AdjG<S>::Threads + t - kAdjGBX] +
-                        part[(3 * S + z) * AdjG<S>::Threads + t - kAdjGBX - 1];
-        const size_t o = (size_t)(z0 + z) * nimg + (size_t)j * g.nx + i;
-        img[o] = base ? fmaf(scale_out, a, __ldg(base + o)) : a;
-    }
-}
-
-// Launch of adj_gather_kernel<S> over `groups` groups of S slices (its shared memory opted in
-// once per device).
-template <int S>
-static int launch_adj_gather(const KGeom &g, const float2 *trig, const float *sino, float *img, int groups, int sub,
-                             int step, int nang, const float *base, float scale, cudaStream_t st)
-{
-    static std::atomic<bool> done[64];
-    int dev = 0;
-    XCT_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return xct_fail(XCT_E_INVALID, "device index out of range");
-    if (!done[dev].load(std::memory_order_acquire)) {
-        XCT_CUDA_TRY(cudaFuncSetAttribute((const void *)adj_gather_kernel<S>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AdjG<S>::Smem));
-        done[dev].store(true, std::memory_order_release);
-    }
-    const int ntx = (g.nx + kAdjGBX - 2) / (kAdjGBX - 1), nty = (g.ny + AdjG<S>::BY - 2) / (AdjG<S>::BY - 1);
-    adj_gather_kernel<S><<<dim3(ntx * nty, 1, groups), AdjG<S>::Threads, AdjG<S>::Smem, st>>>(sino, img, trig, g, ntx, sub,
-                                                                                         step, nang, base, scale);
-    g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-    XCT_CUDA_TRY(cudaGetLastError());
-    return XCT_OK;
-}
-
 // acc -> OSEM1 ratio (meas != nullptr) or raw projection, rows th = sub + k*step; clears acc.
 __global__ void fwd_finalize_kernel(double *acc, const float *meas, float *out, KGeom g, int sub, int step, int nrows)
 {
@@ -1729,89 +1043,6 @@ int launch_fwd_tiled(const KGeom &g, const float2 *trig, const float *img, const
     int rc = launch_fwd_tiled_main(g, trig, img, acc, dN, sub, step, nrows, st);
     if (rc) return rc;
     return launch_fwd_finalize(g, meas, out, acc, dN, sub, step, nrows, st);
-}
-
-int launch_adj_tiled(const KGeom &g, const float2 *trig, const float *sino, float *img, int dN, cudaStream_t st)
-{
-    return launch_adj_subset(g, trig, sino, img, dN, 0, 1, g.pa, nullptr, 0.0f, st);
-}
-
-// Launch of adj_ms_kernel<S> over groups of S slices (its shared memory opted in once per
-// device).
-template <int S>
-static int launch_adj_ms(const KGeom &g, const float2 *trig, const float *sino, float *img, int groups, int sub,
-                         int step, int nang, const float *base, float scale, cudaStream_t st)
-{
-    static std::atomic<bool> done[64];
-    int dev = 0;
-    XCT_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return xct_fail(XCT_E_INVALID, "device index out of range");
-    if (!done[dev].load(std::memory_order_acquire)) {
-        XCT_CUDA_TRY(cudaFuncSetAttribute((const void *)adj_ms_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)AdjMs<S>::Smem));
-        done[dev].store(true, std::memory_order_release);
-    }
-    const int ntx = (g.nx + kAdjMsT - 1) / kAdjMsT, nty = (g.ny + kAdjMsT - 1) / kAdjMsT;
-    adj_ms_kernel<S><<<dim3(ntx * nty, 1, groups), kThreads, AdjMs<S>::Smem, st>>>(sino, img, trig, g, ntx, sub, step,
-                                                                                  nang, base, scale);
-    g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-    XCT_CUDA_TRY(cudaGetLastError());
-    return XCT_OK;
-}
-
-int launch_adj_subset(const KGeom &g, const float2 *trig, const float *sino, float *img, int dN, int sub, int step,
-                      int nang, const float *base, float scale, cudaStream_t st)
-{
-    if (dN <= 0) return XCT_OK;
-    // with the slice-interleaved kernels on, groups of eight or ten slices take the gather
-    // form (its candidate search is shared by the group; for fewer slices the scatter forms
-    // cost less) -- the most groups of ten that leave a multiple of eight (a slice costs less
-    // in a group of ten), then groups of eight -- and groups of four the scatter form with
-    // shared sample work
-    if (g.ms_chunk > 0 && dN >= 8) {
-        const size_t np = (size_t)g.pa * g.px, ni = (size_t)g.nx * g.ny;
-        int rc = XCT_OK;
-        auto advance = [&](int n) {
-            sino += n * np;
-            img += n * ni;
-            if (base) base += n * ni;
-            dN -= n;
-        };
-        int tens = dN / 10;
-        while (tens > 0 && (dN - 10 * tens) % 8 != 0) --tens;
-        if (tens > 0) {
-            if ((rc = launch_adj_gather<10>(g, trig, sino, img, tens, sub, step, nang, base, scale, st))) return rc;
-            advance(tens * 10);
-        }
-        const int groups = dN / 8;
-        if (groups > 0) {
-            if ((rc = launch_adj_gather<8>(g, trig, sino, img, groups, sub, step, nang, base, scale, st))) return rc;
-            advance(groups * 8);
-        }
-        if (dN == 0) return XCT_OK;
-    }
-    if (g.ms_chunk > 0 && dN >= kAdjMsSlices) {
-        const int groups = dN / kAdjMsSlices, ms = groups * kAdjMsSlices;
-        const int rc = launch_adj_ms<kAdjMsSlices>(g, trig, sino, img, groups, sub, step, nang, base, scale, st);
-        if (rc || ms == dN) return rc;
-        sino += (size_t)ms * g.pa * g.px;
-        img += (size_t)ms * g.nx * g.ny;
-        if (base) base += (size_t)ms * g.nx * g.ny;
-        dN -= ms;
-    }
-    const long long big = (long long)((g.nx + kAdjT - 1) / kAdjT) * ((g.ny + kAdjT - 1) / kAdjT) * dN;
-    if (big >= 3LL * device_sm_count()) {
-        const int ntx = (g.nx + kAdjT - 1) / kAdjT, nty = (g.ny + kAdjT - 1) / kAdjT;
-        adj_tiled_kernel<kAdjT><<<dim3(ntx * nty, 1, dN), kThreads, 0, st>>>(sino, img, trig, g, ntx, sub, step, nang,
-                                                                            base, scale);
-    } else {
-        const int ntx = (g.nx + kAdjTSmall - 1) / kAdjTSmall, nty = (g.ny + kAdjTSmall - 1) / kAdjTSmall;
-        adj_tiled_kernel<kAdjTSmall><<<dim3(ntx * nty, 1, dN), kThreads, 0, st>>>(sino, img, trig, g, ntx, sub, step,
-                                                                                  nang, base, scale);
-    }
-    g_xct_launches.fetch_add(1, std::memory_order_relaxed);
-    XCT_CUDA_TRY(cudaGetLastError());
-    return XCT_OK;
 }
 
 // SM count of the current device, cached per device (152 if it cannot be read).
