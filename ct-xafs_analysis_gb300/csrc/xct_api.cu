@@ -1095,14 +1095,12 @@ static int cs_loop(xct_plan *p, int dN, const float *d_sino, float *d_img, const
     const KGeom &g = p->kg;
     const size_t nimg = (size_t)g.nx * g.ny, nb = (size_t)p->g.max_batch;
     if (!p->d_cs) {
-        cudaError_t e = cudaMalloc(&p->d_cs, sizeof(float) * 3 * nb * nimg);
+        cudaError_t e = cudaMalloc(&p->d_cs, sizeof(float) * nb * nimg);
         if (e != cudaSuccess) {
             p->d_cs = nullptr;
             return xct_cuda_fail(e, "cudaMalloc compressed-sensing buffers");
         }
     }
-    float *w = p->d_cs, *beta = p->d_cs + nb * nimg, *xn = p->d_cs + 2 * nb * nimg;
-    const size_t bytes = sizeof(float) * dN * nimg;
     const float *meas = d_sino;
     if (correct && p->g.correction_mode > 0) {
         int rc = launch_sino_correction(g, d_sino, p->d_corr, p->d_corr_ang, p->d_corr_bin, p->g.correction_mode, dN,
@@ -1110,26 +1108,24 @@ static int cs_loop(xct_plan *p, int dN, const float *d_sino, float *d_img, const
         if (rc) return rc;
         meas = p->d_corr;
     }
-    XCT_CUDA_TRY(cudaMemcpyAsync(w, d_img, bytes, cudaMemcpyDeviceToDevice, st));  // w = x (:344)
-    XCT_CUDA_TRY(cudaMemsetAsync(beta, 0, bytes, st));                             // beta = 0 (:342)
-    bool first = true;
+    // the proximal step writes the other of two images, so the loop alternates between them
+    float *cur = d_img, *other = p->d_cs;
     for (int i = 0; i < it; ++i)
         for (int k = 0; k < p->g.ss; ++k) {
-            const int s = sub[k];
-            int rc;
-            if (first) {
-                rc = launch_ista3d(d_img, xn, g.nx, g.ny, dN, lambda, p->ctx->sm_count, st);
-                first = false;
-            } else {
-                // the OS-EM step of the two halves on two streams; the proximal step after the
-                // join couples neighbouring slices
-                rc = dN >= 2 ? subset_step_split(p, dN, meas, d_img, s, st)
-                             : subset_step(p, dN, meas, d_img, p->d_ratio, p->d_acc, s, st);
-                if (!rc) rc = launch_fista3d(w, w, d_img, beta, xn, g.nx, g.ny, dN, lambda, p->ctx->sm_count, st);
-            }
+            const bool first = i == 0 && k == 0;
+            int rc = XCT_OK;
+            // the OS-EM step (the first one's result is discarded by the reference's order of
+            // operations); halves on two streams where that pays, joined before the proximal step, which
+            // couples neighbouring slices
+            if (!first)
+                rc = dN >= 2 ? subset_step_split(p, dN, meas, cur, sub[k], st)
+                             : subset_step(p, dN, meas, cur, p->d_ratio, p->d_acc, sub[k], st);
+            if (!rc) rc = launch_prox(cur, other, g.nx, g.ny, dN, lambda, first, st);
             if (rc) return rc;
-            XCT_CUDA_TRY(cudaMemcpyAsync(d_img, xn, bytes, cudaMemcpyDeviceToDevice, st));
+            std::swap(cur, other);
         }
+    if (cur != d_img)
+        XCT_CUDA_TRY(cudaMemcpyAsync(d_img, cur, sizeof(float) * dN * nimg, cudaMemcpyDeviceToDevice, st));
     return XCT_OK;
 }
 

@@ -14,15 +14,16 @@
 #include <algorithm>
 
 #include "xct_internal.h"
+#include "xct_launch.cuh"
 
 namespace {
 
-__device__ __forceinline__ float texz(const float *__restrict__ vz, int nx, int ny, int X, int Y)
+__device__ __forceinline__ float texz(const float *vz, int nx, int ny, int X, int Y)
 {
-    return (X >= 0 && Y >= 0 && X < nx && Y < ny) ? __ldg(vz + (size_t)Y * nx + X) : 0.0f;
+    return (X >= 0 && Y >= 0 && X < nx && Y < ny) ? vz[(size_t)Y * nx + X] : 0.0f;
 }
 
-__device__ __forceinline__ float cs_select(const float *__restrict__ v, int nx, int ny, int dN, int X, int Y, int Z,
+__device__ __forceinline__ float cs_select(const float *v, int nx, int ny, int dN, int X, int Y, int Z,
                                            float lambda)
 {
     const size_t m = (size_t)nx * ny;
@@ -32,9 +33,9 @@ __device__ __forceinline__ float cs_select(const float *__restrict__ v, int nx, 
     nb[1] = texz(vz, nx, ny, X - 1, Y);
     nb[2] = texz(vz, nx, ny, X, Y + 1);
     nb[3] = texz(vz, nx, ny, X, Y - 1);
-    nb[4] = __ldg(v + (size_t)min(Z + 1, dN - 1) * m + (size_t)Y * nx + X);
-    nb[5] = __ldg(v + (size_t)Y * nx + X);
-    const float vi = __ldg(vz + (size_t)Y * nx + X);
+    nb[4] = v[(size_t)min(Z + 1, dN - 1) * m + (size_t)Y * nx + X];
+    nb[5] = v[(size_t)Y * nx + X];
+    const float vi = vz[(size_t)Y * nx + X];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         const float img1 = nb[i];
@@ -58,6 +59,64 @@ __device__ __forceinline__ float cs_select(const float *__restrict__ v, int nx, 
 #pragma unroll
     for (int i = 0; i < 12; ++i) x = (vi < rng[i]) ? cnd[i + 1] : x;
     return x;
+}
+
+// The proximal step alone (x_new from v; First: ISTA3D's floor of 1e-6 and NaN -> 1e-6), for the
+// compressed-sensing OS-EM, whose momentum image and beta never reach an output (FISTA_OSEM_execution
+// feeds its own w back as x_t, GPU.cpp:243-405, and reads neither).  grid: (ceil(nx/32), ceil(ny/8), dN),
+// 256 threads.  The neighbours go through a 12-exchange sorting network; where one of the six or their sum
+// is not finite, through the reference's exchange loop, whose order among NaNs it keeps.  HBM- or L2-bound:
+// 10 slices of 512^2 take 6 us (the general FISTA3D kernel and the copy of its result back took 32).
+template <bool First>
+__global__ void __launch_bounds__(256) prox_kernel(const float *v, float *x_new, int nx, int ny, int dN, float lambda)
+{
+    const int X = (int)blockIdx.x * 32 + (int)(threadIdx.x & 31), Y = (int)blockIdx.y * 8 + (int)(threadIdx.x >> 5);
+    const int Z = blockIdx.z;
+    xct_grid_wait();
+    xct_grid_trigger();
+    if (X >= nx || Y >= ny) return;
+    const size_t m = (size_t)nx * ny, o = (size_t)Y * nx + X;
+    const float *p = v + (size_t)Z * m + o;
+    const float vi = p[0];
+    float a = X + 1 < nx ? p[1] : 0.0f, b = X > 0 ? p[-1] : 0.0f;
+    float c = Y + 1 < ny ? p[nx] : 0.0f, d = Y > 0 ? p[-nx] : 0.0f;
+    float e = Z + 1 < dN ? p[m] : vi, f = v[o];
+    const float s = ((a + b) + (c + d)) + (e + f);
+    float x;
+    if (fabsf(s) < INFINITY) {
+        // descending a >= b >= ... >= f
+        auto ord = [](float &hi, float &lo) {
+            const float h = fmaxf(hi, lo);
+            lo = fminf(hi, lo);
+            hi = h;
+        };
+        ord(a, b), ord(c, d), ord(e, f);
+        ord(a, c), ord(d, f), ord(b, e);
+        ord(a, b), ord(c, d), ord(e, f);
+        ord(b, c), ord(d, e);
+        ord(c, d);
+        const float l2 = 2.0f * lambda, l4 = 4.0f * lambda, l6 = 6.0f * lambda;
+        x = vi - l6;
+        x = vi < a + l6 ? a : x;
+        x = vi < a + l4 ? vi - l4 : x;
+        x = vi < b + l4 ? b : x;
+        x = vi < b + l2 ? vi - l2 : x;
+        x = vi < c + l2 ? c : x;
+        x = vi < c ? vi : x;
+        x = vi < d ? d : x;
+        x = vi < d - l2 ? vi + l2 : x;
+        x = vi < e - l2 ? e : x;
+        x = vi < e - l4 ? vi + l4 : x;
+        x = vi < f - l4 ? f : x;
+        x = vi < f - l6 ? vi + l6 : x;
+    } else {
+        x = cs_select(v, nx, ny, dN, X, Y, Z, lambda);
+    }
+    if (First) {
+        x = fmaxf(1.0e-6f, x);
+        x = x != x ? 1.0e-6f : x;
+    }
+    x_new[(size_t)Z * m + o] = x;
 }
 
 // grid-stride over dN*ny*nx voxels.
@@ -168,6 +227,14 @@ int launch_ista3d(const float *v, float *x_new, int nx, int ny, int dN, float la
     if (e != cudaSuccess) return xct_cuda_fail(e, "ista3d_kernel launch");
     g_xct_launches.fetch_add(1);
     return XCT_OK;
+}
+
+int launch_prox(const float *v, float *x_new, int nx, int ny, int dN, float lambda, bool first, cudaStream_t st)
+{
+    const dim3 grid((nx + 31) / 32, (ny + 7) / 8, dN);
+    if (dN > 65535) return xct_fail(XCT_E_INVALID, "compressed sensing: too many slices in one call");
+    return first ? xct_launch(prox_kernel<true>, grid, 256, 0, st, v, x_new, nx, ny, dN, lambda)
+                 : xct_launch(prox_kernel<false>, grid, 256, 0, st, v, x_new, nx, ny, dN, lambda);
 }
 
 int launch_fista3d(const float *x_in, float *w, const float *v, float *beta, float *x_new, int nx, int ny, int dN,

@@ -78,7 +78,7 @@ struct xct_plan {
     double *d_red = nullptr;     // [2*max_batch] focus-index sums (rotation-centre search)
     float *d_rc_prm = nullptr;   // [max_batch][16] mask constants per shift
     float *d_fi = nullptr;       // [max_batch] focus indices
-    float *d_cs = nullptr;       // compressed-sensing OS-EM: w, beta, x' [3][max_batch][ny][nx],
+    float *d_cs = nullptr;       // compressed-sensing OS-EM: the other image [max_batch][ny][nx],
                                  // allocated by the first such run
     float *d_fista = nullptr;    // FISTA: v, w, beta, dest [4][max_batch][ny][nx] (first FISTA run)
     float *d_pi = nullptr;       // power iteration: layer images, candidate, projection (first use)
@@ -192,6 +192,8 @@ const char *xct_tune_env_path();
 void xct_plan_default_tuning(xct_plan *p);
 // Compressed-sensing proximal steps (xct_cs.cu): ISTA3D, FISTA3D over dN slices.
 int launch_ista3d(const float *v, float *x_new, int nx, int ny, int dN, float lambda, int sm_count, cudaStream_t st);
+// The proximal step alone (first: ISTA3D's, else FISTA3D's x_{t+1}), v -> x_new.
+int launch_prox(const float *v, float *x_new, int nx, int ny, int dN, float lambda, bool first, cudaStream_t st);
 // FISTA3D with x_t read from x_in (may equal w) and x_{t+1} stored to x_new (may be null).
 int launch_fista3d(const float *x_in, float *w, const float *v, float *beta, float *x_new, int nx, int ny, int dN,
                    float lambda, int sm_count, cudaStream_t st);
