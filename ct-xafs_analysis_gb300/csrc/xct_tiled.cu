@@ -18,14 +18,12 @@
 // and clears it for the next subset.
 //
 // Backprojector (OSEM2, OSEM.cl:71-105), footprint-staged:
-//   * one CTA owns a 64x64 pixel tile; per angle it stages the window of ratio bins its
-//     pixels hit (bin coordinates are monotone in X and in Y, so the tile corners bound the
-//     window exactly) into shared memory with coalesced loads;
-//   * each thread gathers 8 pixels (8 apart) of four rows (16 apart; 128 threads) or, for launches with
-//     few tiles, of two rows (32 apart; 256 threads) per angle, in angle order, evaluating the
-//     reference's bin expression ((Xc*c - Yc*s) + cx) + 0.5 -- the products Xc*c once for
-//     all its rows, the rest with packed f32x2 instructions (each lane rounds exactly like the
-//     scalar expression) and the nearest rule as a round-down add;
+//   * one CTA owns a pixel tile (32x32 of up to eight slices; 64x64 of one in the batched launches); per
+//     angle it stages the window of ratio bins its pixels hit (bin coordinates are monotone in X and in
+//     Y, so the tile corners bound the window exactly) into shared memory;
+//   * each thread gathers its pixels' bins per angle, in angle order, evaluating the
+//     reference's bin expression ((Xc*c - Yc*s) + cx) + 0.5 with packed f32x2 instructions (each
+//     lane rounds exactly like the scalar expression) and the nearest rule as a round-down add;
 //   * the multiplicative update is fused.
 #include <stdint.h>
 
@@ -52,9 +50,8 @@ constexpr int kLanesPerRay = 4;
 constexpr int kRaysPerWarp = 32 / kLanesPerRay;
 
 constexpr int kBpTX = 64, kBpTY = 64;  // backprojection tile (pixels)
-// A backprojector thread takes 8 pixels of R rows (kBpTY / R apart): R = 4 shares the
-// products Xc*c over four rows (128 threads, 80 registers); R = 2 (256 threads, 64 registers)
-// fills the SMs better when a launch has few tiles.
+// A thread of bp_tile takes 8 pixels of R rows (kBpTY / R apart): R = 4 shares the
+// products Xc*c over four rows (128 threads, 80 registers).
 template <int R>
 struct BpCfg {
     static constexpr int Threads = (kBpTX / 8) * (kBpTY / R);
@@ -562,56 +559,58 @@ __device__ __forceinline__ void bp_tile(const KGeom &g, float *__restrict__ img,
     __syncthreads();  // the shared arrays may be restaged by the caller's next tile
 }
 
-// grid: (ntx*nty tiles, 1, dN).
-template <int R>
-__global__ void __launch_bounds__(BpCfg<R>::Threads) bp_tiled_kernel(float *img, const float *ratio,
-                                                            const float2 *__restrict__ trig, KGeom g, int sub,
-                                                            int nang, int ntx, float ssf, float paf)
-{
-    __shared__ BpShared sh;
-    const int z = blockIdx.z;
-    xct_grid_wait();
-    xct_grid_trigger();
-    bp_tile<R>(g, img + (size_t)z * g.nx * g.ny, ratio + (size_t)z * g.pa * g.px, trig, sub, nang,
-            (int)blockIdx.x % ntx, (int)blockIdx.x / ntx, ssf, paf, sh);
-}
-
-// --------------------------------------------- backprojector, eight slices per tile
+// --------------------------------------------- backprojector, one to eight slices per tile
 // For the slices of one OS-EM call (one geometry) a (pixel, angle) pair reads the same bin in
-// all eight slices of a group, so the bin expression is evaluated once for eight gathers.  A
-// CTA of 256 threads owns a 32 x 32 pixel tile of eight slices and stages, per angle and
+// all S slices of a group, so the bin expression is evaluated once for S gathers.  A
+// CTA of 256 threads owns a 32 x 32 pixel tile of S slices and stages, per angle and
 // slice, the window of the tile's bins (< 48, bounded exactly by the tile corners as in
-// bp_tiled_kernel, its start rounded down to a multiple of 4) with asynchronous 16-byte copies
-// (zero-filled off the detector), 24 angles at a time.  A thread takes 4 pixels of one row (8
+// bp_tile, its start rounded down to a multiple of 4) with asynchronous 16-byte copies
+// (zero-filled off the detector), a chunk of angles at a time.  A thread takes 4 pixels of one row (8
 // apart), a warp 8 adjacent pixels in each of 4 rows: the bins one load instruction touches
 // span fewer than 32 consecutive words, so no load has a bank conflict.  Per pixel and angle:
-// the literal bin expression of bp_tiled_kernel, one address, eight 4-byte loads at constant
-// offsets (one per slice), four packed adds -- in angle order, so each slice's sum is
-// bp_tiled_kernel's bit for bit -- and the update at the end.
+// the literal bin expression of bp_tile, one address, S 4-byte loads at constant
+// offsets (one per slice), packed adds over slice pairs (pixel pairs for one slice) -- in angle order,
+// so each slice's sum is bp_tile's bit for bit -- and the update at the end.
+// Bound: the shared-memory data path from two slices on (4 B per gather and slice), issue for one (5
+// instructions, 7 operations of the FP32 pipe a gather).  The small tiles also spread one slice over the SMs:
+// 2048^2 has 4096 of them against 1024 of bp_tile's 64 x 64 (1.7 waves).  100 angles of one 2048^2 slice:
+// 95 us against 108 with 64 x 64 tiles; three slices of 509 x 487 with 31 angles: 15 against 27.
 constexpr int kMsSlices = 8;  // slices per group of the slice-interleaved kernels
 constexpr int kBpMsT = 32;
 constexpr int kBpMsThreads = 256;
 constexpr int kBpMsW = 52;      // staged bins per angle and slice (>= 31|c| + 31|s| + 3 + 3 = 49.9)
-constexpr int kBpMsChunk = 24;  // angles per staging pass
 constexpr int kBpMsPix = 4;     // pixels per thread, 8 apart
-constexpr unsigned kBpMsSliceBytes = (unsigned)(kBpMsChunk * kBpMsW * 4);  // one slice's windows
 
 template <int S>
 struct BpMsShared {
-    float win[S * kBpMsChunk * kBpMsW];          // [slice][angle][bin]
-    float2 scs[kBpMsChunk];                      // (c, s)
-    int slo[kBpMsChunk];                         // first staged bin (a multiple of 4)
-    unsigned soff[kBpMsChunk];                   // byte address of slice 0's entry (bits - BIAS - lo)
+    static constexpr int Chunk = S == 8 ? 24 : S == 4 ? 32 : S == 2 ? 48 : 64;  // angles per staging pass
+    static constexpr unsigned SliceBytes = (unsigned)(Chunk * kBpMsW * 4);      // one slice's windows
+    float win[S * Chunk * kBpMsW];  // [slice][angle][bin]
+    float2 scs[Chunk];              // (c, s)
+    int slo[Chunk];                 // first staged bin (a multiple of 4)
+    unsigned soff[Chunk];           // byte address of slice 0's entry (bits - BIAS - lo)
 };
 
-// grid: (ntx*nty tiles of 32 x 32, 1, dN / S slice groups), S = 8 or 2.  vec: 16-byte staging
+// Slices Z .. S-1 of the bin at byte address ad.
+template <int S, unsigned SliceBytes, int Z = 0>
+__device__ __forceinline__ void bp_loads(unsigned ad, float (&v)[S])
+{
+    if constexpr (Z < S) {
+        v[Z] = lds_f1_at<(int)(Z * SliceBytes)>(ad);
+        bp_loads<S, SliceBytes, Z + 1>(ad, v);
+    }
+}
+
+// grid: (ntx*nty tiles of 32 x 32, 1, dN / S slice groups).  vec: 16-byte staging
 // copies (px a multiple of 4 and a 16-byte aligned ratio array).
 template <int S>
 __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const float *ratio,
                                                              const float2 *__restrict__ trig, KGeom g, int sub,
                                                              int nang, int ntx, float ssf, float paf, int vec)
 {
-    __shared__ __align__(16) BpMsShared<S> sh;
+    typedef BpMsShared<S> C;
+    constexpr int kAcc = S == 1 ? kBpMsPix / 2 : kBpMsPix * (S / 2);
+    __shared__ __align__(16) C sh;
     xct_grid_wait();
     xct_grid_trigger();
     const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
@@ -628,18 +627,16 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
     float xc[kBpMsPix];
 #pragma unroll
     for (int i = 0; i < kBpMsPix; ++i) xc[i] = (float)min(X0 + tx + 8 * i, X1) - g.hx;
-    f2x acc[kBpMsPix][S / 2];  // slice pairs of each pixel
+    f2x acc[kAcc];  // S > 1: slice pairs of each pixel, [pixel][pair]; S = 1: pixel pairs
 #pragma unroll
-    for (int i = 0; i < kBpMsPix; ++i)
-#pragma unroll
-        for (int h = 0; h < S / 2; ++h) acc[i][h] = 0ull;
+    for (int i = 0; i < kAcc; ++i) acc[i] = 0ull;
     const f2x cxp = f2_pack(g.cx, g.cx);
     const f2x hp = f2_pack(0.5f, 0.5f);
     const f2x MM = f2_pack(kMagic, kMagic);
     const unsigned wbase = (unsigned)__cvta_generic_to_shared(sh.win);
 
-    for (int k0 = 0; k0 < nang; k0 += kBpMsChunk) {
-        const int kn = min(kBpMsChunk, nang - k0);
+    for (int k0 = 0; k0 < nang; k0 += C::Chunk) {
+        const int kn = min(C::Chunk, nang - k0);
         __syncthreads();  // the previous chunk's gathers are done with the shared arrays
         for (int k = t; k < kn; k += kBpMsThreads) {
             const float2 cs = trig[sub + (k0 + k) * g.ss];
@@ -668,7 +665,7 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
                 const int th = sub + (k0 + k) * g.ss;
                 const float *row = rz + (size_t)z * nprj + (size_t)th * g.px;
                 const int nb = bin < 0 ? 0 : min(4, g.px - bin);
-                const unsigned dst = wbase + (unsigned)z * kBpMsSliceBytes + 4u * (unsigned)(k * kBpMsW + 4 * q);
+                const unsigned dst = wbase + (unsigned)z * C::SliceBytes + 4u * (unsigned)(k * kBpMsW + 4 * q);
                 cp_async16(dst, nb > 0 ? (const void *)(row + bin) : (const void *)row, nb > 0 ? 4u * (unsigned)nb : 0u);
             }
         } else {
@@ -679,7 +676,7 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
                 const int th = sub + (k0 + k) * g.ss;
                 const float *row = rz + (size_t)z * nprj + (size_t)th * g.px;
                 const bool in = (unsigned)bin < (unsigned)g.px;
-                const unsigned dst = wbase + (unsigned)z * kBpMsSliceBytes + 4u * (unsigned)(k * kBpMsW + j);
+                const unsigned dst = wbase + (unsigned)z * C::SliceBytes + 4u * (unsigned)(k * kBpMsW + j);
                 cp_async4(dst, in ? (const void *)(row + bin) : (const void *)row, in ? 4u : 0u);
             }
         }
@@ -694,33 +691,32 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
             const float q = Yc * s;
 #pragma unroll
             for (int j = 0; j < kBpMsPix / 2; ++j) {
-                // the literal bin expression of bp_tiled_kernel for pixels 2j and 2j+1
+                // the literal bin expression of bp_tile for pixels 2j and 2j+1
                 const float pa_ = xc[2 * j] * c, pb_ = xc[2 * j + 1] * c;
                 const f2x tt = f2_add_rd(f2_add(f2_add(f2_pack(pa_ - q, pb_ - q), cxp), hp), MM);
                 int b0, b1;
                 f2_unpack_bits(tt, b0, b1);
                 const unsigned ad[2] = {(unsigned)b0 * 4u + off, (unsigned)b1 * 4u + off};
+                float v[2][S];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    float v[S];
                     if (XCT_IN(ad[u], wlo, whi, XCT_SITE_BP_WIN)) {
-                        v[0] = lds_f1_at<0 * kBpMsSliceBytes>(ad[u]);
-                        v[1] = lds_f1_at<1 * kBpMsSliceBytes>(ad[u]);
-                        if constexpr (S == 8) {
-                            v[2] = lds_f1_at<2 * kBpMsSliceBytes>(ad[u]);
-                            v[3] = lds_f1_at<3 * kBpMsSliceBytes>(ad[u]);
-                            v[4] = lds_f1_at<4 * kBpMsSliceBytes>(ad[u]);
-                            v[5] = lds_f1_at<5 * kBpMsSliceBytes>(ad[u]);
-                            v[6] = lds_f1_at<6 * kBpMsSliceBytes>(ad[u]);
-                            v[7] = lds_f1_at<7 * kBpMsSliceBytes>(ad[u]);
-                        }
+                        bp_loads<S, C::SliceBytes>(ad[u], v[u]);
                     } else {
 #pragma unroll
-                        for (int z = 0; z < S; ++z) v[z] = 0.0f;
+                        for (int z = 0; z < S; ++z) v[u][z] = 0.0f;
                     }
+                }
+                if constexpr (S == 1) {
+                    acc[j] = f2_add(acc[j], f2_pack(v[0][0], v[1][0]));
+                } else {
 #pragma unroll
-                    for (int h = 0; h < S / 2; ++h)
-                        acc[2 * j + u][h] = f2_add(acc[2 * j + u][h], f2_pack(v[2 * h], v[2 * h + 1]));
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int h = 0; h < S / 2; ++h) {
+                            f2x &a = acc[(2 * j + u) * (S / 2) + h];
+                            a = f2_add(a, f2_pack(v[u][2 * h], v[u][2 * h + 1]));
+                        }
                 }
             }
         }
@@ -731,14 +727,21 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
     for (int i = 0; i < kBpMsPix; ++i) {
         const int X = X0 + tx + 8 * i;
         if (X > X1) continue;
-#pragma unroll
-        for (int h = 0; h < S / 2; ++h) {
+        float *p0 = img + (size_t)z0 * nimg + (size_t)Y * g.nx + X;
+        if constexpr (S == 1) {
             float v0, v1;
-            f2_unpack(acc[i][h], v0, v1);
-            float *p0 = img + (size_t)(z0 + 2 * h) * nimg + (size_t)Y * g.nx + X;
-            *p0 = xct_update(*p0, v0, ssf, paf);
-            float *p1 = p0 + nimg;
-            *p1 = xct_update(*p1, v1, ssf, paf);
+            f2_unpack(acc[i / 2], v0, v1);
+            *p0 = xct_update(*p0, i & 1 ? v1 : v0, ssf, paf);
+        } else {
+#pragma unroll
+            for (int h = 0; h < S / 2; ++h) {
+                float v0, v1;
+                f2_unpack(acc[i * (S / 2) + h], v0, v1);
+                float *p = p0 + (size_t)(2 * h) * nimg;
+                *p = xct_update(*p, v0, ssf, paf);
+                p += nimg;
+                *p = xct_update(*p, v1, ssf, paf);
+            }
         }
     }
 }
@@ -1066,38 +1069,27 @@ int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const
     if (dN <= 0) return XCT_OK;
     if (bp_is_direct(g, dN)) return launch_bp_update_direct(g, trig, img, ratio, dN, sub, st);
     const int nang = (g.pa - sub + g.ss - 1) / g.ss;  // OSEM2's angle loop (OSEM.cl:93)
-    // with the slice-interleaved kernels on, whole groups of eight slices go through the
-    // eight-slice backprojector, pairs of the rest through its two-slice form, and a last
-    // single slice through the per-slice one
-    if (g.ms_chunk > 0 && dN >= 2) {
-        const int mtx = (g.nx + kBpMsT - 1) / kBpMsT, mty = (g.ny + kBpMsT - 1) / kBpMsT;
-        const int vec = g.px % 4 == 0 && ((uintptr_t)ratio & 15u) == 0;
-        const int g8 = dN / kMsSlices, g2 = (dN - g8 * kMsSlices) / 2;
-        int rc = XCT_OK;
-        if (g8 > 0) {
-            rc = xct_launch(bp_ms_kernel<kMsSlices>, dim3(mtx * mty, 1, g8), kBpMsThreads, 0, st, img, ratio, trig, g, sub,
-                            nang, mtx, (float)g.ss, (float)g.pa, vec);
-            img += (size_t)g8 * kMsSlices * g.nx * g.ny;
-            ratio += (size_t)g8 * kMsSlices * g.pa * g.px;
-            dN -= g8 * kMsSlices;
-        }
-        if (g2 > 0 && rc == XCT_OK) {
-            rc = xct_launch(bp_ms_kernel<2>, dim3(mtx * mty, 1, g2), kBpMsThreads, 0, st, img, ratio, trig, g, sub, nang, mtx,
-                            (float)g.ss, (float)g.pa, vec);
-            img += (size_t)g2 * 2 * g.nx * g.ny;
-            ratio += (size_t)g2 * 2 * g.pa * g.px;
-            dN -= g2 * 2;
-        }
-        if (rc || dN == 0) return rc;
-    }
-    const int ntx = (g.nx + kBpTX - 1) / kBpTX, nty = (g.ny + kBpTY - 1) / kBpTY;
-    const dim3 grid(ntx * nty, 1, dN);
-    // four rows per thread once the grid gives three waves of its resident CTAs (6 per SM)
-    if ((long long)ntx * nty * dN >= 3LL * 6 * device_sm_count())
-        return xct_launch(bp_tiled_kernel<4>, grid, BpCfg<4>::Threads, 0, st, img, ratio, trig, g, sub, nang, ntx, (float)g.ss,
-                          (float)g.pa);
-    return xct_launch(bp_tiled_kernel<2>, grid, BpCfg<2>::Threads, 0, st, img, ratio, trig, g, sub, nang, ntx, (float)g.ss,
-                      (float)g.pa);
+    // With the slice-interleaved kernels on, whole groups of eight slices go through the eight-slice form;
+    // the rest (with grouping on) in fours, pairs and singles -- the larger forms cost less per slice, but
+    // only where their grid still gives every SM four CTAs.
+    const int mtx = (g.nx + kBpMsT - 1) / kBpMsT, mty = (g.ny + kBpMsT - 1) / kBpMsT;
+    const int vec = g.px % 4 == 0 && ((uintptr_t)ratio & 15u) == 0;
+    const long long tiles = (long long)mtx * mty, fill = 4LL * device_sm_count();
+    auto run = [&](auto sc, int groups) -> int {
+        constexpr int S = decltype(sc)::value;
+        const int rc = xct_launch(bp_ms_kernel<S>, dim3(mtx * mty, 1, groups), kBpMsThreads, 0, st, img, ratio, trig, g, sub,
+                                  nang, mtx, (float)g.ss, (float)g.pa, vec);
+        img += (size_t)groups * S * g.nx * g.ny;
+        ratio += (size_t)groups * S * g.pa * g.px;
+        dN -= groups * S;
+        return rc;
+    };
+    int rc = XCT_OK;
+    if (g.ms_chunk > 0 && dN >= kMsSlices) rc = run(std::integral_constant<int, 8>{}, dN / kMsSlices);
+    if (!rc && g.fwd_group && dN >= 4 && tiles * (dN / 4) >= fill) rc = run(std::integral_constant<int, 4>{}, dN / 4);
+    if (!rc && g.fwd_group && dN >= 2 && tiles * (dN / 2) >= fill) rc = run(std::integral_constant<int, 2>{}, dN / 2);
+    if (!rc && dN >= 1) rc = run(std::integral_constant<int, 1>{}, dN);
+    return rc;
 }
 
 XCT_CHECK_READER(xct_check_read_tiled)
