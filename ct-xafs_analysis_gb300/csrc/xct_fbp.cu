@@ -19,15 +19,15 @@
 // bins stay in place here and the filtered row is the same in exact arithmetic.  The
 // rounding differs from the reference's radix-2 float FFT at the 1e-6 relative level.
 //
-// FBP backprojection.  Same pixel tiling as the OS-EM backprojector (64 x 64 pixels, 8 per
-// thread in two or four rows, per-angle windows of the filtered row staged in shared
-// memory), with the
+// FBP backprojection.  The OS-EM backprojector's tiling (32 x 32 pixels of up to eight slices,
+// per-angle windows of the filtered rows staged in shared memory), with the
 // reference's linear sampler along the row and its per-pixel expression order, so the
 // image is bit-identical to FBP.cl's for the same filtered sinogram.
 #include <math.h>
 #include <stdio.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "xct_async.cuh"
 #include "xct_check.cuh"
@@ -36,12 +36,6 @@
 #include "xct_internal.h"
 
 namespace {
-
-// backprojection: 64 x 64 pixel tiles (each thread 8 pixels of two rows 32 apart), windows of
-// kFbpW >= 63|c| + 63|s| + 4 bins staged kFbpChunk angles at a time
-// (40 angles of 96 bin pairs: 31 KB of shared memory, so the register-limited six CTAs of the
-// four-row kernel still fit on an SM)
-constexpr int kFbpTX = 64, kFbpTY = 64, kFbpThreads = 256, kFbpChunk = 40, kFbpW = 96;
 
 // ------------------------------------------------------------------ ramp filter (FFT)
 __device__ __forceinline__ int fpad(int i) { return i + (i >> 4); }  // 16-entry rows + 1
@@ -197,19 +191,6 @@ __global__ void __launch_bounds__(1024) fbp_filter_kernel(const float *__restric
 }
 
 // ------------------------------------------------------------ FBP backprojection
-struct FbpShared {
-    float2 win[kFbpChunk * kFbpW];  // entry j of angle k: (t[lo+j], t[lo+j+1]), the lerp's two bins
-    float2 scs[kFbpChunk];
-    int slo[kFbpChunk];
-    unsigned soff[kFbpChunk];  // shared address of angle k's entry for floor bits fb: soff[k] + 8*fb
-    float red[kFbpThreads / 32];
-};
-
-__device__ __forceinline__ void fbp_lds2(unsigned addr, float &t0, float &t1)
-{
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t0), "=f"(t1) : "r"(addr));
-}
-
 // Monotone integer key of a float (atomicMin on keys orders as the floats do).
 __device__ __forceinline__ int fkey(float f)
 {
@@ -218,181 +199,68 @@ __device__ __forceinline__ int fkey(float f)
 }
 __device__ __forceinline__ float fkey_decode(int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7FFFFFFF); }
 
-// grid: (ntx * nty, 1, dN).  img[Y][X] = (1/(2 pa)) sum_th lin(fprj[th], u) for pixels with
-// r < nx/2, else 0 (FBP.cl:178-187); u = ((Xc c - Yc s) + cx) + 0.5, sampled by the linear
+// img[Y][X] = (1/(2 pa)) sum_th lin(fprj[th], u) for pixels with r < nx/2, else 0
+// (FBP.cl:178-187); u = ((Xc c - Yc s) + cx) + 0.5, sampled by the linear
 // sampler at (u, th + 0.5): i = floor(u - 0.5), a = (u - 0.5) - i,
 // (1 - a) t[i] + a t[i+1], zero off the detector.  min_keys (optional): the per-slice
 // minimum of the written image, as keys.
-// R rows per thread (kFbpTY / R apart, 512 / R threads): R = 4 shares the products Xc*c over
-// four rows; R = 2 fills the SMs better when a launch has few tiles.
-template <int R>
-__global__ void __launch_bounds__(512 / R, R == 4 ? 6 : 4) fbp_bp_kernel(const float *__restrict__ fprj, float *__restrict__ img,
-                                                         const float2 *__restrict__ trig, KGeom g, int ntx,
-                                                         int *__restrict__ min_keys)
-{
-    constexpr int kThr = 512 / R, kStride = kFbpTY / R;
-    __shared__ FbpShared sh;
-    const int z = blockIdx.z;
-    const float *rt = fprj + (size_t)z * g.pa * g.px;
-    const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
-    const int X0 = bx * kFbpTX, Y0 = by * kFbpTY;
-    const int X1 = min(X0 + kFbpTX, g.nx) - 1, Y1 = min(Y0 + kFbpTY, g.ny) - 1;
-    // thread tx takes the pixels X0 + tx + 8i (i < 8): the 8 lanes of a row read neighbouring
-    // bins and write neighbouring pixels
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-    float Ycr[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) Ycr[r] = (float)min(Y0 + ty + r * kStride, Y1) - g.hy;
-    float xc[8];
-    f2x acc2[R][4];  // pixel pairs of each row, packed adds (each lane an IEEE add)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) xc[i] = (float)min(X0 + tx + 8 * i, X1) - g.hx;
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc2[r][j] = f2_pack(0.0f, 0.0f);
-    const unsigned wbase = (unsigned)__cvta_generic_to_shared(sh.win);
-    const f2x cxp = f2_pack(g.cx, g.cx), hp = f2_pack(0.5f, 0.5f), MM = f2_pack(12582912.0f, 12582912.0f);
-    const f2x one2 = f2_pack(1.0f, 1.0f);
-    for (int k0 = 0; k0 < g.pa; k0 += kFbpChunk) {
-        const int kn = min(kFbpChunk, g.pa - k0);
-        __syncthreads();
-        for (int k = threadIdx.x; k < kn; k += kThr) {
-            const float2 cs = trig[k0 + k];
-            sh.scs[k] = cs;
-            // u is monotone in X and in Y (every step rounds monotonically): the corners
-            // bound the window of floor(u - 0.5)
-            const float xa = (float)X0 - g.hx, xb = (float)X1 - g.hx;
-            const float qa = ((float)Y0 - g.hy) * cs.y, qb = ((float)Y1 - g.hy) * cs.y;
-            int lo = xct_floor_bits(xct_bin_coord(xa, cs.x, qa, g.cx) - 0.5f);
-            lo = min(lo, xct_floor_bits(xct_bin_coord(xb, cs.x, qa, g.cx) - 0.5f));
-            lo = min(lo, xct_floor_bits(xct_bin_coord(xa, cs.x, qb, g.cx) - 0.5f));
-            lo = min(lo, xct_floor_bits(xct_bin_coord(xb, cs.x, qb, g.cx) - 0.5f));
-            sh.slo[k] = lo - XCT_FLOOR_BIAS;
-            // entry for floor bits fb: k*W + fb - lo  (mod 2^32), 8 bytes each
-            sh.soff[k] = wbase + 8u * (unsigned)(k * kFbpW) - 8u * (unsigned)lo;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < kn * kFbpW; i += kThr) {
-            const int k = i / kFbpW, j = i - k * kFbpW;
-            const int bin = sh.slo[k] + j;
-            const float *rk = rt + (size_t)(k0 + k) * g.px;
-            sh.win[i] = make_float2(((unsigned)bin < (unsigned)g.px) ? __ldg(rk + bin) : 0.0f,
-                                    ((unsigned)(bin + 1) < (unsigned)g.px) ? __ldg(rk + bin + 1) : 0.0f);
-        }
-        __syncthreads();
-        // any entry of the staged windows (each holds both bins of its lerp)
-        const unsigned wlo = wbase, whi = wbase + 8u * (unsigned)(kn * kFbpW - 1);
-        (void)wlo;
-        (void)whi;
-        for (int k = 0; k < kn; ++k) {
-            const float c = sh.scs[k].x, s = sh.scs[k].y;
-            const unsigned off = sh.soff[k];
-            float q[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) q[r] = Ycr[r] * s;
-            // one row's pixel pair from the shared products Xc*c: the additions, the
-            // round-down floor and the fraction packed over the pair, each lane rounding as
-            // the scalar expression uu = (((Xc*c - q) + cx) + 0.5) - 0.5, fi = floor(uu),
-            // a = uu - fi; then acc += (1 - a) t[fi] + a t[fi+1] with the products in scalar
-            // (ptxas fuses a packed multiply feeding a packed add or subtract, and the
-            // reference rounds each operation)
-            auto pair = [&](float p0, float p1, float qq, f2x &acc) {
-                const f2x d = f2_pack(p0 - qq, p1 - qq);
-                const f2x uu = f2_sub(f2_add(f2_add(d, cxp), hp), hp);
-                const f2x tb = f2_add_rd(uu, MM);
-                const f2x a2 = f2_sub(uu, f2_sub(tb, MM));
-                const f2x w2 = f2_sub(one2, a2);
-                int e0, e1;
-                f2_unpack_bits(tb, e0, e1);
-                float a0, a1, w0, w1;
-                f2_unpack(a2, a0, a1);
-                f2_unpack(w2, w0, w1);
-                const unsigned ad0 = (unsigned)e0 * 8u + off, ad1 = (unsigned)e1 * 8u + off;
-                const bool in0 = XCT_IN(ad0, wlo, whi, XCT_SITE_FBP_WIN), in1 = XCT_IN(ad1, wlo, whi, XCT_SITE_FBP_WIN);
-                float t00 = 0.0f, t01 = 0.0f, t10 = 0.0f, t11 = 0.0f;
-                if (in0) fbp_lds2(ad0, t00, t01);
-                if (in1) fbp_lds2(ad1, t10, t11);
-                const float p00 = w0 * t00, p01 = a0 * t01;
-                const float p10 = w1 * t10, p11 = a1 * t11;
-                acc = f2_add(acc, f2_add(f2_pack(p00, p10), f2_pack(p01, p11)));
-            };
-#pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                const float p0 = xc[i] * c, p1 = xc[i + 1] * c;
-#pragma unroll
-                for (int r = 0; r < R; ++r) pair(p0, p1, q[r], acc2[r][i / 2]);
-            }
-        }
-    }
-    const float two_pa = (float)g.pa * 2.0f;
-    float vmin = INFINITY;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int Y = Y0 + ty + r * kStride;
-        const float Yc = Ycr[r];
-        if (Y > Y1) continue;
-        float acc[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) f2_unpack(acc2[r][j], acc[2 * j], acc[2 * j + 1]);
-        float *row = img + ((size_t)z * g.ny + Y) * g.nx;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int X = X0 + tx + 8 * i;
-            if (X <= X1) {
-                const float rr = sqrtf(xc[i] * xc[i] + Yc * Yc);
-                const float v = (rr < g.hx) ? __fdiv_rn(acc[i], two_pa) : 0.0f;
-                row[X] = v;
-                vmin = fminf(vmin, v);
-            }
-        }
-    }
-    if (min_keys != nullptr) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
-        if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = vmin;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float m = sh.red[0];
-            for (int i = 1; i < kThr / 32; ++i) m = fminf(m, sh.red[i]);
-            atomicMin(min_keys + z, fkey(m));
-        }
-    }
-}
-
-// ---------------------------------------- FBP backprojection, eight slices per tile
+//
 // For the slices of one call (one geometry) a (pixel, angle) pair reads the same two bins in
-// all eight slices of a group, so the bin coordinate, floor and fraction are found once for
-// eight lerps.  A CTA of 256 threads owns a 32 x 32 pixel tile of eight slices and stages,
-// per angle and pair of slices, the window of the tile's bins (< 49 with the lerp's second
-// bin, bounded exactly by the tile corners as in fbp_bp_kernel, its start rounded down to a
-// multiple of 4) as (t_z, t_z+1) pairs by asynchronous copies, 24 angles at a time.  A
-// thread takes 4 pixels of one row (8 apart); per pixel and angle: the literal expression of
-// fbp_bp_kernel for u, floor and fraction, two 8-byte loads per slice pair (bins i and
-// i + 1), the products in scalar and their sum and the accumulation packed over the slice
-// pair -- each slice's sum is fbp_bp_kernel's bit for bit.  The epilogue (field-of-view mask,
-// 1/(2 pa), the slice minimum for the base-up) is fbp_bp_kernel's.
-constexpr int kFbpMsT = 32, kFbpMsThreads = 256, kFbpMsW = 52, kFbpMsChunk = 24, kFbpMsPix = 4, kFbpMsSlices = 8;
-constexpr unsigned kFbpMsPairBytes = (unsigned)(kFbpMsChunk * kFbpMsW * 8);  // one slice pair's windows
+// all slices of a group, so the bin coordinate, floor and fraction are found once for
+// S lerps.  A CTA of 256 threads owns a 32 x 32 pixel tile of S slices (8, 2 or 1) and stages the
+// window of the tile's bins (< 49 with the lerp's second bin, bounded exactly by the tile corners -- the
+// coordinate is monotone in X and in Y -- its start rounded down to a multiple of 4) by asynchronous
+// copies, a chunk of angles at a time: per slice pair as (t_z, t_z+1) pairs, for one slice as
+// (t[j], t[j+1]) pairs, so that its lerp is one 64-bit load.  A thread takes 4 pixels of one row (8 apart);
+// per pixel and angle the literal expression for u (products and differences in scalar: ptxas fuses a
+// packed multiply feeding a packed add or subtract, and the reference rounds each operation), floor as
+// a round-down add, the products in scalar, sums and accumulation packed over the slice pair (over the
+// pixel pair for one slice), in angle order, so every form gives a slice the same bits.
+//
+// A warp whose 32 x 4 pixels all lie outside the field of view (their values are 0 whatever the
+// projections) skips its gathers: 20 % of a square image.
+//
+// Bound: the FP32 pipe for one slice (12 operations a lerp that the reference's rounding fixes), the
+// shared-memory data path for eight (8 B per lerp and slice).  One 2048^2 slice, 1500 angles: 2.51 ms with
+// that pipe 72 % busy (2.88 with 64 x 64 tiles that covered the whole square).
+constexpr int kFbpMsT = 32, kFbpMsThreads = 256, kFbpMsW = 52, kFbpMsPix = 4, kFbpMsSlices = 8;
 
 template <int S>
 struct FbpMsShared {
-    float2 win[(S / 2) * kFbpMsChunk * kFbpMsW];  // [pair][angle][bin]: (t_z, t_z+1)
-    float2 scs[kFbpMsChunk];
-    int slo[kFbpMsChunk];
-    unsigned soff[kFbpMsChunk];  // shared address of angle k's entry for floor bits fb: soff[k] + 8*fb
+    static constexpr int P = S == 1 ? 1 : S / 2;           // pairs per bin
+    static constexpr int Chunk = S == 8 ? 24 : 48;         // angles per staging pass
+    static constexpr unsigned PairBytes = (unsigned)(Chunk * kFbpMsW * 8);  // one pair's windows
+    float2 win[P * Chunk * kFbpMsW];  // [pair][angle][bin]
+    float2 scs[Chunk];
+    int slo[Chunk];
+    unsigned soff[Chunk];  // shared address of angle k's entry for floor bits fb: soff[k] + 8*fb
     float red[kFbpMsThreads / 32][S];
 };
 
-// grid: (ntx * nty tiles of 32 x 32, 1, dN / S slice groups), S = 8 or 2.
+// Both bins of slice pair H .. P-1 at byte address ad, weighted and added to the pairs' sums.
+template <int S, int H = 0>
+__device__ __forceinline__ void fbp_pairs(unsigned ad, float w, float a, f2x *acc)
+{
+    if constexpr (H < S / 2) {
+        float t0a, t0b, t1a, t1b;  // (slice 2H, 2H+1) at bins i and i + 1
+        lds_f2_at<(int)(H * FbpMsShared<S>::PairBytes)>(ad, t0a, t0b);
+        lds_f2_at<(int)(H * FbpMsShared<S>::PairBytes + 8)>(ad, t1a, t1b);
+        const float pa0 = w * t0a, pb0 = w * t0b, pa1 = a * t1a, pb1 = a * t1b;
+        acc[H] = f2_add(acc[H], f2_add(f2_pack(pa0, pb0), f2_pack(pa1, pb1)));
+        fbp_pairs<S, H + 1>(ad, w, a, acc);
+    }
+}
+
+// grid: (ntx * nty tiles of 32 x 32, 1, dN / S slice groups).
 template <int S>
 __global__ void __launch_bounds__(kFbpMsThreads) fbp_bp_ms_kernel(const float *__restrict__ fprj,
                                                                   float *__restrict__ img,
                                                                   const float2 *__restrict__ trig, KGeom g, int ntx,
                                                                   int *__restrict__ min_keys)
 {
-    constexpr int P = S / 2;
-    __shared__ __align__(16) FbpMsShared<S> sh;
+    typedef FbpMsShared<S> C;
+    constexpr int kAcc = S == 1 ? kFbpMsPix / 2 : kFbpMsPix * C::P;
+    __shared__ __align__(16) C sh;
     const int z0 = (int)blockIdx.z * S;
     const size_t nprj = (size_t)g.pa * g.px, nimg = (size_t)g.nx * g.ny;
     const float *rz = fprj + (size_t)z0 * nprj;
@@ -404,16 +272,20 @@ __global__ void __launch_bounds__(kFbpMsThreads) fbp_bp_ms_kernel(const float *_
     float xc[kFbpMsPix];
 #pragma unroll
     for (int i = 0; i < kFbpMsPix; ++i) xc[i] = (float)min(X0 + tx + 8 * i, X1) - g.hx;
-    f2x acc[kFbpMsPix][P];
+    f2x acc[kAcc];  // S > 1: [pixel][slice pair]; S = 1: pixel pairs
 #pragma unroll
-    for (int i = 0; i < kFbpMsPix; ++i)
+    for (int i = 0; i < kAcc; ++i) acc[i] = 0ull;
+    // any pixel of this warp inside the field of view (the epilogue's own test)
+    bool in_view = false;
 #pragma unroll
-        for (int h = 0; h < P; ++h) acc[i][h] = 0ull;
+    for (int i = 0; i < kFbpMsPix; ++i) in_view |= sqrtf(xc[i] * xc[i] + Yc * Yc) < g.hx;
+    in_view = __any_sync(0xffffffffu, in_view);
     const unsigned wbase = (unsigned)__cvta_generic_to_shared(sh.win);
     const f2x cxp = f2_pack(g.cx, g.cx), hp = f2_pack(0.5f, 0.5f), MM = f2_pack(12582912.0f, 12582912.0f);
     const f2x one2 = f2_pack(1.0f, 1.0f);
-    for (int k0 = 0; k0 < g.pa; k0 += kFbpMsChunk) {
-        const int kn = min(kFbpMsChunk, g.pa - k0);
+    const int nang = __syncthreads_or(in_view) ? g.pa : 0;  // a tile outside the field of view stages nothing
+    for (int k0 = 0; k0 < nang; k0 += C::Chunk) {
+        const int kn = min(C::Chunk, g.pa - k0);
         __syncthreads();
         for (int k = threadIdx.x; k < kn; k += kFbpMsThreads) {
             const float2 cs = trig[k0 + k];
@@ -429,30 +301,44 @@ __global__ void __launch_bounds__(kFbpMsThreads) fbp_bp_ms_kernel(const float *_
             sh.soff[k] = wbase + 8u * (unsigned)(k * kFbpMsW) - 8u * (unsigned)lo;
         }
         __syncthreads();
-        // window (pair p, angle k, bin lo_k + r) = (t_{2p}, t_{2p+1}), 0 off the detector
-        for (int e = threadIdx.x; e < kn * S * kFbpMsW; e += kFbpMsThreads) {
-            const int r = e % kFbpMsW, t2 = e / kFbpMsW;
-            const int z = t2 % S, k = t2 / S;
-            const int bin = sh.slo[k] + r;
-            const float *row = rz + (size_t)z * nprj + (size_t)(k0 + k) * g.px;
-            const bool in = (unsigned)bin < (unsigned)g.px;
-            const unsigned dst =
-                wbase + (unsigned)(z >> 1) * kFbpMsPairBytes + 8u * (unsigned)(k * kFbpMsW + r) + 4u * (unsigned)(z & 1);
-            cp_async4(dst, in ? (const void *)(row + bin) : (const void *)row, in ? 4u : 0u);
+        // S > 1: window (pair p, angle k, bin lo_k + r) = (t_{2p}, t_{2p+1}); S = 1: (t[r], t[r + 1]); 0 off
+        // the detector
+        if constexpr (S == 1) {
+            for (int e = threadIdx.x; e < kn * kFbpMsW; e += kFbpMsThreads) {
+                const int r = e % kFbpMsW, k = e / kFbpMsW;
+                const int bin = sh.slo[k] + r;
+                const float *row = rz + (size_t)(k0 + k) * g.px;
+                const bool i0 = (unsigned)bin < (unsigned)g.px, i1 = (unsigned)(bin + 1) < (unsigned)g.px;
+                const unsigned dst = wbase + 8u * (unsigned)e;
+                cp_async4(dst, i0 ? (const void *)(row + bin) : (const void *)row, i0 ? 4u : 0u);
+                cp_async4(dst + 4u, i1 ? (const void *)(row + bin + 1) : (const void *)row, i1 ? 4u : 0u);
+            }
+        } else {
+            for (int e = threadIdx.x; e < kn * S * kFbpMsW; e += kFbpMsThreads) {
+                const int r = e % kFbpMsW, t2 = e / kFbpMsW;
+                const int z = t2 % S, k = t2 / S;
+                const int bin = sh.slo[k] + r;
+                const float *row = rz + (size_t)z * nprj + (size_t)(k0 + k) * g.px;
+                const bool in = (unsigned)bin < (unsigned)g.px;
+                const unsigned dst =
+                    wbase + (unsigned)(z >> 1) * C::PairBytes + 8u * (unsigned)(k * kFbpMsW + r) + 4u * (unsigned)(z & 1);
+                cp_async4(dst, in ? (const void *)(row + bin) : (const void *)row, in ? 4u : 0u);
+            }
         }
         cp_async_wait_all();
         __syncthreads();
         // any entry whose next entry (the lerp's second bin) is staged
-        const unsigned wlo = wbase, whi = wbase + 8u * (unsigned)(kn * kFbpMsW - 2);
+        const unsigned wlo = wbase, whi = wbase + 8u * (unsigned)(kn * kFbpMsW - (S == 1 ? 1 : 2));
         (void)wlo;
         (void)whi;
+        if (!in_view) continue;
         for (int k = 0; k < kn; ++k) {
             const float c = sh.scs[k].x, s = sh.scs[k].y;
             const unsigned off = sh.soff[k];
             const float q = Yc * s;
 #pragma unroll
             for (int j = 0; j < kFbpMsPix / 2; ++j) {
-                // fbp_bp_kernel's expression for pixels 2j and 2j+1
+                // uu = (((Xc*c - q) + cx) + 0.5) - 0.5, fi = floor(uu), a = uu - fi for pixels 2j and 2j+1
                 const float p0 = xc[2 * j] * c, p1 = xc[2 * j + 1] * c;
                 const f2x d = f2_pack(p0 - q, p1 - q);
                 const f2x uu = f2_sub(f2_add(f2_add(d, cxp), hp), hp);
@@ -465,27 +351,19 @@ __global__ void __launch_bounds__(kFbpMsThreads) fbp_bp_ms_kernel(const float *_
                 f2_unpack(a2, a[0], a[1]);
                 f2_unpack(w2, w[0], w[1]);
                 const unsigned ad[2] = {(unsigned)e0 * 8u + off, (unsigned)e1 * 8u + off};
+                if constexpr (S == 1) {
+                    float t[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    if (!XCT_IN(ad[u], wlo, whi, XCT_SITE_FBP_WIN)) continue;
+                    for (int u = 0; u < 2; ++u)
+                        if (XCT_IN(ad[u], wlo, whi, XCT_SITE_FBP_WIN)) lds_f2_at<0>(ad[u], t[u][0], t[u][1]);
+                    const float p00 = w[0] * t[0][0], p01 = a[0] * t[0][1];
+                    const float p10 = w[1] * t[1][0], p11 = a[1] * t[1][1];
+                    acc[j] = f2_add(acc[j], f2_add(f2_pack(p00, p10), f2_pack(p01, p11)));
+                } else {
 #pragma unroll
-                    for (int h = 0; h < P; ++h) {
-                        float t0a, t0b, t1a, t1b;  // (slice 2h, 2h+1) at bins i and i + 1
-                        if (h == 0) {
-                            lds_f2_at<0>(ad[u], t0a, t0b);
-                            lds_f2_at<8>(ad[u], t1a, t1b);
-                        } else if (h == 1) {
-                            lds_f2_at<1 * kFbpMsPairBytes>(ad[u], t0a, t0b);
-                            lds_f2_at<1 * kFbpMsPairBytes + 8>(ad[u], t1a, t1b);
-                        } else if (h == 2) {
-                            lds_f2_at<2 * kFbpMsPairBytes>(ad[u], t0a, t0b);
-                            lds_f2_at<2 * kFbpMsPairBytes + 8>(ad[u], t1a, t1b);
-                        } else {
-                            lds_f2_at<3 * kFbpMsPairBytes>(ad[u], t0a, t0b);
-                            lds_f2_at<3 * kFbpMsPairBytes + 8>(ad[u], t1a, t1b);
-                        }
-                        const float pa0 = w[u] * t0a, pb0 = w[u] * t0b, pa1 = a[u] * t1a, pb1 = a[u] * t1b;
-                        acc[2 * j + u][h] = f2_add(acc[2 * j + u][h], f2_add(f2_pack(pa0, pb0), f2_pack(pa1, pb1)));
+                    for (int u = 0; u < 2; ++u) {
+                        if (!XCT_IN(ad[u], wlo, whi, XCT_SITE_FBP_WIN)) continue;
+                        fbp_pairs<S>(ad[u], w[u], a[u], acc + (2 * j + u) * C::P);
                     }
                 }
             }
@@ -503,16 +381,12 @@ __global__ void __launch_bounds__(kFbpMsThreads) fbp_bp_ms_kernel(const float *_
             if (X > X1) continue;
             const float rr = sqrtf(xc[i] * xc[i] + Yc * Yc);
 #pragma unroll
-            for (int h = 0; h < P; ++h) {
+            for (int z = 0; z < S; ++z) {
                 float v2[2];
-                f2_unpack(acc[i][h], v2[0], v2[1]);
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int z = 2 * h + u;
-                    const float v = (rr < g.hx) ? __fdiv_rn(v2[u], two_pa) : 0.0f;
-                    img[(size_t)(z0 + z) * nimg + (size_t)Y * g.nx + X] = v;
-                    vmin[z] = fminf(vmin[z], v);
-                }
+                f2_unpack(S == 1 ? acc[i / 2] : acc[i * C::P + z / 2], v2[0], v2[1]);
+                const float v = (rr < g.hx) ? __fdiv_rn(v2[S == 1 ? i & 1 : z & 1], two_pa) : 0.0f;
+                img[(size_t)(z0 + z) * nimg + (size_t)Y * g.nx + X] = v;
+                vmin[z] = fminf(vmin[z], v);
             }
         }
     }
@@ -612,50 +486,31 @@ int launch_fbp_filter(const KGeom &g, const float *sino, float *out, int dN, int
 int launch_fbp_bp(const KGeom &g, const float2 *trig, const float *fprj, float *img, int dN, int *min_keys,
                   cudaStream_t st)
 {
-    const int ntx = (g.nx + kFbpTX - 1) / kFbpTX, nty = (g.ny + kFbpTY - 1) / kFbpTY;
     if (min_keys != nullptr) {
         cudaError_t e = cudaMemsetAsync(min_keys, 0x7F, sizeof(int) * dN, st);  // key of a huge float
         if (e != cudaSuccess) return xct_cuda_fail(e, "fbp min reset");
     }
-    // with the slice-interleaved kernels on, groups of eight slices go through the
-    // eight-slice backprojector, pairs of the rest through its two-slice form, and a last
-    // single slice through the per-slice one
-    if (g.ms_chunk > 0 && dN >= 2) {
-        const int mtx = (g.nx + kFbpMsT - 1) / kFbpMsT, mty = (g.ny + kFbpMsT - 1) / kFbpMsT;
-        const int g8 = dN / kFbpMsSlices, g2 = (dN - g8 * kFbpMsSlices) / 2;
-        auto advance = [&](int n) {
-            fprj += (size_t)n * g.pa * g.px;
-            img += (size_t)n * g.nx * g.ny;
-            if (min_keys != nullptr) min_keys += n;
-            dN -= n;
-        };
-        if (g8 > 0) {
-            fbp_bp_ms_kernel<kFbpMsSlices><<<dim3(mtx * mty, 1, g8), kFbpMsThreads, 0, st>>>(fprj, img, trig, g, mtx,
-                                                                                             min_keys);
-            cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return xct_cuda_fail(e, "fbp_bp_ms_kernel launch");
-            g_xct_launches.fetch_add(1);
-            advance(g8 * kFbpMsSlices);
-        }
-        if (g2 > 0) {
-            fbp_bp_ms_kernel<2><<<dim3(mtx * mty, 1, g2), kFbpMsThreads, 0, st>>>(fprj, img, trig, g, mtx, min_keys);
-            cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return xct_cuda_fail(e, "fbp_bp_ms_kernel launch");
-            g_xct_launches.fetch_add(1);
-            advance(g2 * 2);
-        }
-        if (dN == 0) return XCT_OK;
-    }
-    dim3 grid(ntx * nty, 1, dN);
-    // four rows per thread once the grid gives three waves of its resident CTAs (6 per SM)
-    if ((long long)grid.x * grid.z >= 3LL * 6 * device_sm_count())
-        fbp_bp_kernel<4><<<grid, 128, 0, st>>>(fprj, img, trig, g, ntx, min_keys);
-    else
-        fbp_bp_kernel<2><<<grid, 256, 0, st>>>(fprj, img, trig, g, ntx, min_keys);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return xct_cuda_fail(e, "fbp_bp_kernel launch");
-    g_xct_launches.fetch_add(1);
-    return XCT_OK;
+    // with the slice-interleaved kernels on, groups of eight slices go through the eight-slice form; the
+    // rest (with grouping on) in pairs, and a last single slice alone
+    const int mtx = (g.nx + kFbpMsT - 1) / kFbpMsT, mty = (g.ny + kFbpMsT - 1) / kFbpMsT;
+    auto run = [&](auto sc, int groups) -> int {
+        constexpr int S = decltype(sc)::value;
+        if (groups <= 0) return XCT_OK;
+        fbp_bp_ms_kernel<S><<<dim3(mtx * mty, 1, groups), kFbpMsThreads, 0, st>>>(fprj, img, trig, g, mtx, min_keys);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return xct_cuda_fail(e, "fbp_bp_ms_kernel launch");
+        g_xct_launches.fetch_add(1);
+        fprj += (size_t)groups * S * g.pa * g.px;
+        img += (size_t)groups * S * g.nx * g.ny;
+        if (min_keys != nullptr) min_keys += groups * S;
+        dN -= groups * S;
+        return XCT_OK;
+    };
+    int rc = XCT_OK;
+    if (g.ms_chunk > 0) rc = run(std::integral_constant<int, kFbpMsSlices>{}, dN / kFbpMsSlices);
+    if (!rc && g.fwd_group) rc = run(std::integral_constant<int, 2>{}, dN / 2);
+    if (!rc) rc = run(std::integral_constant<int, 1>{}, dN);
+    return rc;
 }
 
 int launch_base_up(const KGeom &g, float *img, int dN, int order, const int *min_keys, int sm_count, cudaStream_t st)
