@@ -22,12 +22,13 @@ constexpr int kDirRays = 8, kDirLanes = 4;  // a warp reads 8 rays x 4 consecuti
 constexpr int kDirWarps = 8;                // warps sharing the samples of the CTA's rays
 
 // Where the small-problem kernels run.  They read texels through L1 at about 0.3 samples per ns
-// whatever the size, the tiled forward kernel about 0.95 once its tiles fill the SMs; measured
-// per subset step with both (one slice, 10 to 15 subsets): 64^2 6 against 23 us, 256^2 x 18 angles
-// 11 against 37, three such slices 20 against 41, 384^2 x 27 angles 25 against 41, 512^2 x 36
-// angles 45 against 37.  The line is drawn between the last two.  The backprojector: one slice
-// of 512^2 x 36 angles 4 against 14 us a launch, 1024^2 x 72 angles 46 against 31.
-constexpr long long kDirectTaps = 4500000;  // image texels x subset angles x slices
+// whatever the size, the tiled forward kernels about 0.95 once their tiles fill the SMs; measured per
+// subset step with both (taps in millions): 64^2 x 9 angles, one slice (0.04) 5.9 against 8.7 us; 128^2
+// x 9 x ten slices (1.5) 13.6 against 17.0; 256^2 x 18, one (1.2) 10.8 against 12.0, three (3.5) 23.4
+// against 17.8; 300^2 x 25, one (2.2) 16.4 against 13.9; 384^2 x 27, one (4.0) 25.2 against 17.9.  The
+// line is drawn between 1.5 and 2.2.  The backprojector: one slice of 512^2 x 36 angles 4 against
+// 14 us a launch, 1024^2 x 72 angles 46 against 31.
+constexpr long long kDirectTaps = 1600000;  // image texels x subset angles x slices
 constexpr long long kDirectPixels = 600000; // image pixels x slices
 
 // grid: (ceil(px / 8), nrows, dN), kDirWarps warps.  meas != nullptr: OSEM1 ratio; else raw ray sums.
