@@ -33,14 +33,16 @@ struct xct_batch_plan {
     std::vector<int> sub;             // subset order (GPU.cpp:564-582)
     std::vector<XctItemDev> host;     // descriptors (pointers filled per run)
     XctItemDev *d_items = nullptr;
-    int *d_bases = nullptr;           // [3][m+1] over the graph's m slices
-    int *d_queues = nullptr;          // [it*ss][3]
+    int *d_bases = nullptr;           // prefix sums of the launches' work units
+    int *d_queues = nullptr;          // [it*ss][2]
     float2 *d_trig = nullptr;
     float *d_ratio = nullptr;
     double *d_acc = nullptr;
-    int grids[3] = {0, 0, 0};
-    int fwd_T = 92, fwd_chunk = 128;  // forward tiles of every slice (autotuned, cached)
-    std::vector<int> bases;           // [3][n+1] work-unit prefix sums for fwd_T, fwd_chunk
+    XctBatchStep step;                // the launches of one subset step
+    XctBatchSide side;
+    int fwd_T = 92, fwd_chunk = 128;  // forward tiles of the single slices
+    bool tuned = false;               // ... from the autotuner or its cache
+    std::vector<int> bases;           // host copy of d_bases
     size_t n_acc = 0;
     std::string key;                  // tune-cache key of the batch's shapes
     cudaStream_t cap = nullptr;       // capture stream
@@ -68,10 +70,13 @@ struct xct_batch_plan {
         size_t nprj = 0, nimg = 0;
     };
     std::vector<Group> groups;
+    std::vector<std::vector<int>> classes;  // the slices of each geometry, in order
     std::vector<int> rest;
     bool grouping = true;          // xct_batch_plan_set_grouping
     float *d_gscratch = nullptr;   // [batch][pa][px] sinograms then [batch][ny][nx] images
-    std::vector<int> glist;        // the graph's slices, in descriptor order
+    std::vector<int> want;         // the graph's slices, in item order
+    std::vector<int> glist;        // the same in descriptor order: packs of four, of two, singles
+    bool packing = true;           // with which setting of `grouping` glist was laid out
     std::vector<XctItemDev> gdesc; // their descriptors
     bool glist_corr = false;       // some slice of the graph has a sinogram correction
 };
@@ -81,6 +86,11 @@ static void batch_free(xct_batch_plan *p)
     if (!p) return;
     if (p->exec) cudaGraphExecDestroy(p->exec);
     if (p->cap) cudaStreamDestroy(p->cap);
+    for (int j = 0; j < 2; ++j) {
+        if (p->side.stream[j]) cudaStreamDestroy(p->side.stream[j]);
+        if (p->side.join[j]) cudaEventDestroy(p->side.join[j]);
+    }
+    if (p->side.fork) cudaEventDestroy(p->side.fork);
     cudaFree(p->d_items);
     cudaFree(p->d_bases);
     cudaFree(p->d_queues);
@@ -97,32 +107,166 @@ static void batch_free(xct_batch_plan *p)
     delete p;
 }
 
-// Forward tiles (T, chunk) for every slice: work units, their prefix sums over the graph's
-// slices (uploaded), the persistent grids; a captured graph is dropped (the next run
-// captures again).
-static int batch_layout(xct_batch_plan *p, int T, int chunk)
+// How the graph serves its slices: packs of four, of two and singles (their members one after the
+// other), and the packs' angle chunks.
+struct Arrangement {
+    std::vector<int> list[3];
+    int chunk[2] = {0, 0};
+};
+
+// Modelled forward work and tail of packs of S slices (first members in `firsts`) with tile side T, and
+// the angle chunk of least time.
+static int pack_chunk(const xct_batch_plan *p, int S, int T, const std::vector<int> &firsts, double &work, double &tail)
 {
-    std::vector<int> units(3 * p->host.size());  // forward, finalize, backprojection units
-    for (size_t i = 0; i < p->host.size(); ++i) {
-        XctItemDev &d = p->host[i];
-        d.g.fwd_T = T;
-        d.g.fwd_chunk = chunk;
-        xct_batched_units(d.g, d.fwd_ntx, d.fwd_nty, units[3 * i], units[3 * i + 1], d.bp_ntx, units[3 * i + 2]);
+    int best = 0;
+    const double sms = p->ctx->sm_count;
+    for (int c = fwd_tiled_rows_cap(); c >= 4; c -= std::max(1, c / 8)) {
+        double w = 0.0, t = 0.0;
+        for (int i : firsts) {
+            const KGeom &g = p->host[i].g;
+            double ti;
+            w += xct_fwd_work(g.nx, g.ny, S, T, (g.pa + g.ss - 1) / g.ss, c, 1, ti);
+            t = std::max(t, ti);
+        }
+        if (best == 0 || w / sms + t < work / sms + tail) {
+            best = c;
+            work = w;
+            tail = t;
+        }
     }
-    const int m = (int)p->glist.size();
-    p->bases.assign(3 * (size_t)(m + 1), 0);
-    p->glist_corr = false;
-    for (int j = 0; j < m; ++j) {
-        const int i = p->glist[j];
-        for (int q = 0; q < 3; ++q) p->bases[q * (m + 1) + j + 1] = p->bases[q * (m + 1) + j] + units[3 * i + q];
-        p->glist_corr = p->glist_corr || p->host[i].corr_mode > 0;
+    return best;
+}
+
+// Slices of one geometry are packed (with `grouping` on) in fours and twos, twos or not at all,
+// whichever has the least modelled forward time: a pack does less work per slice, but a few small
+// slices fill the SMs better one by one.
+static Arrangement arrange(const xct_batch_plan *p, const std::vector<int> &want)
+{
+    std::vector<char> in(p->n, 0);
+    for (int i : want) in[i] = 1;
+    const double sms = p->ctx->sm_count;
+    Arrangement best;
+    double least = 0.0;
+    for (int most = p->grouping ? 4 : 1; most >= 1; most /= 2) {
+        Arrangement a;
+        std::vector<int> firsts[2];
+        for (const auto &c : p->classes) {
+            if (!in[c[0]]) continue;  // the graph serves all slices of a geometry or none
+            size_t at = 0;
+            for (int S = most; S > 1; S /= 2)
+                for (; at + S <= c.size(); at += S) {
+                    const int q = S == 4 ? 0 : 1;
+                    firsts[q].push_back(c[at]);
+                    a.list[q].insert(a.list[q].end(), c.begin() + at, c.begin() + at + S);
+                }
+            a.list[2].insert(a.list[2].end(), c.begin() + at, c.end());
+        }
+        std::sort(a.list[2].begin(), a.list[2].end());
+        double work = 0.0, tail = 0.0;
+        auto add = [&](double w, double t) {
+            work += w;
+            tail = std::max(tail, t);
+        };
+        for (int q = 0; q < 2; ++q)
+            if (!firsts[q].empty()) {
+                const int S = q == 0 ? 4 : 2;
+                double w = 0.0, t = 0.0;
+                a.chunk[q] = pack_chunk(p, S, xct_pack_tile(S), firsts[q], w, t);
+                add(w, t);
+            }
+        if (!a.list[2].empty()) {
+            double w = 0.0, t = 0.0;
+            for (int T : {92, 76, 60, 44}) {
+                double wi = 0.0, ti = 0.0;
+                pack_chunk(p, 1, T, a.list[2], wi, ti);
+                if (T == 92 || wi / sms + ti < w / sms + t) w = wi, t = ti;
+            }
+            add(w, t);
+        }
+        const double cost = work / sms + tail;
+        if (most == 4 || !p->grouping || cost < least) {
+            least = cost;
+            best = std::move(a);
+        }
     }
-    XCT_CUDA_TRY(cudaMemcpy(p->d_bases, p->bases.data(), sizeof(int) * p->bases.size(), cudaMemcpyHostToDevice));
-    int rc = xct_batched_grids(p->ctx->device, p->ctx->sm_count, T, p->grids);
-    if (rc) return rc;
+    return best;
+}
+
+// Forward tiles of the single slices when nothing was tuned (of every slice when all are packed).
+static TuneChoice default_tiles(const xct_batch_plan *p, const Arrangement &a, const std::vector<int> &want)
+{
+    const std::vector<int> &of = a.list[2].empty() ? want : a.list[2];
+    return xct_tune_default(p->ctx->sm_count, [&](int T, int ch) {
+        long long t = 0;
+        for (int i : of) {
+            const KGeom &g = p->host[i].g;
+            const int rows = (g.pa + g.ss - 1) / g.ss;
+            t += (long long)((g.nx + T) / T) * ((g.ny + T) / T) * ((rows + ch - 1) / ch);
+        }
+        return t;
+    });
+}
+
+// The graph's slices `want` in descriptor order and the launches of a subset step: work units,
+// prefix sums (uploaded), grids; `tiles`: the single slices' (null: the tuned choice, else the default
+// rule).  A captured graph is dropped (the next run captures again).
+static int batch_layout(xct_batch_plan *p, const std::vector<int> &want, const TuneChoice *tiles)
+{
+    const Arrangement a = arrange(p, want);
+    const TuneChoice c = tiles ? *tiles : p->tuned ? TuneChoice{p->fwd_T, p->fwd_chunk, 0.0f} : default_tiles(p, a, want);
+    const int T = c.T, chunk = c.chunk;
+    const std::vector<int> *list = a.list;
+    const int *pack_ch = a.chunk;
+    p->want = want;
+    p->packing = p->grouping;
+    p->glist.clear();
+    XctBatchStep &b = p->step;
+    b = XctBatchStep();
+    b.items = p->d_items;
+    b.m = (int)want.size();
+    p->bases.clear();
+    size_t at_fwd[3], at_bp[3];
+    std::vector<int> fin(1, 0);
+    for (int q = 0; q < 3; ++q) {
+        const int S = q == 0 ? 4 : q == 1 ? 2 : 1;
+        b.packs[q] = (int)list[q].size() / S;
+        std::vector<int> f(1, 0), r(1, 0);
+        for (size_t j = 0; j < list[q].size(); ++j) {
+            XctItemDev &d = p->host[list[q][j]];
+            d.g.fwd_T = S > 1 ? xct_pack_tile(S) : T;
+            d.g.fwd_chunk = S > 1 ? pack_ch[q] : chunk;
+            int uf, un, ub;
+            xct_batched_units(d.g, S, d.fwd_ntx, d.fwd_nty, uf, un, d.bp_ntx, ub);
+            if (j % S == 0) {
+                f.push_back(f.back() + uf);
+                r.push_back(r.back() + ub);
+            }
+            fin.push_back(fin.back() + un);
+            p->glist.push_back(list[q][j]);
+        }
+        b.fwd_units[q] = f.back();
+        b.bp_units[q] = r.back();
+        at_fwd[q] = p->bases.size();
+        p->bases.insert(p->bases.end(), f.begin(), f.end());
+        at_bp[q] = p->bases.size();
+        p->bases.insert(p->bases.end(), r.begin(), r.end());
+    }
+    const size_t at_fin = p->bases.size();
+    p->bases.insert(p->bases.end(), fin.begin(), fin.end());
     // the finalize step runs one CTA per unit (ratio row) rather than a persistent grid: its
     // units are short, so a device queue's per-unit latency would dominate
-    p->grids[1] = p->bases[1 * (m + 1) + m];
+    b.fin_units = fin.back();
+    for (int q = 0; q < 3; ++q) {
+        b.fwd_base[q] = p->d_bases + at_fwd[q];
+        b.bp_base[q] = p->d_bases + at_bp[q];
+    }
+    b.fin_base = p->d_bases + at_fin;
+    p->glist_corr = false;
+    for (int i : want) p->glist_corr = p->glist_corr || p->host[i].corr_mode > 0;
+    XCT_CUDA_TRY(cudaMemcpy(p->d_bases, p->bases.data(), sizeof(int) * p->bases.size(), cudaMemcpyHostToDevice));
+    b.fwd_T = T;
+    int rc = xct_batched_grids(p->ctx->sm_count, T, b.fwd_grid, b.bp_grid);
+    if (rc) return rc;
     p->fwd_T = T;
     p->fwd_chunk = chunk;
     if (p->exec) {
@@ -180,7 +324,7 @@ static std::vector<int> all_items(int n)
 static std::string graph_key(const xct_batch_plan *p)
 {
     unsigned long long h = 1469598103934665603ull;  // FNV-1a over the shapes
-    for (int i : p->glist) {
+    for (int i : p->want) {
         const KGeom &g = p->host[i].g;
         const int v[6] = {g.nx, g.ny, g.px, g.pa, p->host[i].cover ? 1 : 0, 0};
         for (int q = 0; q < 6; ++q) {
@@ -189,8 +333,8 @@ static std::string graph_key(const xct_batch_plan *p)
         }
     }
     char kb[96];
-    snprintf(kb, sizeof kb, "batch%d-%016llx", (int)p->glist.size(), h);
-    return xct_tune_key(p->ctx->name, 0, 0, 0, 0, p->ss, (int)p->glist.size()) + "|" + kb;
+    snprintf(kb, sizeof kb, "batch%d-%016llx", (int)p->want.size(), h);
+    return xct_tune_key(p->ctx->name, 0, 0, 0, 0, p->ss, (int)p->want.size()) + "|" + kb;
 }
 
 extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms, int it, xct_batch_plan **out)
@@ -219,6 +363,45 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
         batch_free(p);
         return r;
     };
+    // geometry groups: slices of one geometry, found through a hash of the geometry and
+    // checked member by member
+    {
+        std::vector<std::pair<unsigned long long, int>> hs(n);
+        for (int i = 0; i < n; ++i) hs[i] = {geom_hash(geoms[i]), i};
+        std::stable_sort(hs.begin(), hs.end());
+        std::vector<char> taken(n, 0);
+        for (size_t a0 = 0; a0 < hs.size();) {
+            size_t a1 = a0;
+            while (a1 < hs.size() && hs[a1].first == hs[a0].first) ++a1;
+            for (size_t u = a0; u < a1; ++u) {
+                const int i = hs[u].second;
+                if (taken[i]) continue;
+                std::vector<int> members{i};
+                taken[i] = 1;
+                for (size_t v = u + 1; v < a1; ++v) {
+                    const int j = hs[v].second;
+                    if (!taken[j] && same_geom(geoms[i], geoms[j])) {
+                        members.push_back(j);
+                        taken[j] = 1;
+                    }
+                }
+                std::sort(members.begin(), members.end());
+                p->classes.push_back(members);
+                if ((int)members.size() >= kGroupMin) {
+                    xct_batch_plan::Group G;
+                    G.items = members;
+                    p->groups.push_back(std::move(G));
+                } else {
+                    p->rest.insert(p->rest.end(), members.begin(), members.end());
+                }
+            }
+            a0 = a1;
+        }
+        std::sort(p->classes.begin(), p->classes.end());  // (by their first slices)
+        std::sort(p->rest.begin(), p->rest.end());
+        std::sort(p->groups.begin(), p->groups.end(),
+                  [](const xct_batch_plan::Group &x, const xct_batch_plan::Group &y) { return x.items[0] < y.items[0]; });
+    }
     // sizes
     size_t n_trig = 0, n_ratio = 0, n_acc = 0, n_corr = 0, n_fac = 0;
     p->host.resize(n);
@@ -250,12 +433,14 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
             n_fac += 2 * (size_t)g.pa + g.px;
         }
     }
+    n_ratio += 3 * p->classes.size();  // each geometry's ratio images start on 16 bytes
     cudaError_t e;
     if ((e = cudaMalloc(&p->d_items, sizeof(XctItemDev) * n)) != cudaSuccess) return fail(e, "cudaMalloc items");
-    if ((e = cudaMalloc(&p->d_bases, sizeof(int) * 3 * (size_t)(n + 1))) != cudaSuccess)
+    // prefix sums: two per pack size and one over the slices
+    if ((e = cudaMalloc(&p->d_bases, sizeof(int) * (3 * (size_t)n + 7))) != cudaSuccess)
         return fail(e, "cudaMalloc bases");
     p->n_acc = n_acc;
-    p->queue_bytes = sizeof(int) * 3 * (size_t)std::max(1, it * ss);
+    p->queue_bytes = sizeof(int) * 2 * (size_t)std::max(1, it * ss);
     if ((e = cudaMalloc(&p->d_queues, p->queue_bytes)) != cudaSuccess) return fail(e, "cudaMalloc queues");
     if ((e = cudaMalloc(&p->d_trig, sizeof(float2) * n_trig)) != cudaSuccess) return fail(e, "cudaMalloc trig");
     if ((e = cudaMalloc(&p->d_ratio, sizeof(float) * n_ratio)) != cudaSuccess) return fail(e, "cudaMalloc ratio");
@@ -268,7 +453,16 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
         if ((e = cudaMalloc(&p->d_corr, sizeof(float) * n_corr)) != cudaSuccess) return fail(e, "cudaMalloc corr");
         if ((e = cudaMalloc(&p->d_corr_fac, sizeof(float) * n_fac)) != cudaSuccess) return fail(e, "cudaMalloc fac");
     }
-    size_t ot = 0, orat = 0, oacc = 0, ocorr = 0, ofac = 0;
+    // the ratio images of one geometry lie one after the other (the packs' backprojector reads them so)
+    size_t orat = 0;
+    for (const auto &c : p->classes) {
+        orat = (orat + 3) / 4 * 4;
+        for (int i : c) {
+            p->host[i].ratio = p->d_ratio + orat;
+            orat += (size_t)geoms[i].pa * geoms[i].px;
+        }
+    }
+    size_t ot = 0, oacc = 0, ocorr = 0, ofac = 0;
     std::vector<float2> cs;
     std::vector<float> af, bf;
     for (int i = 0; i < n; ++i) {
@@ -278,7 +472,6 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
         if ((e = cudaMemcpy(p->d_trig + ot, cs.data(), sizeof(float2) * g.pa, cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(e, "upload trig");
         d.trig = p->d_trig + ot;
-        d.ratio = p->d_ratio + orat;
         d.acc = p->d_acc + oacc;
         d.sino = nullptr;
         d.img = nullptr;
@@ -300,45 +493,7 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
             ofac += af.size() + bf.size();
         }
         ot += g.pa;
-        orat += (size_t)g.pa * g.px;
         oacc += (size_t)((g.pa + g.ss - 1) / g.ss) * g.px;
-    }
-    // geometry groups: slices of one geometry, found through a hash of the geometry and
-    // checked member by member
-    {
-        std::vector<std::pair<unsigned long long, int>> hs(n);
-        for (int i = 0; i < n; ++i) hs[i] = {geom_hash(geoms[i]), i};
-        std::stable_sort(hs.begin(), hs.end());
-        std::vector<char> taken(n, 0);
-        for (size_t a0 = 0; a0 < hs.size();) {
-            size_t a1 = a0;
-            while (a1 < hs.size() && hs[a1].first == hs[a0].first) ++a1;
-            for (size_t u = a0; u < a1; ++u) {
-                const int i = hs[u].second;
-                if (taken[i]) continue;
-                std::vector<int> members{i};
-                taken[i] = 1;
-                for (size_t v = u + 1; v < a1; ++v) {
-                    const int j = hs[v].second;
-                    if (!taken[j] && same_geom(geoms[i], geoms[j])) {
-                        members.push_back(j);
-                        taken[j] = 1;
-                    }
-                }
-                std::sort(members.begin(), members.end());
-                if ((int)members.size() >= kGroupMin) {
-                    xct_batch_plan::Group G;
-                    G.items = members;
-                    p->groups.push_back(std::move(G));
-                } else {
-                    p->rest.insert(p->rest.end(), members.begin(), members.end());
-                }
-            }
-            a0 = a1;
-        }
-        std::sort(p->rest.begin(), p->rest.end());
-        std::sort(p->groups.begin(), p->groups.end(),
-                  [](const xct_batch_plan::Group &x, const xct_batch_plan::Group &y) { return x.items[0] < y.items[0]; });
     }
     size_t scratch = 0;
     for (auto &G : p->groups) {
@@ -361,24 +516,21 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
     // the graph's slices with groups in use (every slice when all are grouped: the graph
     // then serves them only with groups off), its tiles: this list's cached choice, else the
     // default rule
-    p->glist = p->rest.empty() ? all_items(n) : p->rest;
+    p->want = p->rest.empty() ? all_items(n) : p->rest;
     p->key = graph_key(p);
     TuneChoice c;
-    if (!xct_tune_lookup(p->key, xct_tune_env_path(), c))
-        c = xct_tune_default(ctx->sm_count, [&](int T, int ch) {
-            long long t = 0;
-            for (int i : p->glist) {
-                const int rows = (geoms[i].pa + ss - 1) / ss;
-                t += (long long)((geoms[i].nx + T) / T) * ((geoms[i].ny + T) / T) * ((rows + ch - 1) / ch);
-            }
-            return t;
-        });
-    int rc = batch_layout(p, c.T, c.chunk);
+    p->tuned = xct_tune_lookup(p->key, xct_tune_env_path(), c);
+    int rc = batch_layout(p, std::vector<int>(p->want), p->tuned ? &c : nullptr);
     if (rc) {
         batch_free(p);
         return rc;
     }
     if ((e = cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "stream");
+    for (int j = 0; j < 2; ++j) {
+        if ((e = cudaStreamCreateWithFlags(&p->side.stream[j], cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "stream");
+        if ((e = cudaEventCreateWithFlags(&p->side.join[j], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
+    }
+    if ((e = cudaEventCreateWithFlags(&p->side.fork, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
     *out = p;
     return XCT_OK;
 }
@@ -415,8 +567,8 @@ static int capture(xct_batch_plan *p)
                 rc = launch_ista3d_stacks(p->d_stacks, ns, p->max_vox, p->cs_lambda, sm, p->cap);
                 first = false;
             } else {
-                rc = launch_osem_step_batched(p->d_items, p->d_bases, m, p->sub[k],
-                                              p->d_queues + 3 * (size_t)(i * p->ss + k), p->grids, p->fwd_T, p->cap);
+                rc = launch_osem_step_batched(p->step, p->sub[k], p->d_queues + 2 * (size_t)(i * p->ss + k), p->cap,
+                                              p->side);
                 if (rc == XCT_OK && cs) rc = launch_fista3d_stacks(p->d_stacks, ns, p->max_vox, p->cs_lambda, sm, p->cap);
             }
             if (rc == XCT_OK && cs) rc = launch_stack_copy(p->d_stacks, ns, p->max_vox, 0, sm, p->cap);
@@ -474,9 +626,8 @@ extern "C" int xct_batch_run(xct_batch_plan *p, const float *const *d_sino, floa
     }
     // the graph: the slices of no group, or every slice
     const std::vector<int> want = use_groups ? p->rest : all_items(p->n);
-    if (want != p->glist) {
-        p->glist = want;
-        int rc = batch_layout(p, p->fwd_T, p->fwd_chunk);
+    if (want != p->want || p->grouping != p->packing) {
+        int rc = batch_layout(p, want, nullptr);
         if (rc) return rc;
     }
     if (!p->exec) {
@@ -508,10 +659,12 @@ extern "C" int xct_batch_run(xct_batch_plan *p, const float *const *d_sino, floa
         XCT_CUDA_TRY(cudaMemcpyAsync(p->d_stacks, p->stacks.data(), sizeof(XctStackDev) * p->stacks.size(),
                                      cudaMemcpyHostToDevice, st));
     XCT_CUDA_TRY(cudaGraphLaunch(p->exec, st));
-    // three per OS-EM step (the first step has none with compressed sensing), the
-    // correction, and with compressed sensing the setup copy plus two per step
+    // a forward and a backprojection launch per pack size in use and the finalize per OS-EM step (the
+    // first step has none with compressed sensing), the correction, and with compressed sensing the setup copy plus two per step
     const long long steps = (long long)p->it * p->ss, cs = p->stacks.empty() ? 0 : 1;
-    g_xct_launches.fetch_add(3 * (steps - cs) + (p->glist_corr ? (m + 65534) / 65535 : 0) + cs * (1 + 2 * steps),
+    int sizes = 0;
+    for (int q = 0; q < 3; ++q) sizes += p->step.packs[q] > 0;
+    g_xct_launches.fetch_add((2 * sizes + 1) * (steps - cs) + (p->glist_corr ? (m + 65534) / 65535 : 0) + cs * (1 + 2 * steps),
                              std::memory_order_relaxed);
     return XCT_OK;
 }
@@ -640,15 +793,16 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
     // are grouped: the graph then serves them only with groups off)
     const bool use_groups = p->grouping && p->stacks.empty() && !p->groups.empty();
     const std::vector<int> want = use_groups && !p->rest.empty() ? p->rest : all_items(p->n);
-    if (want != p->glist) {
-        p->glist = want;
-        int rc = batch_layout(p, p->fwd_T, p->fwd_chunk);
+    if (want != p->want || p->grouping != p->packing) {
+        int rc = batch_layout(p, want, nullptr);
         if (rc) return rc;
     }
     p->key = graph_key(p);
     TuneChoice best;
-    if (!(flags & XCT_TUNE_FORCE) && xct_tune_lookup(p->key, cache_path, best))
-        return batch_layout(p, best.T, best.chunk);
+    if (!(flags & XCT_TUNE_FORCE) && xct_tune_lookup(p->key, cache_path, best)) {
+        p->tuned = true;
+        return batch_layout(p, want, &best);
+    }
     XCT_CUDA_TRY(cudaSetDevice(p->ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
     const int m = (int)p->glist.size();
@@ -665,13 +819,14 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    const int T0 = p->fwd_T, c0 = p->fwd_chunk;
-    best = TuneChoice{T0, c0, 3.0e38f};
+    const TuneChoice before{p->fwd_T, p->fwd_chunk, 3.0e38f};
+    best = before;
     int rc = cudaMemsetAsync(scratch, 0, sizeof(float) * maxpix, st) == cudaSuccess ? XCT_OK
                                                                                     : xct_fail(XCT_E_CUDA, "memset");
+    if (p->step.packs[2] == 0) best.ms = 0.0f;  // packs only: nothing to choose
     for (const TuneChoice &c : xct_tune_candidates(max_rows)) {
-        if (rc) break;
-        if ((rc = batch_layout(p, c.T, c.chunk))) break;
+        if (rc || p->step.packs[2] == 0) break;
+        if ((rc = batch_layout(p, want, &c))) break;
         for (int j = 0; j < m; ++j) {
             tmp[j] = p->host[p->glist[j]];
             tmp[j].img = scratch;
@@ -683,7 +838,7 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
             cudaMemsetAsync(p->d_acc, 0, sizeof(double) * p->n_acc, st);
             cudaMemsetAsync(p->d_queues, 0, sizeof(int), st);
             cudaEventRecord(e0, st);
-            rc = launch_fwd_batched(p->d_items, p->d_bases, m, p->sub[0], p->d_queues, p->grids[0], c.T, st);
+            rc = launch_fwd_batched(p->step, p->sub[0], p->d_queues, st);
             cudaEventRecord(e1, st);
             cudaError_t e = cudaEventSynchronize(e1);
             if (rc == XCT_OK && e != cudaSuccess) rc = xct_cuda_fail(e, "xct_batch_plan_autotune");
@@ -699,10 +854,11 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
     cudaEventDestroy(e1);
     cudaFree(scratch);
     if (rc) {
-        batch_layout(p, T0, c0);
+        batch_layout(p, want, &before);
         return rc;
     }
-    rc = batch_layout(p, best.T, best.chunk);
+    p->tuned = true;
+    rc = batch_layout(p, want, &best);
     if (rc) return rc;
     return xct_tune_store(p->key, cache_path, best);
 }

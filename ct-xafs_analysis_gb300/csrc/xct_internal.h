@@ -45,6 +45,23 @@ struct XctItemDev {
     const float *corr_bin;    // [px] per-bin correction factors
 };
 
+// The launches of one batched subset step: the graph's slices, in packs of four, packs of two and
+// single ones (q = 0, 1, 2), with each launch's units as prefix sums over the packs.
+struct XctBatchStep {
+    const XctItemDev *items = nullptr;
+    int m = 0;                   // slices
+    int packs[3] = {0, 0, 0};
+    const int *fwd_base[3] = {}, *bp_base[3] = {}, *fin_base = nullptr;  // device, [packs + 1], [m + 1]
+    int fwd_units[3] = {}, bp_units[3] = {}, fin_units = 0;
+    int fwd_T = 92, fwd_grid = 0, bp_grid = 0;  // the single slices' forward tile and persistent grids
+    int first(int q) const { return q == 0 ? 0 : q == 1 ? 4 * packs[0] : 4 * packs[0] + 2 * packs[1]; }
+};
+// Streams and events for the launches that run side by side.
+struct XctBatchSide {
+    cudaStream_t stream[2] = {};
+    cudaEvent_t fork = nullptr, join[2] = {};
+};
+
 // A stack of consecutive slices of one shape in a batch plan with compressed sensing: its
 // images form one [dN][ny][nx] array (the proximal step's third axis), with its own w, beta
 // and x' buffers of the same size.
@@ -136,6 +153,7 @@ int launch_fwd_tiled_main(const KGeom &g, const float2 *trig, const float *img, 
                           int nrows, cudaStream_t st);
 // Modelled time of a forward launch (see its definition), for the choice of tiles and chunks.
 double xct_fwd_cost(int nx, int ny, int S, int T, int nrows, int chunk, int groups, int sms);
+double xct_fwd_work(int nx, int ny, int S, int T, int nrows, int chunk, int groups, double &tail);
 // Slices per group of the slice-interleaved backprojectors.
 int fwd_ms_slices();
 int launch_fwd_finalize(const KGeom &g, const float *meas, float *out, double *acc, int dN, int sub, int step,
@@ -151,17 +169,16 @@ int launch_fwd_direct(const KGeom &g, const float2 *trig, const float *img, cons
                       int step, int nrows, cudaStream_t st);
 int launch_bp_update_direct(const KGeom &g, const float2 *trig, float *img, const float *ratio, int dN, int sub,
                             cudaStream_t st);
-// Batched launches (xct_tiled.cu): work units of one slice, persistent grid sizes, and one
-// subset step (forward, finalize, backprojection) over all slices; bases is [3][n+1]
-// prefix sums of the units of each kernel, queues 3 zeroed counters.
-void xct_batched_units(const KGeom &g, int &fwd_ntx, int &fwd_nty, int &fwd_units, int &fin_units, int &bp_ntx,
+// Batched launches (xct_tiled.cu): the work units of a pack of S slices of one geometry, the
+// persistent grids of the single slices, and one subset step (forward, finalize, backprojection) over
+// all slices.
+void xct_batched_units(const KGeom &g, int S, int &fwd_ntx, int &fwd_nty, int &fwd_units, int &fin_units, int &bp_ntx,
                        int &bp_units);
-int xct_batched_grids(int device, int sm_count, int fwd_T, int grids[3]);
-int launch_osem_step_batched(const XctItemDev *items, const int *bases, int n, int sub, int *queues,
-                             const int grids[3], int fwd_T, cudaStream_t st);
+int xct_pack_tile(int S);
+int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid);
+int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queues, cudaStream_t st, const XctBatchSide &side);
 bool xct_fwd_tile_valid(int T);
-int launch_fwd_batched(const XctItemDev *items, const int *bases, int n, int sub, int *queue, int grid, int fwd_T,
-                       cudaStream_t st);
+int launch_fwd_batched(const XctBatchStep &b, int sub, int *queue, cudaStream_t st);
 int xct_check_geom(const xct_geom *g);
 // Exact adjoint of the forward projector over all angles: img = A^T sino (overwrites img).
 int launch_adj_tiled(const KGeom &g, const float2 *trig, const float *sino, float *img, int dN, cudaStream_t st);

@@ -189,11 +189,11 @@ __device__ __forceinline__ float fwd_reduce(const float (&sum)[S], int ph, float
     return v;
 }
 
-// The work of one CTA: tile (bx, by) of S slices (images from im, accumulators from acc [S][nrows][px])
-// for the subset angles k0 .. k0+chunk-1 (chunk <= kAngChunk).  Starts and ends with all threads in
-// step.
-template <int S, int T>
-__device__ __forceinline__ void fwd_tile(const KGeom &g, const float *im, double *acc, const float2 *__restrict__ trig,
+// The work of one CTA: tile (bx, by) of S slices (slice z: image image(z), accumulator accum(z)
+// [nrows][px]) for the subset angles k0 .. k0+chunk-1 (chunk <= kAngChunk).  Starts and ends with all
+// threads in step.
+template <int S, int T, class Image, class Accum>
+__device__ __forceinline__ void fwd_tile(const KGeom &g, Image image, Accum accum, const float2 *__restrict__ trig,
                                          int sub, int step, int nrows, int bx, int by, int k0, int chunk,
                                          unsigned char *smem_raw)
 {
@@ -204,7 +204,6 @@ __device__ __forceinline__ void fwd_tile(const KGeom &g, const float *im, double
     const int kn = min(chunk, nrows - k0);
     if (kn <= 0) return;
     const int x0 = -1 + bx * T, y0 = -1 + by * T;
-    const size_t nimg = (size_t)g.nx * g.ny;
 
     // element (c, r) = (t(x0+c, y0+r), t(x0+c+1, y0+r) - t(x0+c, y0+r)), zero border.  A warp stages
     // rows of a slice: each texel is loaded once, its right neighbour comes from the next lane.
@@ -216,7 +215,7 @@ __device__ __forceinline__ void fwd_tile(const KGeom &g, const float *im, double
             const int z = q / C::Rows, r = q - z * C::Rows;
             const int gy = y0 + r;
             const bool rv = (unsigned)gy < (unsigned)g.ny;
-            const float *row = im + (size_t)z * nimg + ((long long)gy * g.nx + x0);
+            const float *row = image(z) + ((long long)gy * g.nx + x0);
             float t[kCols + 1];
 #pragma unroll
             for (int u = 0; u < kCols; ++u) {
@@ -288,7 +287,7 @@ __device__ __forceinline__ void fwd_tile(const KGeom &g, const float *im, double
     const bool bound_x = ph < 2;
     const bool upper = (ph & 1) != 0;
     const float blo = bound_x ? xlo : ylo, bhi = bound_x ? xhi : yhi;
-    double *accl = acc + (S > 1 ? (size_t)(ph < S ? ph : 0) * nrows * g.px : 0);
+    double *accl = accum(S > 1 && ph < S ? ph : 0);
 
     // items (angle, 8 consecutive rays), strided over the warps
     int k = 0;
@@ -368,7 +367,7 @@ __device__ __forceinline__ void fwd_tile(const KGeom &g, const float *im, double
         if (len > 0 && XCT_IN((long long)(k0 + k) * g.px + X, 0, (long long)nrows * g.px - 1, XCT_SITE_FWD_ACC)) {
             const size_t o = (size_t)(k0 + k) * g.px + X;
             if (ph < S) atomicAdd(accl + o, (double)tot);
-            if (S == 5 && ph == 0) atomicAdd(acc + (size_t)4 * nrows * g.px + o, (double)fifth);
+            if (S == 5 && ph == 0) atomicAdd(accum(S - 1) + o, (double)fifth);
         }
     }
 }
@@ -382,9 +381,13 @@ __global__ void __launch_bounds__(FwdTile<S, T>::Threads, FwdTile<S, T>::MinBloc
     extern __shared__ __align__(16) unsigned char smem_raw[];
     xct_grid_wait();
     xct_grid_trigger();
-    const size_t z = (size_t)blockIdx.z * S;
-    fwd_tile<S, T>(g, img + z * g.nx * g.ny, acc + z * nrows * g.px, trig, sub, step, nrows, (int)blockIdx.x % ntx,
-                   (int)blockIdx.x / ntx, (int)blockIdx.y * chunk, chunk, smem_raw);
+    const size_t z0 = (size_t)blockIdx.z * S, nimg = (size_t)g.nx * g.ny, nacc = (size_t)nrows * g.px;
+    const float *im = img + z0 * nimg;
+    double *ac = acc + z0 * nacc;
+    fwd_tile<S, T>(
+        g, [&](int z) { return S == 1 ? im : im + (size_t)z * nimg; },
+        [&](int z) { return S == 1 ? ac : ac + (size_t)z * nacc; }, trig, sub, step, nrows,
+        (int)blockIdx.x % ntx, (int)blockIdx.x / ntx, (int)blockIdx.y * chunk, chunk, smem_raw);
 }
 
 // acc -> OSEM1 ratio (meas != nullptr) or raw projection, rows th = sub + k*step; clears acc.
@@ -601,22 +604,16 @@ __device__ __forceinline__ void bp_loads(unsigned ad, float (&v)[S])
     }
 }
 
-// grid: (ntx*nty tiles of 32 x 32, 1, dN / S slice groups).  vec: 16-byte staging
-// copies (px a multiple of 4 and a 16-byte aligned ratio array).
-template <int S>
-__global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const float *ratio,
-                                                             const float2 *__restrict__ trig, KGeom g, int sub,
-                                                             int nang, int ntx, float ssf, float paf, int vec)
+// The work of one CTA: pixel tile (bx, by) of S slices (slice z: image image(z), ratio rz + z * pa * px).
+// vec: 16-byte staging copies (px a multiple of 4 and a 16-byte aligned rz).
+template <int S, class Image>
+__device__ __forceinline__ void bp_ms_tile(const KGeom &g, Image image, const float *rz, const float2 *__restrict__ trig,
+                                           int sub, int nang, int bx, int by, float ssf, float paf, int vec,
+                                           BpMsShared<S> &sh)
 {
     typedef BpMsShared<S> C;
     constexpr int kAcc = S == 1 ? kBpMsPix / 2 : kBpMsPix * (S / 2);
-    __shared__ __align__(16) C sh;
-    xct_grid_wait();
-    xct_grid_trigger();
-    const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
-    const int z0 = (int)blockIdx.z * S;
-    const size_t nimg = (size_t)g.nx * g.ny, nprj = (size_t)g.pa * g.px;
-    const float *rz = ratio + (size_t)z0 * nprj;
+    const size_t nprj = (size_t)g.pa * g.px;
     const int X0 = bx * kBpMsT, Y0 = by * kBpMsT;
     const int X1 = min(X0 + kBpMsT, g.nx) - 1, Y1 = min(Y0 + kBpMsT, g.ny) - 1;
     const int t = threadIdx.x;
@@ -727,30 +724,53 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
     for (int i = 0; i < kBpMsPix; ++i) {
         const int X = X0 + tx + 8 * i;
         if (X > X1) continue;
-        float *p0 = img + (size_t)z0 * nimg + (size_t)Y * g.nx + X;
+        const size_t o = (size_t)Y * g.nx + X;
         if constexpr (S == 1) {
             float v0, v1;
             f2_unpack(acc[i / 2], v0, v1);
-            *p0 = xct_update(*p0, i & 1 ? v1 : v0, ssf, paf);
+            float *p = image(0) + o;
+            *p = xct_update(*p, i & 1 ? v1 : v0, ssf, paf);
         } else {
 #pragma unroll
             for (int h = 0; h < S / 2; ++h) {
                 float v0, v1;
                 f2_unpack(acc[i * (S / 2) + h], v0, v1);
-                float *p = p0 + (size_t)(2 * h) * nimg;
+                float *p = image(2 * h) + o;
                 *p = xct_update(*p, v0, ssf, paf);
-                p += nimg;
+                p = image(2 * h + 1) + o;
                 *p = xct_update(*p, v1, ssf, paf);
             }
         }
     }
 }
 
+// grid: (ntx*nty tiles of 32 x 32, 1, dN / S slice groups).
+template <int S>
+__global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const float *ratio,
+                                                             const float2 *__restrict__ trig, KGeom g, int sub,
+                                                             int nang, int ntx, float ssf, float paf, int vec)
+{
+    __shared__ __align__(16) BpMsShared<S> sh;
+    xct_grid_wait();
+    xct_grid_trigger();
+    const size_t z0 = (size_t)blockIdx.z * S, nimg = (size_t)g.nx * g.ny;
+    float *im = img + z0 * nimg;
+    bp_ms_tile<S>(
+        g, [&](int z) { return im + (size_t)z * nimg; }, ratio + z0 * ((size_t)g.pa * g.px), trig, sub, nang,
+        (int)blockIdx.x % ntx, (int)blockIdx.x / ntx, ssf, paf, vec, sh);
+}
+
 // ----------------------------------------------------------------- batched launches
-// One subset step of many slices of different shapes in one persistent launch per kernel:
-// CTAs take (slice, tile) work units from a device queue (an atomic counter) until the
-// units run out.  Units of slice i are [base[i], base[i+1]); they are independent within a
-// launch, so there is no waiting on other CTAs.
+// One subset step of many slices of different shapes, one launch per kernel and pack size.  Slices
+// of one geometry go in packs of four and of two through the grouped forward projector and the
+// several-slice backprojector, one CTA per (pack, tile) unit; the others one by one through persistent
+// CTAs that take (slice, tile) units from a device queue (an atomic counter) until the units run
+// out.  Units of pack (slice) i are [base[i], base[i+1]); they are independent within a launch, so
+// there is no waiting on other CTAs.
+// A pack pays per slice what the forward and backward kernels of several slices save (coordinates,
+// addresses and weights once): one iteration of 24 slices, 12 geometries 512 to 2048 wide, takes 30.3 ms
+// in packs of two and 43.3 one by one; 21 of seven geometries 570 to 1140 wide, in packs of two and
+// single slices, 6.7 against about 7.3.
 __device__ __forceinline__ int queue_take(int *queue, int *s_unit)
 {
     if (threadIdx.x == 0) *s_unit = atomicAdd(queue, 1);
@@ -796,10 +816,30 @@ __global__ void __launch_bounds__(FwdTile<1, T>::Threads, FwdTile<1, T>::MinBloc
         const int local = u - base[i];
         const int tiles = it.fwd_ntx * it.fwd_nty;
         const int t = local % tiles, ch = local / tiles;
-        fwd_tile<1, T>(g, it.img, it.acc, it.trig, sub, g.ss, nrows, t % it.fwd_ntx, t / it.fwd_ntx, ch * g.fwd_chunk,
-                    g.fwd_chunk, smem_raw);
+        fwd_tile<1, T>(
+            g, [&](int) { return it.img; }, [&](int) { return it.acc; }, it.trig, sub, g.ss, nrows, t % it.fwd_ntx,
+            t / it.fwd_ntx, ch * g.fwd_chunk, g.fwd_chunk, smem_raw);
         __syncthreads();  // the tile in shared memory is restaged by the next unit
     }
+}
+
+// grid: one CTA per forward unit; pack i is the slices items[i * S] .. items[i * S + S - 1].
+template <int S, int T>
+__global__ void __launch_bounds__(FwdTile<S, T>::Threads, FwdTile<S, T>::MinBlocks)
+    fwd_pack_kernel(const XctItemDev *__restrict__ items, const int *__restrict__ base, int n, int sub)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_item;
+    const int u = blockIdx.x, i = unit_item(base, n, u, &s_item);
+    const XctItemDev *pk = items + (size_t)i * S;
+    const KGeom &g = pk->g;
+    const int nrows = pk->cover ? (g.pa - sub + g.ss - 1) / g.ss : g.pa / g.ss;
+    const int local = u - base[i];
+    const int tiles = pk->fwd_ntx * pk->fwd_nty;
+    const int t = local % tiles, ch = local / tiles;
+    fwd_tile<S, T>(
+        g, [&](int z) { return pk[z].img; }, [&](int z) { return pk[z].acc; }, pk->trig, sub, g.ss, nrows, t % pk->fwd_ntx,
+        t / pk->fwd_ntx, ch * g.fwd_chunk, g.fwd_chunk, smem_raw);
 }
 
 // grid: one CTA per finalize unit (a ratio row of an item's largest subset), base[n] of them.
@@ -844,6 +884,24 @@ __global__ void __launch_bounds__(BpCfg<4>::Threads) bp_batched_kernel(const Xct
     }
 }
 
+// grid: one CTA per backprojection unit; a pack's ratio images lie one after the other.
+template <int S>
+__global__ void __launch_bounds__(kBpMsThreads) bp_pack_kernel(const XctItemDev *__restrict__ items,
+                                                               const int *__restrict__ base, int n, int sub)
+{
+    __shared__ __align__(16) BpMsShared<S> sh;
+    __shared__ int s_item;
+    const int u = blockIdx.x, i = unit_item(base, n, u, &s_item);
+    const XctItemDev *pk = items + (size_t)i * S;
+    const KGeom &g = pk->g;
+    const int nang = (g.pa - sub + g.ss - 1) / g.ss;
+    const int t = u - base[i];
+    const int vec = g.px % 4 == 0 && ((size_t)pk->ratio & 15u) == 0;
+    bp_ms_tile<S>(
+        g, [&](int z) { return pk[z].img; }, pk->ratio, pk->trig, sub, nang, t % pk->bp_ntx, t / pk->bp_ntx, (float)g.ss,
+        (float)g.pa, vec, sh);
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------- tile-size dispatch
@@ -877,7 +935,8 @@ static int with_tile(int T, F &&f)
     }
 }
 
-void xct_batched_units(const KGeom &g, int &fwd_ntx, int &fwd_nty, int &fwd_units, int &fin_units, int &bp_ntx,
+// Work units of a pack of S slices (the forward tile side and chunk are g.fwd_T and g.fwd_chunk).
+void xct_batched_units(const KGeom &g, int S, int &fwd_ntx, int &fwd_nty, int &fwd_units, int &fin_units, int &bp_ntx,
                        int &bp_units)
 {
     fwd_ntx = (g.nx + 1 + g.fwd_T - 1) / g.fwd_T;
@@ -885,13 +944,17 @@ void xct_batched_units(const KGeom &g, int &fwd_ntx, int &fwd_nty, int &fwd_unit
     const int rows = (g.pa + g.ss - 1) / g.ss;  // the largest subset (cover mode)
     fwd_units = fwd_ntx * fwd_nty * ((rows + g.fwd_chunk - 1) / g.fwd_chunk);
     fin_units = rows;
-    bp_ntx = (g.nx + kBpTX - 1) / kBpTX;
-    bp_units = bp_ntx * ((g.ny + kBpTY - 1) / kBpTY);
+    const int tx = S > 1 ? kBpMsT : kBpTX, ty = S > 1 ? kBpMsT : kBpTY;
+    bp_ntx = (g.nx + tx - 1) / tx;
+    bp_units = bp_ntx * ((g.ny + ty - 1) / ty);
 }
 
-int xct_batched_grids(int device, int sm_count, int fwd_T, int grids[3])
+// Forward tile side of a pack of S slices.
+int xct_pack_tile(int S) { return S == 4 ? FwdGroup<4>::T : FwdGroup<2>::T; }
+
+// Persistent grids of the single slices' launches; the packs' shared-memory limits.
+int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid)
 {
-    (void)device;
     int a = 0, c = 0;
     int rc = with_tile(fwd_T, [&](auto tc) -> int {
         constexpr int T = decltype(tc)::value;
@@ -904,40 +967,77 @@ int xct_batched_grids(int device, int sm_count, int fwd_T, int grids[3])
     });
     if (rc) return rc;
     XCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, bp_batched_kernel, BpCfg<4>::Threads, 0));
-    grids[0] = sm_count * (a > 0 ? a : 1);
-    grids[1] = 0;  // the finalize grid is the plan's unit count
-    grids[2] = sm_count * (c > 0 ? c : 1);
+    fwd_grid = sm_count * (a > 0 ? a : 1);
+    bp_grid = sm_count * (c > 0 ? c : 1);
     return XCT_OK;
 }
 
-int launch_osem_step_batched(const XctItemDev *items, const int *bases /*[3][n+1]*/, int n, int sub,
-                             int *queues /*[3]*/, const int grids[3], int fwd_T, cudaStream_t st)
+template <int S>
+static int launch_fwd_pack(const XctBatchStep &b, int q, int sub, cudaStream_t st)
 {
-    int rc = with_tile(fwd_T, [&](auto tc) -> int {
+    constexpr int T = FwdGroup<S>::T;
+    static std::atomic<bool> done[64];
+    const int r = smem_attr((const void *)fwd_pack_kernel<S, T>, FwdTile<S, T>::Smem, done);
+    if (r) return r;
+    fwd_pack_kernel<S, T><<<b.fwd_units[q], FwdTile<S, T>::Threads, FwdTile<S, T>::Smem, st>>>(
+        b.items + b.first(q), b.fwd_base[q], b.packs[q], sub);
+    XCT_CUDA_TRY(cudaGetLastError());
+    return XCT_OK;
+}
+
+// The forward launch of the single slices of one subset step (the autotuner times it alone).
+int launch_fwd_batched(const XctBatchStep &b, int sub, int *queue, cudaStream_t st)
+{
+    return with_tile(b.fwd_T, [&](auto tc) -> int {
         constexpr int T = decltype(tc)::value;
-        fwd_batched_kernel<T><<<grids[0], FwdTile<1, T>::Threads, FwdTile<1, T>::Smem, st>>>(items, bases, n, sub, queues);
+        fwd_batched_kernel<T><<<b.fwd_grid, FwdTile<1, T>::Threads, FwdTile<1, T>::Smem, st>>>(
+            b.items + b.first(2), b.fwd_base[2], b.packs[2], sub, queue);
         XCT_CUDA_TRY(cudaGetLastError());
         return XCT_OK;
     });
-    if (rc) return rc;
-    if (grids[1] > 0) {
-        fwd_finalize_batched_kernel<<<grids[1], 256, 0, st>>>(items, bases + (n + 1), n, sub);
-        XCT_CUDA_TRY(cudaGetLastError());
-    }
-    bp_batched_kernel<<<grids[2], BpCfg<4>::Threads, 0, st>>>(items, bases + 2 * (n + 1), n, sub, queues + 2);
-    XCT_CUDA_TRY(cudaGetLastError());
-    return XCT_OK;  // launches are counted when the captured graph is replayed
 }
 
-// The forward launch of one batched subset step alone (the autotuner times it).
-int launch_fwd_batched(const XctItemDev *items, const int *bases, int n, int sub, int *queue, int grid, int fwd_T,
-                       cudaStream_t st)
+// One subset step.  The launches of the pack sizes in use run side by side (sizes beyond the first on
+// side streams, so that one's last CTAs and the next one's first share the SMs).
+int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queues /*[2]*/, cudaStream_t st, const XctBatchSide &side)
 {
-    return with_tile(fwd_T, [&](auto tc) -> int {
-        constexpr int T = decltype(tc)::value;
-        fwd_batched_kernel<T><<<grid, FwdTile<1, T>::Threads, FwdTile<1, T>::Smem, st>>>(items, bases, n, sub, queue);
-        XCT_CUDA_TRY(cudaGetLastError());
+    auto parallel = [&](auto &&launch) -> int {
+        int used = 0, rc = XCT_OK;
+        for (int q = 0; q < 3; ++q)
+            if (b.packs[q] > 0) ++used;
+        if (used > 1) XCT_CUDA_TRY(cudaEventRecord(side.fork, st));
+        int k = 0;
+        for (int q = 0; q < 3; ++q) {
+            if (b.packs[q] <= 0) continue;
+            const cudaStream_t on = k == 0 ? st : side.stream[k - 1];
+            if (k > 0) XCT_CUDA_TRY(cudaStreamWaitEvent(on, side.fork, 0));
+            if ((rc = launch(q, on))) return rc;
+            if (k > 0) XCT_CUDA_TRY(cudaEventRecord(side.join[k - 1], on));
+            ++k;
+        }
+        for (int j = 0; j + 1 < used; ++j) XCT_CUDA_TRY(cudaStreamWaitEvent(st, side.join[j], 0));
         return XCT_OK;
+    };
+    int rc = parallel([&](int q, cudaStream_t on) -> int {
+        return q == 0 ? launch_fwd_pack<4>(b, q, sub, on)
+               : q == 1 ? launch_fwd_pack<2>(b, q, sub, on)
+                        : launch_fwd_batched(b, sub, queues, on);
+    });
+    if (rc) return rc;
+    if (b.fin_units > 0) {
+        fwd_finalize_batched_kernel<<<b.fin_units, 256, 0, st>>>(b.items, b.fin_base, b.m, sub);
+        XCT_CUDA_TRY(cudaGetLastError());
+    }
+    return parallel([&](int q, cudaStream_t on) -> int {
+        const XctItemDev *it = b.items + b.first(q);
+        if (q == 0)
+            bp_pack_kernel<4><<<b.bp_units[q], kBpMsThreads, 0, on>>>(it, b.bp_base[q], b.packs[q], sub);
+        else if (q == 1)
+            bp_pack_kernel<2><<<b.bp_units[q], kBpMsThreads, 0, on>>>(it, b.bp_base[q], b.packs[q], sub);
+        else
+            bp_batched_kernel<<<b.bp_grid, BpCfg<4>::Threads, 0, on>>>(it, b.bp_base[q], b.packs[q], sub, queues + 1);
+        XCT_CUDA_TRY(cudaGetLastError());
+        return XCT_OK;  // launches are counted when the captured graph is replayed
     });
 }
 
@@ -966,13 +1066,22 @@ static int launch_fwd_group(const KGeom &g, const float2 *trig, const float *img
 // S = 2, T = 83; 2010 for S = 4, T = 58).
 double xct_fwd_cost(int nx, int ny, int S, int T, int nrows, int chunk, int groups, int sms)
 {
+    double tail = 0.0;
+    const double work = xct_fwd_work(nx, ny, S, T, nrows, chunk, groups, tail);
+    return work / sms + tail;
+}
+
+// The two parts of it: the work of all tiles, and half a CTA's own time (tail).
+double xct_fwd_work(int nx, int ny, int S, int T, int nrows, int chunk, int groups, double &tail)
+{
     const double t2 = (double)T * T;
     const double angle = t2 * (0.15 + 0.085 * S) + 7.0 * T, stage = 0.2 * S * t2 + 400.0;
     const int blocks = S > 1 ? 2 : T <= 76 ? 4 : 3;
     const double area = (nx + 1.0) * (ny + 1.0) / t2 * groups;
     const double tiles = (double)((nx + T) / T) * ((ny + T) / T) * groups;
     const int n = (nrows + chunk - 1) / chunk;
-    return (tiles * n * stage + area * nrows * angle) / sms + 0.5 * blocks * (stage + chunk * angle);
+    tail = 0.5 * blocks * (stage + chunk * angle);
+    return tiles * n * stage + area * nrows * angle;
 }
 
 // Subset angles per CTA of the grouped forms: the even split with the least modelled time.

@@ -137,14 +137,16 @@ int xct_osem_run_volume(xct_plan *plan, int n, const float *const *sino_host, fl
  * per xct_osem_run_device call (the slice-interleaved kernels serve such slices faster than
  * the persistent launches): in place when a call's slices are consecutive in one pair of
  * arrays ([k][pa][px], [k][ny][nx]), else copied into a contiguous scratch pair of the plan
- * and the images copied back.  The graph serves the other slices; with compressed sensing
- * (stacks set) it serves every slice.  Results agree with the graph's to float rounding.
+ * and the images copied back.  The graph serves the other slices, two to seven of one geometry
+ * in packs of four and of two (where the modelled time of the whole graph is lower so) and the
+ * rest one by one; with compressed sensing (stacks set) it serves every slice.  Results agree
+ * to float rounding whichever way a slice goes.
  * Each group holds a single-shape plan with the buffers of up to 16 slices of its geometry
  * (staging, ratio and accumulator: about 0.6 GB for 2048^2 with 1200 angles), so a stack of
  * many groups holds as many such sets; the graph's buffers cover every slice once.
  * xct_batch_plan_groups reports the number of groups and the slices they hold;
- * xct_batch_plan_set_grouping(plan, 0) turns the groups off (the graph serves every slice),
- * 1 on again (the default).  xct_batch_plan_uniform reports the slices per call when every
+ * xct_batch_plan_set_grouping(plan, 0) turns the groups and the packs off (the graph serves
+ * every slice by itself), 1 on again (the default).  xct_batch_plan_uniform reports the slices per call when every
  * slice is in one group (0: not so). */
 typedef struct xct_batch_plan xct_batch_plan;
 int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms, int it, xct_batch_plan **out);
