@@ -349,10 +349,11 @@ static int xct_osem_split(const xct_plan *p, int dN)
 // The same for a call whose slices are already on the device.  Two streams let one half's
 // backprojection fill what the other half's forward projection leaves (12 slices of 736^2: 2.07 against
 // 2.19 ms), but halves of a single slice would lose the grouped forward kernel (two slices of 840^2:
-// 6.46 against 4.52 ms), so fewer than four slices stay on one stream.
+// 6.46 against 4.52 ms), so fewer than four slices stay on one stream; so do small problems.
 static int xct_stream_split(const xct_plan *p, int dN)
 {
-    return p->g.kernels == XCT_KERNELS_TILED && p->kg.fwd_group && dN < 4 ? dN : xct_osem_split(p, dN);
+    const bool one = dN < 4 || fwd_is_small(p->kg, dN, (p->g.pa + p->g.ss - 1) / p->g.ss);
+    return p->g.kernels == XCT_KERNELS_TILED && p->kg.fwd_group && one ? dN : xct_osem_split(p, dN);
 }
 
 // One subset step (OSEM1 then OSEM2) of dN slices with the given plan buffers (ratio

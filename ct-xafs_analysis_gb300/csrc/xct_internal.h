@@ -25,6 +25,7 @@ struct KGeom {
     int ms_chunk = 0;  // slice-interleaved kernels: most subset angles per forward CTA (1..128);
                        // 0 = off (the backprojectors and the adjoint then work slice by slice)
     int fwd_group = 1;   // forward projection of several slices per CTA (0: one, by hand)
+    int fwd_tuned = 0;   // fwd_T and fwd_chunk were measured or set by hand: single slices keep them
     int fwd_direct = 1;  // small problems take the kernels of xct_direct.cu (0: a tile chosen by hand)
 };
 
@@ -165,6 +166,7 @@ int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const
 // accumulator) and launch_bp_update_tiled, and whether a launch of dN slices takes them.
 bool fwd_is_direct(const KGeom &g, int dN, int nrows);
 bool bp_is_direct(const KGeom &g, int dN);
+bool fwd_is_small(const KGeom &g, int dN, int nrows);  // (xct_tiled.cu)
 int launch_fwd_direct(const KGeom &g, const float2 *trig, const float *img, const float *meas, float *out, int dN, int sub,
                       int step, int nrows, cudaStream_t st);
 int launch_bp_update_direct(const KGeom &g, const float2 *trig, float *img, const float *ratio, int dN, int sub,
@@ -199,6 +201,7 @@ struct TuneChoice {
     int T, chunk;
     float ms;
     int ms_chunk = 0;  // slice-interleaved forward projector's angle chunk; 0 = off
+    int runs = 0;      // a slice by itself is faster in runs of (tile, angle) units than with T and chunk
 };
 std::string xct_tune_key(const char *device, int nx, int ny, int px, int pa, int ss, int dN);
 bool xct_tune_lookup(const std::string &key, const char *path, TuneChoice &c);

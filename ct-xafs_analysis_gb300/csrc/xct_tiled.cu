@@ -3,10 +3,11 @@
 // Forward projector (OSEM1 / projection, OSEM.cl:38-68, reconstShare.cl:213-241),
 // tile-stationary:
 //   * one CTA owns an image tile of up to five slices: the samples whose base texel (floor(x),
-//     floor(y)) lies in [x0, x0+T) x [y0, y0+T), with x0 = -1 + bx*T (base texel -1 still reaches
-//     texel 0).  It stages the tile ONCE per subset in shared memory as (t, t[x+1] - t) pairs, so
+//     floor(y)) lies in [x0, x0+tx) x [y0, y0+ty), tx, ty <= T, the first at -1 (base texel -1 still
+//     reaches texel 0).  It stages the tile once in shared memory as (t, t[x+1] - t) pairs, so
 //     the x-lerp of a bilinear sample is one FMA and its 2x2 footprint is two 64-bit
-//     loads, and serves every angle of its angle chunk from there;
+//     loads, and serves its angles from there; a run of (tile, angle) units of equal modelled time per
+//     CTA, so that the grid is one wave whatever the image's size and the angle count;
 //   * a warp takes one angle and 8 consecutive rays, 4 lanes per ray; the exact interval of
 //     sample indices Y whose base texel lies in the tile (the coordinates are monotone in Y)
 //     comes from four boundary searches, one per lane of the ray's group; the 4 lanes then
@@ -25,6 +26,7 @@
 //     reference's bin expression ((Xc*c - Yc*s) + cx) + 0.5 with packed f32x2 instructions (each
 //     lane rounds exactly like the scalar expression) and the nearest rule as a round-down add;
 //   * the multiplicative update is fused.
+#include <math.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -87,8 +89,12 @@ __device__ __forceinline__ float lds_f1(unsigned addr)
 // rows one load touches, and neighbouring samples then mostly share their elements: 0.127 with a
 // pitch of 3 or 5 (mod 8).  The weight of the odd row is the distance |y - (even row)|.
 //
-// S up to 5 and T: two CTAs of 512 threads per SM fill shared memory (one stages while the other
-// computes); with S = 1 the tile side is the plan's choice (44, 60, 76 or 92).
+// T: the side that fills shared memory with one CTA of 1024 threads per SM (163 for one slice, 83 for
+// four), or with two of 512 (one stages while the other computes).  A larger tile has longer rays, so less
+// of the time goes to finding a ray's interval and to its last, partly used step: per sample and slice
+// 0.21 SM cycles against 0.26 for one slice (T = 163, 92), 0.147 against 0.167 for two (115, 83), 0.141
+// against 0.148 for four (83, 58).  The sides 44, 60, 76 and 92 of one slice are a plan's choice by hand or by
+// the tuner, and the batch plans'.
 template <int S, int T>
 struct FwdTile {
     // element pitch: the smallest of 3 or 5 (mod 8) that holds a row
@@ -98,16 +104,19 @@ struct FwdTile {
     // per chunk angle: (c, s, 1/c, 1/s) and (first ray, last ray, first item, end item)
     static constexpr size_t TableOff = ((size_t)S * Plane + 15) & ~(size_t)15;
     static constexpr size_t Smem = TableOff + (size_t)kAngChunk * 32;
-    // S = 1: 12 warps per CTA, 4 CTAs per SM where four tiles fit (T <= 76), else 3
-    static constexpr int Threads = S == 1 ? 384 : 512;
-    static constexpr int MinBlocks = S > 1 ? 2 : (Smem + 1024) * 4 <= 228u * 1024u ? 4 : 3;
+    // large tiles: one CTA of 32 warps per SM; of S = 1, 12 warps per CTA, 4 CTAs per SM where four tiles
+    // fit (T <= 76), else 3
+    static constexpr bool Large = (Smem + 1024) * 2 > 228u * 1024u;
+    static constexpr int Threads = Large ? 1024 : S == 1 && T <= 92 ? 384 : 512;
+    static constexpr int MinBlocks = Large ? 1 : S > 1 || T > 92 ? 2 : (Smem + 1024) * 4 <= 228u * 1024u ? 4 : 3;
     static_assert((P % 8 == 3 || P % 8 == 5) && P >= T, "tile pitch");
     static_assert((Smem + 1024) * MinBlocks <= 228u * 1024u, "tiles exceed shared memory");
 };
-// tile side of the grouped forms (S = 2 .. 5): the largest that two CTAs per SM hold
+// Tile sides of the forms with S slices: the largest that one CTA per SM holds, and that two hold.
 template <int S>
 struct FwdGroup {
-    static constexpr int T = S == 2 ? 83 : S == 3 ? 67 : S == 4 ? 58 : 51;
+    static constexpr int Large = S == 1 ? 163 : S == 2 ? 115 : S == 3 ? 93 : S == 4 ? 83 : 75;
+    static constexpr int T = S == 1 ? 115 : S == 2 ? 83 : S == 3 ? 67 : S == 4 ? 58 : 51;
 };
 
 template <int kOff>
@@ -189,13 +198,13 @@ __device__ __forceinline__ float fwd_reduce(const float (&sum)[S], int ph, float
     return v;
 }
 
-// The work of one CTA: tile (bx, by) of S slices (slice z: image image(z), accumulator accum(z)
-// [nrows][px]) for the subset angles k0 .. k0+chunk-1 (chunk <= kAngChunk).  Starts and ends with all
-// threads in step.
+// The tile of S slices (slice z: image image(z), accumulator accum(z) [nrows][px]) whose base texels are
+// [x0, x0+tx) x [y0, y0+ty) (tx, ty <= T), for the subset angles k0 .. k0+chunk-1 (chunk <= kAngChunk).
+// Starts and ends with all threads in step.
 template <int S, int T, class Image, class Accum>
 __device__ __forceinline__ void fwd_tile(const KGeom &g, Image image, Accum accum, const float2 *__restrict__ trig,
-                                         int sub, int step, int nrows, int bx, int by, int k0, int chunk,
-                                         unsigned char *smem_raw)
+                                         int sub, int step, int nrows, int x0, int y0, int tx, int ty, int k0,
+                                         int chunk, unsigned char *smem_raw)
 {
     typedef FwdTile<S, T> C;
     constexpr int kThr = C::Threads;
@@ -203,16 +212,17 @@ __device__ __forceinline__ void fwd_tile(const KGeom &g, Image image, Accum accu
     int4 *s_ray = reinterpret_cast<int4 *>(s_cs + kAngChunk);
     const int kn = min(chunk, nrows - k0);
     if (kn <= 0) return;
-    const int x0 = -1 + bx * T, y0 = -1 + by * T;
 
     // element (c, r) = (t(x0+c, y0+r), t(x0+c+1, y0+r) - t(x0+c, y0+r)), zero border.  A warp stages
     // rows of a slice: each texel is loaded once, its right neighbour comes from the next lane.
     const int lane = threadIdx.x & 31;
     {
         constexpr int kCols = T / 32 + 1;  // lanes cover columns 0 .. T
-#pragma unroll 2
-        for (int q = threadIdx.x >> 5; q < S * C::Rows; q += kThr / 32) {
-            const int z = q / C::Rows, r = q - z * C::Rows;
+        const int rows = ty + 1;
+        constexpr int kUnroll = kThr == 384 ? 2 : C::Large ? 8 : 4;  // rows in flight (small tiles of one slice: 40 registers)
+#pragma unroll kUnroll
+        for (int q = threadIdx.x >> 5; q < S * rows; q += kThr / 32) {
+            const int z = S == 1 ? 0 : q / rows, r = q - z * rows;
             const int gy = y0 + r;
             const bool rv = (unsigned)gy < (unsigned)g.ny;
             const float *row = image(z) + ((long long)gy * g.nx + x0);
@@ -233,8 +243,8 @@ __device__ __forceinline__ void fwd_tile(const KGeom &g, Image image, Accum accu
         }
     }
     // owned base-texel ranges (the union over tiles is [-1, n-1])
-    const float xlo = (float)x0, xhi = (float)min(x0 + T, g.nx);
-    const float ylo = (float)y0, yhi = (float)min(y0 + T, g.ny);
+    const float xlo = (float)x0, xhi = (float)min(x0 + tx, g.nx);
+    const float ylo = (float)y0, yhi = (float)min(y0 + ty, g.ny);
     for (int k = threadIdx.x; k < kn; k += kThr) {
         const float2 cs = trig[sub + (k0 + k) * step];
         s_cs[k] = make_float4(cs.x, cs.y, 1.0f / cs.x, 1.0f / cs.y);
@@ -372,22 +382,57 @@ __device__ __forceinline__ void fwd_tile(const KGeom &g, Image image, Accum accu
     }
 }
 
-// grid: (ntx*nty tiles, angle chunks, groups of S slices).  acc: [groups * S][nrows][px] doubles.
+// How a forward launch divides groups * ntx * nty tiles (sides tx, ty) x nrows angles among its CTAs.
+// chunk > 0: a CTA per tile and chunk of angles, chunks of all tiles one after the other.  chunk = 0: CTA i
+// takes the run of (tile, angle) units start[i] .. start[i+1]-1 (tile by tile), whatever tile boundaries it
+// crosses.
+constexpr int kMaxRuns = 320;
+struct FwdSplit {
+    int ntx, nty, tx, ty, chunk, ctas;
+    int cap;  // most angles a CTA serves from one staging
+    unsigned start[kMaxRuns + 1];
+};
+
+// acc: [groups * S][nrows][px] doubles.
 template <int S, int T>
 __global__ void __launch_bounds__(FwdTile<S, T>::Threads, FwdTile<S, T>::MinBlocks)
     fwd_tiled_kernel(const float *img, double *acc, const float2 *__restrict__ trig, KGeom g, int sub, int step, int nrows,
-                     int ntx, int chunk)
+                     const __grid_constant__ FwdSplit f, long long units)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     xct_grid_wait();
     xct_grid_trigger();
-    const size_t z0 = (size_t)blockIdx.z * S, nimg = (size_t)g.nx * g.ny, nacc = (size_t)nrows * g.px;
-    const float *im = img + z0 * nimg;
-    double *ac = acc + z0 * nacc;
-    fwd_tile<S, T>(
-        g, [&](int z) { return S == 1 ? im : im + (size_t)z * nimg; },
-        [&](int z) { return S == 1 ? ac : ac + (size_t)z * nacc; }, trig, sub, step, nrows,
-        (int)blockIdx.x % ntx, (int)blockIdx.x / ntx, (int)blockIdx.y * chunk, chunk, smem_raw);
+    // the run, in shared memory: it is live across the tile's loops, where registers are short
+    __shared__ long long s_at, s_end;
+    auto angles = [&](long long u, int k0) { return (int)min((long long)min(nrows - k0, f.cap), s_end - u); };
+    if (threadIdx.x == 0) {
+        if (f.chunk > 0) {
+            const int tiles = (int)(units / nrows), ch = (int)blockIdx.x / tiles, t = (int)blockIdx.x - ch * tiles;
+            s_at = (long long)t * nrows + ch * f.chunk;
+            s_end = s_at + min(f.chunk, nrows - ch * f.chunk);
+        } else {
+            s_at = f.start[blockIdx.x];
+            s_end = f.start[blockIdx.x + 1];
+        }
+    }
+    __syncthreads();
+    while (s_at < s_end) {
+        {
+            const long long u = s_at;
+            const int t = (int)(u / nrows), k0 = (int)(u - (long long)t * nrows);
+            const int z = t / (f.ntx * f.nty), b = t - z * (f.ntx * f.nty), by = b / f.ntx, bx = b - by * f.ntx;
+            const size_t nimg = (size_t)g.nx * g.ny, nacc = (size_t)nrows * g.px;
+            const float *im = img + (size_t)z * S * nimg;
+            double *ac = acc + (size_t)z * S * nacc;
+            fwd_tile<S, T>(
+                g, [&](int q) { return S == 1 ? im : im + (size_t)q * nimg; },
+                [&](int q) { return S == 1 ? ac : ac + (size_t)q * nacc; }, trig, sub, step, nrows, -1 + bx * f.tx,
+                -1 + by * f.ty, f.tx, f.ty, k0, angles(u, k0), smem_raw);
+        }
+        __syncthreads();  // the next tile is staged over this one
+        if (threadIdx.x == 0) s_at += angles(s_at, (int)(s_at % nrows));
+        __syncthreads();
+    }
 }
 
 // acc -> OSEM1 ratio (meas != nullptr) or raw projection, rows th = sub + k*step; clears acc.
@@ -820,8 +865,8 @@ __global__ void __launch_bounds__(FwdTile<1, T>::Threads, FwdTile<1, T>::MinBloc
         const int tiles = it.fwd_ntx * it.fwd_nty;
         const int t = local % tiles, ch = local / tiles;
         fwd_tile<1, T>(
-            g, [&](int) { return it.img; }, [&](int) { return it.acc; }, it.trig, sub, g.ss, nrows, t % it.fwd_ntx,
-            t / it.fwd_ntx, ch * g.fwd_chunk, g.fwd_chunk, smem_raw);
+            g, [&](int) { return it.img; }, [&](int) { return it.acc; }, it.trig, sub, g.ss, nrows,
+            -1 + t % it.fwd_ntx * T, -1 + t / it.fwd_ntx * T, T, T, ch * g.fwd_chunk, g.fwd_chunk, smem_raw);
         __syncthreads();  // the tile in shared memory is restaged by the next unit
     }
 }
@@ -841,8 +886,8 @@ __global__ void __launch_bounds__(FwdTile<S, T>::Threads, FwdTile<S, T>::MinBloc
     const int tiles = pk->fwd_ntx * pk->fwd_nty;
     const int t = local % tiles, ch = local / tiles;
     fwd_tile<S, T>(
-        g, [&](int z) { return pk[z].img; }, [&](int z) { return pk[z].acc; }, pk->trig, sub, g.ss, nrows, t % pk->fwd_ntx,
-        t / pk->fwd_ntx, ch * g.fwd_chunk, g.fwd_chunk, smem_raw);
+        g, [&](int z) { return pk[z].img; }, [&](int z) { return pk[z].acc; }, pk->trig, sub, g.ss, nrows,
+        -1 + t % pk->fwd_ntx * T, -1 + t / pk->fwd_ntx * T, T, T, ch * g.fwd_chunk, g.fwd_chunk, smem_raw);
 }
 
 // grid: one CTA per finalize unit (a ratio row of an item's largest subset), base[n] of them.  Four bins per
@@ -1058,16 +1103,102 @@ int fwd_ms_slices() { return kMsSlices; }
 
 // One forward launch over groups * S slices.
 template <int S, int T>
-static int launch_fwd_group(const KGeom &g, const float2 *trig, const float *img, double *acc, int groups, int sub, int step,
-                            int nrows, int chunk, cudaStream_t st)
+static int launch_fwd_group(const KGeom &g, const float2 *trig, const float *img, double *acc, const FwdSplit &f, int groups,
+                            int sub, int step, int nrows, cudaStream_t st)
 {
     typedef FwdTile<S, T> C;
     static std::atomic<bool> done[64];
     const int r = smem_attr((const void *)fwd_tiled_kernel<S, T>, C::Smem, done);
     if (r) return r;
-    const int ntx = (g.nx + 1 + T - 1) / T, nty = (g.ny + 1 + T - 1) / T;  // base texels -1 .. n-1
-    return xct_launch(fwd_tiled_kernel<S, T>, dim3(ntx * nty, (nrows + chunk - 1) / chunk, groups), C::Threads, C::Smem, st,
-                      img, acc, trig, g, sub, step, nrows, ntx, chunk);
+    return xct_launch(fwd_tiled_kernel<S, T>, dim3(f.ctas), C::Threads, C::Smem, st, img, acc, trig, g, sub, step, nrows, f,
+                      (long long)f.ntx * f.nty * groups * nrows);
+}
+
+// A CTA per tile of side T and chunk of angles.
+static void fwd_split_chunks(const KGeom &g, int T, int nrows, int chunk, int groups, FwdSplit &f)
+{
+    f.ntx = (g.nx + T) / T;  // base texels -1 .. n-1
+    f.nty = (g.ny + T) / T;
+    f.tx = f.ty = T;
+    f.chunk = chunk;
+    f.ctas = f.ntx * f.nty * groups * ((nrows + chunk - 1) / chunk);
+    f.cap = chunk;
+}
+
+// Before runs, a CTA took a tile and a chunk of angles, and the last wave of CTAs was nearly empty at many
+// sizes (three slices of 509 x 487: 64 tiles x 5 chunks on 304 places).  A subset step then and now, with the
+// large tiles: one slice of 2048^2 x 100 angles 464 / 419 us, of 512^2 x 36 28.5 / 25.5; three of 509 x 487 x 31
+// 45.7 / 39.2; ten of 512^2 x 36 107 / 93.
+//
+// Runs of equal modelled time for `blocks` CTAs per SM, on tiles as equal as T allows; returns that time (SM
+// cycles; 0: more units than start[] can count).  A full tile and angle take `angle` cycles of an SM, the
+// staging of a tile `stage`.  The work of a tile whose centre is further from the axis than half the detector
+// is scaled by the share of half a turn in which that centre is projected onto it (a 2048^2 slice on 2048
+// bins: 0.5 in the corners; with equal runs instead, corner CTAs finished early and the launch took 6 %
+// longer).  A run takes the rest of its tile where another staging would cost more than that rest.
+static double fwd_split_runs(const KGeom &g, int T, int blocks, double angle, double stage, int nrows, int groups,
+                             FwdSplit &f)
+{
+    f.ntx = (g.nx + T) / T;
+    f.nty = (g.ny + T) / T;
+    f.tx = (g.nx + f.ntx) / f.ntx;
+    f.ty = (g.ny + f.nty) / f.nty;
+    f.chunk = 0;
+    f.cap = g.ms_chunk > 0 ? g.ms_chunk : kAngChunk;
+    const int plane = f.ntx * f.nty;
+    const long long tiles = (long long)plane * groups, units = tiles * nrows;
+    if (units >= 0xffffffffLL || plane > 4096) return 0.0;
+    const double fill = (double)f.tx * f.ty / ((double)T * T);
+    const double one = angle * fill + 2.0 * T * (1.0 - fill);
+    stage = stage * fill + 0.25 * one;  // and the last round of its rays, which fill the warps unevenly
+    float weight[4096];
+    double sum = 0.0, heaviest = 0.0;
+    for (int t = 0; t < plane; ++t) {
+        const double x = (t % f.ntx + 0.5) * f.tx - 0.5 - g.hx, y = (t / f.ntx + 0.5) * f.ty - 0.5 - g.hy;
+        const double r = sqrt(x * x + y * y), h = 0.5 * g.px;
+        weight[t] = (float)(r <= h ? one : one * 0.6366197723675814 * asin(h / r));
+        sum += weight[t];
+        heaviest = std::max(heaviest, (double)weight[t]);
+    }
+    const int most = (int)std::min<long long>(std::min(device_sm_count() * blocks, kMaxRuns), units);
+    double left = sum * groups * nrows, longest = 0.0;  // angle work not assigned yet
+    long long t = 0;
+    int k = 0, i = 0;
+    for (; i < most && t < tiles; ++i) {
+        f.start[i] = (unsigned)(t * nrows + k);
+        const long long rest = most - i, todo = tiles - t;
+        const double budget = left / rest + stage * (todo > rest ? 1.0 + (double)todo / rest : 1.0);
+        double used = 0.0;
+        while (t < tiles) {
+            const double w = weight[t % plane];
+            if (used > 0.0 && i + 1 < most && budget - used < stage + w) break;
+            used += stage;
+            int n = nrows - k;
+            if (i + 1 < most) {
+                const int fit = std::max(1, (int)ceil((budget - used) / w - 0.05));
+                if (fit < n && (n - fit) * w > 0.5 * stage) n = fit;
+            }
+            used += n * w;
+            left -= n * w;
+            k += n;
+            if (k < nrows) break;
+            k = 0;
+            ++t;
+        }
+        longest = std::max(longest, used);
+    }
+    if (tiles <= most) {  // or the same number of runs for every tile, none of which crosses a boundary
+        const int m = (int)std::min<long long>(most / tiles, nrows);
+        const double own = (nrows + m - 1) / m * heaviest + stage;
+        if (own < longest) {
+            longest = own;
+            i = (int)tiles * m;
+            for (int q = 0; q < i; ++q) f.start[q] = (unsigned)(q / m * nrows + (long long)nrows * (q % m) / m);
+        }
+    }
+    f.ctas = i;
+    f.start[i] = (unsigned)units;
+    return longest * blocks;
 }
 
 // Modelled time (SM cycles) of a forward launch of `groups` groups of S slices with tile side T and
@@ -1095,54 +1226,57 @@ double xct_fwd_work(int nx, int ny, int S, int T, int nrows, int chunk, int grou
     return tiles * n * stage + area * nrows * angle;
 }
 
-// Subset angles per CTA of the grouped forms: the even split with the least modelled time.
-static int fwd_group_chunk(const KGeom &g, int S, int T, int nrows, int groups, int most)
-{
-    int best = 0;
-    double cost = 0.0;
-    for (int n = (nrows + most - 1) / most; n <= nrows; n += std::max(1, n / 8)) {
-        const int chunk = (nrows + n - 1) / n;
-        const double c = xct_fwd_cost(g.nx, g.ny, S, T, nrows, chunk, groups, device_sm_count());
-        if (best == 0 || c < cost) {
-            best = chunk;
-            cost = c;
-        }
-    }
-    return best;
-}
-
+// Groups of S slices with the form (tile side) of least modelled time.
 template <int S>
 static int launch_fwd_groups(const KGeom &g, const float2 *trig, const float *&img, double *&acc, int &dN, int groups,
                              int sub, int step, int nrows, cudaStream_t st)
 {
-    constexpr int T = FwdGroup<S>::T;
     if (groups <= 0) return XCT_OK;
-    const int chunk = fwd_group_chunk(g, S, T, nrows, groups, g.ms_chunk > 0 ? g.ms_chunk : kAngChunk);
-    const int rc = launch_fwd_group<S, T>(g, trig, img, acc, groups, sub, step, nrows, chunk, st);
+    constexpr int T1 = FwdGroup<S>::Large, T2 = FwdGroup<S>::T;
+    constexpr double angle[5][2] = {{5450, 2900}, {3900, 2300}, {3700, 2060}, {3880, 1990}, {4150, 1990}};
+    constexpr double stage[5][2] = {{8500, 3500}, {9200, 4800}, {9100, 5300}, {10700, 5600}, {10600, 5700}};
+    FwdSplit f1, f2;
+    const double t1 = fwd_split_runs(g, T1, FwdTile<S, T1>::MinBlocks, angle[S - 1][0], stage[S - 1][0], nrows, groups, f1);
+    const double t2 = fwd_split_runs(g, T2, FwdTile<S, T2>::MinBlocks, angle[S - 1][1], stage[S - 1][1], nrows, groups, f2);
+    if (t1 <= 0.0) fwd_split_chunks(g, T1, nrows, std::min(nrows, kAngChunk), groups, f1);
+    const int rc = t1 <= 0.0 || t2 <= 0.0 || t1 <= t2 ? launch_fwd_group<S, T1>(g, trig, img, acc, f1, groups, sub, step, nrows, st)
+                                                      : launch_fwd_group<S, T2>(g, trig, img, acc, f2, groups, sub, step, nrows, st);
     img += (size_t)groups * S * g.nx * g.ny;
     acc += (size_t)groups * S * nrows * g.px;
     dN -= groups * S;
     return rc;
 }
 
+// Whether the launches of dN slices are bound by latency: one launch of groups of five then serves ten slices
+// better than groups of four and two, and one stream better than two halves (ten slices of 256^2 x 18 angles,
+// 11.8 M samples: 25.1 us a subset step, 27.1 in fours and twos, 30.6 in two halves; of 512^2 x 36, 94 M: 103
+// against 96 and 97).
+bool fwd_is_small(const KGeom &g, int dN, int nrows) { return (long long)g.nx * g.ny * nrows * dN <= 30000000; }
+
 // The forward projection of dN slices into the accumulator: groups of four slices, the rest as one
-// group of five, three or two; a single slice (or every slice, with grouping off) with the plan's
-// tile.
+// group of five, three, two or one (small batches of five, ten ...: fives); with grouping off or a tuned tile
+// every slice by itself in chunks of angles.
 int launch_fwd_tiled_main(const KGeom &g, const float2 *trig, const float *img, double *acc, int dN, int sub, int step,
                           int nrows, cudaStream_t st)
 {
     if (nrows <= 0 || dN <= 0) return XCT_OK;
-    if (g.fwd_group && dN >= 2) {
-        const bool five = dN % 4 == 1;
-        int rc = launch_fwd_groups<4>(g, trig, img, acc, dN, five ? dN / 4 - 1 : dN / 4, sub, step, nrows, st);
+    if (g.fwd_group && (dN >= 2 || !g.fwd_tuned)) {
+        int rc = XCT_OK;
+        if (dN % 5 == 0 && fwd_is_small(g, dN, nrows)) return launch_fwd_groups<5>(g, trig, img, acc, dN, dN / 5, sub, step, nrows, st);
+        const bool five = dN > 1 && dN % 4 == 1;
+        rc = launch_fwd_groups<4>(g, trig, img, acc, dN, five ? dN / 4 - 1 : dN / 4, sub, step, nrows, st);
         if (!rc && five) rc = launch_fwd_groups<5>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
         if (!rc && dN == 3) rc = launch_fwd_groups<3>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
         if (!rc && dN == 2) rc = launch_fwd_groups<2>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
+        if (!rc && dN == 1) rc = launch_fwd_groups<1>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
         return rc;
     }
     if (g.fwd_chunk <= 0 || g.fwd_chunk > kAngChunk) return xct_fail(XCT_E_INVALID, "forward angle chunk out of range");
     return with_tile(g.fwd_T, [&](auto tc) -> int {
-        return launch_fwd_group<1, decltype(tc)::value>(g, trig, img, acc, dN, sub, step, nrows, g.fwd_chunk, st);
+        constexpr int T = decltype(tc)::value;
+        FwdSplit f;
+        fwd_split_chunks(g, T, nrows, g.fwd_chunk, dN, f);
+        return launch_fwd_group<1, T>(g, trig, img, acc, f, dN, sub, step, nrows, st);
     });
 }
 

@@ -31,7 +31,7 @@ const int kChunks[] = {128, 64, 32, 16};
 std::mutex g_tune_mu;
 std::map<std::string, TuneChoice> g_tune_mem;  // this process's choices
 
-// One entry per line inside "entries": "<key>": {"fwd_tile": T, "ang_chunk": C, "ms": t}
+// One entry per line inside "entries": "<key>": {"fwd_tile": T, "ang_chunk": C, "ms": t, "runs": 0|1}
 bool parse_line(const char *line, std::string &key, TuneChoice &c)
 {
     const char *q0 = strchr(line, '"');
@@ -40,10 +40,12 @@ bool parse_line(const char *line, std::string &key, TuneChoice &c)
     if (!q1) return false;
     key.assign(q0 + 1, q1 - q0 - 1);
     const char *a = strstr(q1, "\"fwd_tile\":"), *b = strstr(q1, "\"ang_chunk\":"), *m = strstr(q1, "\"ms\":");
+    const char *r = strstr(q1, "\"runs\":");  // absent in files written before it was: the chunked form
     if (!a || !b) return false;
     c.T = atoi(a + 11);
     c.chunk = atoi(b + 12);
     c.ms = m ? (float)atof(m + 5) : 0.0f;
+    c.runs = r ? atoi(r + 7) : 0;
     return xct_fwd_tile_valid(c.T) && c.chunk >= 1 && c.chunk <= fwd_tiled_rows_cap();
 }
 
@@ -70,8 +72,8 @@ int save_file(const char *path, const std::map<std::string, TuneChoice> &m)
     fprintf(f, "{\n  \"xct_tune_cache\": 1,\n  \"entries\": {\n");
     size_t i = 0;
     for (const auto &kv : m) {
-        fprintf(f, "    \"%s\": {\"fwd_tile\": %d, \"ang_chunk\": %d, \"ms\": %.5g}%s\n", kv.first.c_str(),
-                kv.second.T, kv.second.chunk, (double)kv.second.ms, ++i < m.size() ? "," : "");
+        fprintf(f, "    \"%s\": {\"fwd_tile\": %d, \"ang_chunk\": %d, \"ms\": %.5g, \"runs\": %d}%s\n", kv.first.c_str(),
+                kv.second.T, kv.second.chunk, (double)kv.second.ms, kv.second.runs, ++i < m.size() ? "," : "");
     }
     fprintf(f, "  }\n}\n");
     const bool ok = fclose(f) == 0;
@@ -195,7 +197,9 @@ void xct_plan_default_tuning(xct_plan *p)
 {
     TuneChoice c;
     const std::string key = xct_tune_key(p->ctx->name, p->g.nx, p->g.ny, p->g.px, p->g.pa, p->g.ss, p->g.max_batch);
-    if (!xct_tune_lookup(key, xct_tune_env_path(), c)) c = plan_default_tiles(p);
+    const bool cached = xct_tune_lookup(key, xct_tune_env_path(), c);
+    if (!cached) c = plan_default_tiles(p);
+    p->kg.fwd_tuned = cached && !c.runs;
     // the cache holds the per-slice kernel's tiles; the slice-interleaved kernels' switch
     // follows the plan's shape
     c.ms_chunk = plan_default_ms_chunk(p);
@@ -222,6 +226,7 @@ int xct_plan_set_tuning(xct_plan *p, int fwd_tile, int ang_chunk)
         return xct_fail(XCT_E_INVALID, "ang_chunk must be in 1..128");
     p->kg.fwd_T = fwd_tile;
     p->kg.fwd_chunk = ang_chunk;
+    p->kg.fwd_tuned = 1;
     p->kg.fwd_direct = 0;  // tiles chosen by hand are used whatever the size and the batch
     p->kg.fwd_group = 0;
     return XCT_OK;
@@ -259,6 +264,7 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
     if (!(flags & XCT_TUNE_FORCE) && xct_tune_lookup(key, cache_path, best)) {
         p->kg.fwd_T = best.T;
         p->kg.fwd_chunk = best.chunk;
+        p->kg.fwd_tuned = !best.runs;
         return XCT_OK;
     }
     XCT_CUDA_TRY(cudaSetDevice(p->ctx->device));
@@ -273,16 +279,12 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
     best = TuneChoice{0, 0, 3.0e38f};
     int rc = XCT_OK;
     // the cost depends on the geometry only; the plan's staging image is the input
-    for (const TuneChoice &c : xct_tune_candidates(rows)) {
-        p->kg.fwd_T = c.T;
-        p->kg.fwd_chunk = c.chunk;
+    auto timed = [&](const KGeom &k, int slices) {
         float tmin = 3.0e38f;
         for (int r = 0; r < 3 && rc == XCT_OK; ++r) {  // first run warms up
             cudaMemsetAsync(p->d_acc, 0, acc_bytes, st);
             cudaEventRecord(e0, st);
-            KGeom k = p->kg;
-            k.fwd_group = 0;  // the choice is the per-slice kernel's
-            rc = launch_fwd_tiled_main(k, p->d_trig, p->d_img, p->d_acc, dN, 0, p->g.ss, nrows, st);
+            rc = launch_fwd_tiled_main(k, p->d_trig, p->d_img, p->d_acc, slices, 0, p->g.ss, nrows, st);
             cudaEventRecord(e1, st);
             cudaError_t e = cudaEventSynchronize(e1);
             if (rc == XCT_OK && e != cudaSuccess) rc = xct_cuda_fail(e, "xct_plan_autotune");
@@ -290,19 +292,33 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
             cudaEventElapsedTime(&ms, e0, e1);
             if (r > 0) tmin = std::min(tmin, ms);
         }
+        return tmin;
+    };
+    KGeom k = saved;
+    k.fwd_group = 0;  // the choice is the per-slice kernel's
+    for (const TuneChoice &c : xct_tune_candidates(rows)) {
+        k.fwd_T = c.T;
+        k.fwd_chunk = c.chunk;
+        const float tmin = timed(k, dN);
         if (rc) break;
         if (tmin < best.ms) best = TuneChoice{c.T, c.chunk, tmin};
+    }
+    if (rc == XCT_OK) {  // or, for a slice by itself, runs of (tile, angle) units
+        k.fwd_T = best.T;
+        k.fwd_chunk = best.chunk;
+        const float chunks = timed(k, 1);
+        k.fwd_group = 1;
+        k.fwd_tuned = 0;
+        best.runs = timed(k, 1) <= chunks;
     }
     cudaMemsetAsync(p->d_acc, 0, acc_bytes, st);
     cudaStreamSynchronize(st);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (rc) {
-        p->kg = saved;
-        return rc;
-    }
+    if (rc) return rc;
     p->kg.fwd_T = best.T;
     p->kg.fwd_chunk = best.chunk;
+    p->kg.fwd_tuned = !best.runs;
     return xct_tune_store(key, cache_path, best);
 }
 

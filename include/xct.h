@@ -401,8 +401,9 @@ int xct_osem_profile(xct_plan *plan, int dN, const float *d_sino, float *d_img, 
  * projector has two launch-shape parameters: the tile side (44, 60, 76 or 92 texels) and the
  * subset angles one CTA serves (1..128).  A plan starts with the choice cached for its shape
  * (device name, nx, ny, px, pa, ss, max_batch) -- in this process, or in the JSON file named by
- * the environment variable XCT_TUNE_CACHE -- or else the largest tiles that still give two
- * waves of CTAs.  xct_plan_autotune times every candidate for dN slices on the plan's own
+ * the environment variable XCT_TUNE_CACHE -- or else the tiles of least modelled time; a slice by
+ * itself then goes through larger tiles in equal runs of (tile, angle) units, which the autotuner
+ * times against its choice.  xct_plan_autotune times every candidate for dN slices on the plan's own
  * geometry (its staging buffers are the input; no caller data is read or written), keeps the
  * fastest, and records it in memory and in cache_path (NULL: XCT_TUNE_CACHE; no file if
  * neither).  A cached entry is reused without timing unless flags has XCT_TUNE_FORCE.
@@ -420,12 +421,10 @@ int xct_batch_plan_tuning(xct_batch_plan *plan, int *fwd_tile, int *ang_chunk);
 /* ---- slice-interleaved kernels ---------------------------------------------------------
  * No counterpart in the reference (its OSEM1/OSEM2 work-items each serve one slice).  The
  * slices of one call share their geometry, so a plan can serve them in groups:
- *  - forward projection (OSEM1, xct_fwd) in groups of XCT_MULTISLICE_SLICES (eight): a CTA
- *    stages one tile of the eight slices (one 128-byte line of bilinear coefficients per
- *    texel), a quarter-warp walks two rays, and each lane reads the eight slices of its sample
- *    in a rotated order (no shared-memory bank conflict; a sample's coordinates are found once
- *    for all eight).  Results agree with the per-slice kernel to float rounding of the partial
- *    ray sums;
+ *  - forward projection (OSEM1, xct_fwd) in groups of four slices and one of five, three or two:
+ *    a CTA stages a tile of all slices of a group, and a sample's coordinates, addresses and
+ *    weights are found once for all of them.  Results agree with the per-slice kernel to float
+ *    rounding of the partial ray sums;
  *  - backprojection + update (OSEM2) in groups of eight, and a pair left over in a two-slice
  *    form: one bin expression per eight (two) gathers; bit-identical to the per-slice kernel;
  *    the FBP backprojection (xct_fbp_backproject, the FBP and hybrid runs) the same way, also
@@ -439,8 +438,8 @@ int xct_batch_plan_tuning(xct_batch_plan *plan, int *fwd_tile, int *ang_chunk);
  *    form exactly where its fixed-point path applies).
  * With it on, a call's slices go in groups through these kernels and the rest through the
  * per-slice ones, and a call that runs as two halves cuts them at a multiple of eight.  The
- * value is the number of subset angles one forward CTA serves (1..128); 0 turns all three
- * off.  Plans start on (128) when max_batch >= 8 and the forward tiles of one group give at
+ * value is the most subset angles a forward CTA serves from one staging of a tile (1..128); 0
+ * turns all three off.  Plans start on (128) when max_batch >= 8 and the forward tiles of one group give at
  * least two CTAs per SM, else off (the tile cache and the autotuner leave this switch
  * alone). */
 #define XCT_MULTISLICE_SLICES 8
