@@ -114,9 +114,10 @@ struct Arrangement {
     int chunk[2] = {0, 0};
 };
 
-// Modelled forward work and tail of packs of S slices (first members in `firsts`) with tile side T, and
-// the angle chunk of least time.
-static int pack_chunk(const xct_batch_plan *p, int S, int T, const std::vector<int> &firsts, double &work, double &tail)
+// Modelled forward work and tail of packs of S slices (first members in `firsts`) by `model`(geometry, angles,
+// chunk, tail), and the angle chunk of least time.
+template <class Model>
+static int pack_chunk(const xct_batch_plan *p, const std::vector<int> &firsts, Model &&model, double &work, double &tail)
 {
     int best = 0;
     const double sms = p->ctx->sm_count;
@@ -125,7 +126,7 @@ static int pack_chunk(const xct_batch_plan *p, int S, int T, const std::vector<i
         for (int i : firsts) {
             const KGeom &g = p->host[i].g;
             double ti;
-            w += xct_fwd_work(g.nx, g.ny, S, T, (g.pa + g.ss - 1) / g.ss, c, 1, ti);
+            w += model(g, (g.pa + g.ss - 1) / g.ss, c, ti);
             t = std::max(t, ti);
         }
         if (best == 0 || w / sms + t < work / sms + tail) {
@@ -139,7 +140,8 @@ static int pack_chunk(const xct_batch_plan *p, int S, int T, const std::vector<i
 
 // Slices of one geometry are packed (with `grouping` on) in fours and twos, twos or not at all,
 // whichever has the least modelled forward time: a pack does less work per slice, but a few small
-// slices fill the SMs better one by one.
+// slices fill the SMs better one by one.  (Compared at the sides that two CTAs per SM hold, 58 and 83, as the
+// single slices' tiles are.)
 static Arrangement arrange(const xct_batch_plan *p, const std::vector<int> &want)
 {
     std::vector<char> in(p->n, 0);
@@ -163,6 +165,11 @@ static Arrangement arrange(const xct_batch_plan *p, const std::vector<int> &want
         }
         std::sort(a.list[2].begin(), a.list[2].end());
         double work = 0.0, tail = 0.0;
+        auto by_side = [](int S, int T) {
+            return [S, T](const KGeom &g, int rows, int chunk, double &t) {
+                return xct_fwd_work(g.nx, g.ny, S, T, rows, chunk, 1, t);
+            };
+        };
         auto add = [&](double w, double t) {
             work += w;
             tail = std::max(tail, t);
@@ -171,14 +178,18 @@ static Arrangement arrange(const xct_batch_plan *p, const std::vector<int> &want
             if (!firsts[q].empty()) {
                 const int S = q == 0 ? 4 : 2;
                 double w = 0.0, t = 0.0;
-                a.chunk[q] = pack_chunk(p, S, xct_pack_tile(S), firsts[q], w, t);
+                pack_chunk(p, firsts[q], by_side(S, S == 4 ? 58 : 83), w, t);
                 add(w, t);
+                auto pack = [S](const KGeom &g, int rows, int chunk, double &tail_) {
+                    return xct_pack_work(g.nx, g.ny, S, rows, chunk, tail_);
+                };
+                a.chunk[q] = pack_chunk(p, firsts[q], pack, w, t);
             }
         if (!a.list[2].empty()) {
             double w = 0.0, t = 0.0;
             for (int T : {92, 76, 60, 44}) {
                 double wi = 0.0, ti = 0.0;
-                pack_chunk(p, 1, T, a.list[2], wi, ti);
+                pack_chunk(p, a.list[2], by_side(1, T), wi, ti);
                 if (T == 92 || wi / sms + ti < w / sms + t) w = wi, t = ti;
             }
             add(w, t);

@@ -177,6 +177,7 @@ int launch_bp_update_direct(const KGeom &g, const float2 *trig, float *img, cons
 void xct_batched_units(const KGeom &g, int S, int &fwd_ntx, int &fwd_nty, int &fwd_units, int &fin_units, int &bp_ntx,
                        int &bp_units);
 int xct_pack_tile(int S);
+double xct_pack_work(int nx, int ny, int S, int nrows, int chunk, double &tail);
 int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid);
 int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queues, cudaStream_t st, const XctBatchSide &side);
 bool xct_fwd_tile_valid(int T);

@@ -816,9 +816,10 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
 // out.  Units of pack (slice) i are [base[i], base[i+1]); they are independent within a launch, so
 // there is no waiting on other CTAs.
 // A pack pays per slice what the forward and backward kernels of several slices save (coordinates,
-// addresses and weights once): one iteration of 24 slices, 12 geometries 512 to 2048 wide, takes 30.3 ms
-// in packs of two and 43.3 one by one; 21 of seven geometries 570 to 1140 wide, in packs of two and
-// single slices, 6.7 against about 7.3.
+// addresses and weights once), and takes the large tiles, one CTA per SM: one iteration of 24 slices, 12
+// geometries 512 to 2048 wide, takes 27.8 ms in packs of two and 43.3 one by one (29.3 with tiles of two CTAs per
+// SM); 21 of seven geometries 570 to 1140 wide, in packs of two and single slices, 8.7 ms (9.3); 6 of
+// three, 200 to 400 wide, 0.33 with either.
 __device__ __forceinline__ int queue_take(int *queue, int *s_unit)
 {
     if (threadIdx.x == 0) *s_unit = atomicAdd(queue, 1);
@@ -1006,7 +1007,7 @@ void xct_batched_units(const KGeom &g, int S, int &fwd_ntx, int &fwd_nty, int &f
 }
 
 // Forward tile side of a pack of S slices.
-int xct_pack_tile(int S) { return S == 4 ? FwdGroup<4>::T : FwdGroup<2>::T; }
+int xct_pack_tile(int S) { return S == 4 ? FwdGroup<4>::Large : FwdGroup<2>::Large; }
 
 // Persistent grids of the single slices' launches; the packs' shared-memory limits.
 int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid)
@@ -1031,7 +1032,7 @@ int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid)
 template <int S>
 static int launch_fwd_pack(const XctBatchStep &b, int q, int sub, cudaStream_t st)
 {
-    constexpr int T = FwdGroup<S>::T;
+    constexpr int T = FwdGroup<S>::Large;
     static std::atomic<bool> done[64];
     const int r = smem_attr((const void *)fwd_pack_kernel<S, T>, FwdTile<S, T>::Smem, done);
     if (r) return r;
@@ -1201,6 +1202,26 @@ static double fwd_split_runs(const KGeom &g, int T, int blocks, double angle, do
     return longest * blocks;
 }
 
+// Cycles of an SM that a full tile of S = 1 .. 5 slices and an angle take, and the tile's staging: large and
+// small tiles (fits of launches on 256^2 to 2048^2 slices).
+struct FwdForm {
+    double angle[2], stage[2];
+};
+static const FwdForm kFwdForm[5] = {{{5450, 2900}, {8500, 3500}},
+                                    {{3900, 2300}, {9200, 4800}},
+                                    {{3700, 2060}, {9100, 5300}},
+                                    {{3880, 1990}, {10700, 5600}},
+                                    {{4150, 1990}, {10600, 5700}}};
+
+// Modelled forward work of one pack of S slices in chunks of angles, and half a CTA's own time (tail).
+double xct_pack_work(int nx, int ny, int S, int nrows, int chunk, double &tail)
+{
+    const double angle = kFwdForm[S - 1].angle[0], stage = kFwdForm[S - 1].stage[0];
+    const int T = xct_pack_tile(S), n = (nrows + chunk - 1) / chunk;
+    tail = 0.5 * (stage + chunk * angle);
+    return (double)((nx + T) / T) * ((ny + T) / T) * n * stage + (nx + 1.0) * (ny + 1.0) / ((double)T * T) * nrows * angle;
+}
+
 // Modelled time (SM cycles) of a forward launch of `groups` groups of S slices with tile side T and
 // nrows angles in chunks: the work of all tiles over the SMs, plus half a CTA's own time for the
 // unevenness of the last wave.  A tile and angle take T^2 (0.15 + 0.085 S) + 7 T cycles and its
@@ -1233,11 +1254,10 @@ static int launch_fwd_groups(const KGeom &g, const float2 *trig, const float *&i
 {
     if (groups <= 0) return XCT_OK;
     constexpr int T1 = FwdGroup<S>::Large, T2 = FwdGroup<S>::T;
-    constexpr double angle[5][2] = {{5450, 2900}, {3900, 2300}, {3700, 2060}, {3880, 1990}, {4150, 1990}};
-    constexpr double stage[5][2] = {{8500, 3500}, {9200, 4800}, {9100, 5300}, {10700, 5600}, {10600, 5700}};
+    const FwdForm &m = kFwdForm[S - 1];
     FwdSplit f1, f2;
-    const double t1 = fwd_split_runs(g, T1, FwdTile<S, T1>::MinBlocks, angle[S - 1][0], stage[S - 1][0], nrows, groups, f1);
-    const double t2 = fwd_split_runs(g, T2, FwdTile<S, T2>::MinBlocks, angle[S - 1][1], stage[S - 1][1], nrows, groups, f2);
+    const double t1 = fwd_split_runs(g, T1, FwdTile<S, T1>::MinBlocks, m.angle[0], m.stage[0], nrows, groups, f1);
+    const double t2 = fwd_split_runs(g, T2, FwdTile<S, T2>::MinBlocks, m.angle[1], m.stage[1], nrows, groups, f2);
     if (t1 <= 0.0) fwd_split_chunks(g, T1, nrows, std::min(nrows, kAngChunk), groups, f1);
     const int rc = t1 <= 0.0 || t2 <= 0.0 || t1 <= t2 ? launch_fwd_group<S, T1>(g, trig, img, acc, f1, groups, sub, step, nrows, st)
                                                       : launch_fwd_group<S, T2>(g, trig, img, acc, f2, groups, sub, step, nrows, st);
