@@ -1050,8 +1050,8 @@ def main():
 
     # ---- roofline of the dominant kernel (live CUDA events, same stream) ----
     # The timed batch of 10 runs as halves of 8 | 2 slices; the 8-slice half's forward
-    # projection is one launch of the slice-interleaved kernel per subset (fwd_ms_kernel),
-    # 82 % of the forward time of a step.  It is timed here on 8 slices: every launch of a
+    # projection is one launch of the grouped kernel per subset (fwd_tiled_kernel<4, 83>, two groups
+    # of four), most of the forward time of a step.  It is timed here on 8 slices: every launch of a
     # 4 x 15 profile run bracketed by CUDA events on the launch stream.
     G = xct.MULTISLICE_SLICES
     prof = plan.profile(sino[:G], imgs[:G].fill_(1.0), dN=G, stream=stream)
@@ -1066,17 +1066,17 @@ def main():
     # HBM view of the same kernel: it reads each image once per subset and adds one double
     # per (ray, tile) -- compulsory bytes are tiny next to its arithmetic
     fwd_bytes = G * NX * NY * 4.0
-    # the kernel's own bound: the L1/shared-memory data path, one 16-byte record per tap and
-    # slice (the four bilinear coefficients of the footprint) against 128 B/clk/SM
+    # the kernel's own bound: the L1/shared-memory data path, two 8-byte elements per tap and
+    # slice (the two rows of the footprint) against 128 B/clk/SM
     props = torch.cuda.get_device_properties(dev)
     sm_mhz = clk.summary().get("sm_mhz") or 2070.0
     l1_peak = 128.0 * props.multi_processor_count * sm_mhz * 1e6
     roofline = {
-        "bound": "fp32", "kernel": "fwd_ms_kernel (OSEM1 forward projection, 8 slices per launch)",
+        "bound": "fp32", "kernel": "fwd_tiled_kernel (OSEM1 forward projection, 8 slices per launch in groups of four)",
         "l1_shared": {"achieved_tbs": taps_per_launch * 16.0 / (fwd_ms_avg * 1e-3) / 1e12,
                       "peak_tbs": l1_peak / 1e12,
                       "frac": taps_per_launch * 16.0 / (fwd_ms_avg * 1e-3) / l1_peak,
-                      "note": "16 B (one float4 record) per tap and slice over 128 B/clk/SM at the sampled SM "
+                      "note": "16 B (two 8-byte elements) per tap and slice over 128 B/clk/SM at the sampled SM "
                               "clock"},
         "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
         "peak_source": "measured live by xct_fp32_peak (FMA-chain kernel) in this run",
@@ -1097,14 +1097,14 @@ def main():
         pass
     # DRAM traffic of the forward kernel per launch from the committed ncu capture of the same
     # launch shape (8 slices of 2048^2, one subset of 100 angles)
-    prof_md = os.path.join(REPO, "profiles", "fwd_ms_kernel_2048x2048_1500ang_8slices.md")
+    prof_md = os.path.join(REPO, "profiles", "forward_adjoint_2048_1024.md")
     try:
         with open(prof_md) as f:
             for line in f:
                 if line.startswith("dram_bytes_per_launch:"):
                     roofline["traffic"] = float(line.split(":")[1])
                     roofline["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch, "
-                                                  "profiles/fwd_ms_kernel_2048x2048_1500ang_8slices.md")
+                                                  "profiles/forward_adjoint_2048_1024.md")
     except Exception:
         pass
 
