@@ -42,6 +42,7 @@ struct xct_batch_plan {
     XctBatchSide side;
     int fwd_T = 92, fwd_chunk = 128;  // forward tiles of the single slices
     bool tuned = false;               // ... from the autotuner or its cache
+    int tuned_runs = 0;               // ... and the large tiles were faster
     std::vector<int> bases;           // host copy of d_bases
     size_t n_acc = 0;
     std::string key;                  // tune-cache key of the batch's shapes
@@ -203,11 +204,23 @@ static Arrangement arrange(const xct_batch_plan *p, const std::vector<int> &want
     return best;
 }
 
-// Forward tiles of the single slices when nothing was tuned (of every slice when all are packed).
+// Angle chunk of the single slices' large tiles (one CTA per SM), 0 without single slices.
+static int large_chunk(const xct_batch_plan *p, const std::vector<int> &singles)
+{
+    double work = 0.0, tail = 0.0;
+    auto model = [](const KGeom &g, int rows, int chunk, double &t) { return xct_pack_work(g.nx, g.ny, 1, rows, chunk, t); };
+    return singles.empty() ? 0 : pack_chunk(p, singles, model, work, tail);
+}
+
+// Forward tiles of the single slices when nothing was tuned (of every slice when all are packed).  The large
+// tiles serve them where every SM has at least 32 (tile, angle) units of them to do: one iteration of 12 slices
+// 512 to 2048 wide (500 units) 20.4 ms against 22.3, of five 722 to 1444 wide 3.81 against 4.45, of 21 slices of
+// which 7 single ones 570 to 1140 wide (60 units) 8.33 against 8.70; but of 30 with 10 single ones 327 to 654 wide
+// (25 units) 2.24 against 2.20, and of 8 slices 150 to 300 wide (2 units) 0.69 against 0.61.
 static TuneChoice default_tiles(const xct_batch_plan *p, const Arrangement &a, const std::vector<int> &want)
 {
     const std::vector<int> &of = a.list[2].empty() ? want : a.list[2];
-    return xct_tune_default(p->ctx->sm_count, [&](int T, int ch) {
+    TuneChoice c = xct_tune_default(p->ctx->sm_count, [&](int T, int ch) {
         long long t = 0;
         for (int i : of) {
             const KGeom &g = p->host[i].g;
@@ -216,6 +229,14 @@ static TuneChoice default_tiles(const xct_batch_plan *p, const Arrangement &a, c
         }
         return t;
     });
+    double units = 0.0;
+    const double T = xct_pack_tile(1);
+    for (int i : a.list[2]) {
+        const KGeom &g = p->host[i].g;
+        units += (g.nx + 1.0) * (g.ny + 1.0) / (T * T) * (g.pa / g.ss);
+    }
+    c.runs = units >= 32.0 * p->ctx->sm_count;
+    return c;
 }
 
 // The graph's slices `want` in descriptor order and the launches of a subset step: work units,
@@ -224,8 +245,11 @@ static TuneChoice default_tiles(const xct_batch_plan *p, const Arrangement &a, c
 static int batch_layout(xct_batch_plan *p, const std::vector<int> &want, const TuneChoice *tiles)
 {
     const Arrangement a = arrange(p, want);
-    const TuneChoice c = tiles ? *tiles : p->tuned ? TuneChoice{p->fwd_T, p->fwd_chunk, 0.0f} : default_tiles(p, a, want);
+    const TuneChoice c = tiles ? *tiles
+                         : p->tuned ? TuneChoice{p->fwd_T, p->fwd_chunk, 0.0f, 0, p->tuned_runs}
+                                    : default_tiles(p, a, want);
     const int T = c.T, chunk = c.chunk;
+    const int big = c.runs ? large_chunk(p, a.list[2]) : 0;
     const std::vector<int> *list = a.list;
     const int *pack_ch = a.chunk;
     p->want = want;
@@ -240,12 +264,13 @@ static int batch_layout(xct_batch_plan *p, const std::vector<int> &want, const T
     std::vector<int> fin(1, 0);
     for (int q = 0; q < 3; ++q) {
         const int S = q == 0 ? 4 : q == 1 ? 2 : 1;
+        const bool large = S > 1 || big > 0;
         b.packs[q] = (int)list[q].size() / S;
         std::vector<int> f(1, 0), r(1, 0);
         for (size_t j = 0; j < list[q].size(); ++j) {
             XctItemDev &d = p->host[list[q][j]];
-            d.g.fwd_T = S > 1 ? xct_pack_tile(S) : T;
-            d.g.fwd_chunk = S > 1 ? pack_ch[q] : chunk;
+            d.g.fwd_T = large ? xct_pack_tile(S) : T;
+            d.g.fwd_chunk = S > 1 ? pack_ch[q] : large ? big : chunk;
             int uf, un, ub;
             xct_batched_units(d.g, S, d.fwd_ntx, d.fwd_nty, uf, un, d.bp_ntx, ub);
             if (j % S == 0) {
@@ -276,6 +301,7 @@ static int batch_layout(xct_batch_plan *p, const std::vector<int> &want, const T
     for (int i : want) p->glist_corr = p->glist_corr || p->host[i].corr_mode > 0;
     XCT_CUDA_TRY(cudaMemcpy(p->d_bases, p->bases.data(), sizeof(int) * p->bases.size(), cudaMemcpyHostToDevice));
     b.fwd_T = T;
+    b.large = big > 0;
     int rc = xct_batched_grids(p->ctx->sm_count, T, b.fwd_grid, b.bp_grid);
     if (rc) return rc;
     p->fwd_T = T;
@@ -531,6 +557,7 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
     p->key = graph_key(p);
     TuneChoice c;
     p->tuned = xct_tune_lookup(p->key, xct_tune_env_path(), c);
+    p->tuned_runs = c.runs;
     int rc = batch_layout(p, std::vector<int>(p->want), p->tuned ? &c : nullptr);
     if (rc) {
         batch_free(p);
@@ -812,6 +839,7 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
     TuneChoice best;
     if (!(flags & XCT_TUNE_FORCE) && xct_tune_lookup(p->key, cache_path, best)) {
         p->tuned = true;
+        p->tuned_runs = best.runs;
         return batch_layout(p, want, &best);
     }
     XCT_CUDA_TRY(cudaSetDevice(p->ctx->device));
@@ -830,12 +858,14 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    const TuneChoice before{p->fwd_T, p->fwd_chunk, 3.0e38f};
+    const TuneChoice before{p->fwd_T, p->fwd_chunk, 3.0e38f, 0, (int)p->step.large};
     best = before;
     int rc = cudaMemsetAsync(scratch, 0, sizeof(float) * maxpix, st) == cudaSuccess ? XCT_OK
                                                                                     : xct_fail(XCT_E_CUDA, "memset");
     if (p->step.packs[2] == 0) best.ms = 0.0f;  // packs only: nothing to choose
-    for (const TuneChoice &c : xct_tune_candidates(max_rows)) {
+    std::vector<TuneChoice> choices = xct_tune_candidates(max_rows);
+    choices.push_back(TuneChoice{before.T, before.chunk, 0.0f, 0, 1});  // the large tiles
+    for (const TuneChoice &c : choices) {
         if (rc || p->step.packs[2] == 0) break;
         if ((rc = batch_layout(p, want, &c))) break;
         for (int j = 0; j < m; ++j) {
@@ -857,7 +887,7 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
             cudaEventElapsedTime(&ms, e0, e1);
             if (r > 0) tmin = std::min(tmin, ms);
         }
-        if (rc == XCT_OK && tmin < best.ms) best = TuneChoice{c.T, c.chunk, tmin};
+        if (rc == XCT_OK && tmin < best.ms) best = c.runs ? TuneChoice{best.T, best.chunk, tmin, 0, 1} : TuneChoice{c.T, c.chunk, tmin};
     }
     cudaMemsetAsync(p->d_acc, 0, sizeof(double) * p->n_acc, st);
     cudaStreamSynchronize(st);
@@ -869,6 +899,7 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
         return rc;
     }
     p->tuned = true;
+    p->tuned_runs = best.runs;
     rc = batch_layout(p, want, &best);
     if (rc) return rc;
     return xct_tune_store(p->key, cache_path, best);

@@ -55,6 +55,7 @@ struct XctBatchStep {
     const int *fwd_base[3] = {}, *bp_base[3] = {}, *fin_base = nullptr;  // device, [packs + 1], [m + 1]
     int fwd_units[3] = {}, bp_units[3] = {}, fin_units = 0;
     int fwd_T = 92, fwd_grid = 0, bp_grid = 0;  // the single slices' forward tile and persistent grids
+    bool large = false;                         // ... or the large tiles, a CTA per unit
     int first(int q) const { return q == 0 ? 0 : q == 1 ? 4 * packs[0] : 4 * packs[0] + 2 * packs[1]; }
 };
 // Streams and events for the launches that run side by side.
@@ -202,7 +203,7 @@ struct TuneChoice {
     int T, chunk;
     float ms;
     int ms_chunk = 0;  // slice-interleaved forward projector's angle chunk; 0 = off
-    int runs = 0;      // a slice by itself is faster in runs of (tile, angle) units than with T and chunk
+    int runs = 0;      // a slice by itself is faster on the large tiles than with T and chunk
 };
 std::string xct_tune_key(const char *device, int nx, int ny, int px, int pa, int ss, int dN);
 bool xct_tune_lookup(const std::string &key, const char *path, TuneChoice &c);

@@ -811,8 +811,8 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
 // ----------------------------------------------------------------- batched launches
 // One subset step of many slices of different shapes, one launch per kernel and pack size.  Slices
 // of one geometry go in packs of four and of two through the grouped forward projector and the
-// several-slice backprojector, one CTA per (pack, tile) unit; the others one by one through persistent
-// CTAs that take (slice, tile) units from a device queue (an atomic counter) until the units run
+// several-slice backprojector, one CTA per (pack, tile) unit; the others one by one on the large tiles in the same
+// way, or on smaller ones through persistent CTAs that take (slice, tile) units from a device queue (an atomic counter) until the units run
 // out.  Units of pack (slice) i are [base[i], base[i+1]); they are independent within a launch, so
 // there is no waiting on other CTAs.
 // A pack pays per slice what the forward and backward kernels of several slices save (coordinates,
@@ -1007,7 +1007,7 @@ void xct_batched_units(const KGeom &g, int S, int &fwd_ntx, int &fwd_nty, int &f
 }
 
 // Forward tile side of a pack of S slices.
-int xct_pack_tile(int S) { return S == 4 ? FwdGroup<4>::Large : FwdGroup<2>::Large; }
+int xct_pack_tile(int S) { return S == 4 ? FwdGroup<4>::Large : S == 2 ? FwdGroup<2>::Large : FwdGroup<1>::Large; }
 
 // Persistent grids of the single slices' launches; the packs' shared-memory limits.
 int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid)
@@ -1045,6 +1045,7 @@ static int launch_fwd_pack(const XctBatchStep &b, int q, int sub, cudaStream_t s
 // The forward launch of the single slices of one subset step (the autotuner times it alone).
 int launch_fwd_batched(const XctBatchStep &b, int sub, int *queue, cudaStream_t st)
 {
+    if (b.large) return launch_fwd_pack<1>(b, 2, sub, st);
     return with_tile(b.fwd_T, [&](auto tc) -> int {
         constexpr int T = decltype(tc)::value;
         fwd_batched_kernel<T><<<b.fwd_grid, FwdTile<1, T>::Threads, FwdTile<1, T>::Smem, st>>>(

@@ -409,7 +409,8 @@ int xct_osem_profile(xct_plan *plan, int dN, const float *d_sino, float *d_img, 
  * neither).  A cached entry is reused without timing unless flags has XCT_TUNE_FORCE.
  * Synchronous.  xct_batch_plan_autotune does the same for a batch plan: each geometry
  * group's plan, and one choice for the slices its graph serves (the next xct_batch_run
- * captures its graph again).  The *_tuning calls report
+ * captures its graph again), the large tiles among its candidates; the tile reported is then the
+ * best of the others.  The *_tuning calls report
  * the current choice; xct_plan_set_tuning sets one by hand. */
 #define XCT_TUNE_FORCE 1
 int xct_plan_autotune(xct_plan *plan, int dN, const char *cache_path, int flags, void *stream);
