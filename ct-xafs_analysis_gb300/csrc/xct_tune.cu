@@ -1,6 +1,7 @@
 // xct_tune.cu -- the forward projector's tile autotuner and its cache.
 //
-// The tiled forward projector has two launch-shape parameters: the tile side T (44, 60, 76 or
+// The forward projector divides a launch into runs of (tile, angle) units by itself; a slice alone (or every slice,
+// with grouping off) can instead take a CTA per tile and chunk of angles, which has two launch-shape parameters: the tile side T (44, 60, 76 or
 // 92 base texels; a CTA stages one tile and serves its angles from shared memory) and the
 // number of subset angles one CTA serves (the chunk, 16..128).  Large values amortise the
 // staging and the per-ray interval search; small values give more CTAs, which small slices
@@ -8,7 +9,7 @@
 // three (36 warps) for T = 92, so the choice changes the occupancy, the grid's granularity and
 // the per-tile overheads -- a trade-off that depends on the slice size, the angles per subset
 // and the slices per call, so it is measured: xct_plan_autotune times every candidate on the plan's
-// own geometry and keeps the fastest; the choice is cached per (device, shape) in memory and,
+// own geometry, keeps the fastest and times the runs against it; the choice is cached per (device, shape) in memory and,
 // optionally, in a JSON file that later plans (and processes) read.
 #include <stdio.h>
 #include <stdlib.h>
@@ -174,8 +175,8 @@ static int plan_default_ms_chunk(const xct_plan *p)
 }
 
 // The per-slice forward tiles of a plan that has no cached choice: the tile side and the even split
-// of the subset's angles with the least modelled time for one slice (several slices go through the
-// grouped forms, whose tiles are fixed).
+// of the subset's angles with the least modelled time for one slice (used with grouping off; otherwise the
+// slices go through the grouped forms, whose tiles are fixed).
 static TuneChoice plan_default_tiles(const xct_plan *p)
 {
     const int rows = (p->g.pa + p->g.ss - 1) / p->g.ss, cap = fwd_tiled_rows_cap();
