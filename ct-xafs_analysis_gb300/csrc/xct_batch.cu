@@ -1,12 +1,12 @@
-// xct_batch.cu -- OS-EM over many slices of different shapes in one graph of persistent
+// xct_batch.cu -- OS-EM over many slices of different shapes in one captured graph of
 // launches (CT-XAFS stacks: energies x slices, every slice its own width, bin count and
 // angle list).
 //
 // The reference reconstructs a batch of dN slices of ONE shape per OSEM_execution call
 // (GPU.cpp:125-240).  A batch plan instead holds n slices of any shapes that share the
-// subset count; every subset step is three persistent launches -- forward projection,
-// ratio, backprojection+update -- whose CTAs take (slice, tile) work units from a device
-// queue, so small slices fill the GPU together with large ones.  The whole subset/iteration
+// subset count; every subset step is three launches -- forward projection, ratio,
+// backprojection+update -- over the (slice, tile) work units of all slices, so small slices
+// fill the GPU together with large ones.  The whole subset/iteration
 // loop is captured once in a CUDA graph and replayed; the slices' buffer pointers live in a
 // device descriptor table written before each replay, so one plan serves any buffers of
 // the planned shapes.
@@ -34,7 +34,7 @@ struct xct_batch_plan {
     std::vector<XctItemDev> host;     // descriptors (pointers filled per run)
     XctItemDev *d_items = nullptr;
     int *d_bases = nullptr;           // prefix sums of the launches' work units
-    int *d_queues = nullptr;          // [it*ss][2]
+    int *d_queues = nullptr;          // [it*ss]
     float2 *d_trig = nullptr;
     float *d_ratio = nullptr;
     double *d_acc = nullptr;
@@ -302,7 +302,7 @@ static int batch_layout(xct_batch_plan *p, const std::vector<int> &want, const T
     XCT_CUDA_TRY(cudaMemcpy(p->d_bases, p->bases.data(), sizeof(int) * p->bases.size(), cudaMemcpyHostToDevice));
     b.fwd_T = T;
     b.large = big > 0;
-    int rc = xct_batched_grids(p->ctx->sm_count, T, b.fwd_grid, b.bp_grid);
+    int rc = xct_batched_grid(p->ctx->sm_count, T, b.fwd_grid);
     if (rc) return rc;
     p->fwd_T = T;
     p->fwd_chunk = chunk;
@@ -477,7 +477,7 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
     if ((e = cudaMalloc(&p->d_bases, sizeof(int) * (3 * (size_t)n + 7))) != cudaSuccess)
         return fail(e, "cudaMalloc bases");
     p->n_acc = n_acc;
-    p->queue_bytes = sizeof(int) * 2 * (size_t)std::max(1, it * ss);
+    p->queue_bytes = sizeof(int) * (size_t)std::max(1, it * ss);
     if ((e = cudaMalloc(&p->d_queues, p->queue_bytes)) != cudaSuccess) return fail(e, "cudaMalloc queues");
     if ((e = cudaMalloc(&p->d_trig, sizeof(float2) * n_trig)) != cudaSuccess) return fail(e, "cudaMalloc trig");
     if ((e = cudaMalloc(&p->d_ratio, sizeof(float) * n_ratio)) != cudaSuccess) return fail(e, "cudaMalloc ratio");
@@ -605,7 +605,7 @@ static int capture(xct_batch_plan *p)
                 rc = launch_ista3d_stacks(p->d_stacks, ns, p->max_vox, p->cs_lambda, sm, p->cap);
                 first = false;
             } else {
-                rc = launch_osem_step_batched(p->step, p->sub[k], p->d_queues + 2 * (size_t)(i * p->ss + k), p->cap,
+                rc = launch_osem_step_batched(p->step, p->sub[k], p->d_queues + (size_t)(i * p->ss + k), p->cap,
                                               p->side);
                 if (rc == XCT_OK && cs) rc = launch_fista3d_stacks(p->d_stacks, ns, p->max_vox, p->cs_lambda, sm, p->cap);
             }

@@ -54,7 +54,7 @@ struct XctBatchStep {
     int packs[3] = {0, 0, 0};
     const int *fwd_base[3] = {}, *bp_base[3] = {}, *fin_base = nullptr;  // device, [packs + 1], [m + 1]
     int fwd_units[3] = {}, bp_units[3] = {}, fin_units = 0;
-    int fwd_T = 92, fwd_grid = 0, bp_grid = 0;  // the single slices' forward tile and persistent grids
+    int fwd_T = 92, fwd_grid = 0;               // the single slices' forward tile and persistent grid
     bool large = false;                         // ... or the large tiles, a CTA per unit
     int first(int q) const { return q == 0 ? 0 : q == 1 ? 4 * packs[0] : 4 * packs[0] + 2 * packs[1]; }
 };
@@ -173,14 +173,14 @@ int launch_fwd_direct(const KGeom &g, const float2 *trig, const float *img, cons
 int launch_bp_update_direct(const KGeom &g, const float2 *trig, float *img, const float *ratio, int dN, int sub,
                             cudaStream_t st);
 // Batched launches (xct_tiled.cu): the work units of a pack of S slices of one geometry, the
-// persistent grids of the single slices, and one subset step (forward, finalize, backprojection) over
+// persistent grid of the single slices, and one subset step (forward, finalize, backprojection) over
 // all slices.
 void xct_batched_units(const KGeom &g, int S, int &fwd_ntx, int &fwd_nty, int &fwd_units, int &fin_units, int &bp_ntx,
                        int &bp_units);
 int xct_pack_tile(int S);
 double xct_pack_work(int nx, int ny, int S, int nrows, int chunk, double &tail);
-int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid);
-int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queues, cudaStream_t st, const XctBatchSide &side);
+int xct_batched_grid(int sm_count, int fwd_T, int &fwd_grid);
+int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queue, cudaStream_t st, const XctBatchSide &side);
 bool xct_fwd_tile_valid(int T);
 int launch_fwd_batched(const XctBatchStep &b, int sub, int *queue, cudaStream_t st);
 int xct_check_geom(const xct_geom *g);

@@ -18,15 +18,6 @@ __device__ __forceinline__ void xct_grid_wait() { asm volatile("griddepcontrol.w
 // lets the next launch's blocks be scheduled as this grid's leave room for them
 __device__ __forceinline__ void xct_grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// A plain global load (never the read-only path: its data may have been written while this grid was
-// already resident) through a pointer that is otherwise not aliased.
-__device__ __forceinline__ float ld_global(const float *p)
-{
-    float v;
-    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
 template <class... P, class... A>
 static inline int xct_launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A &&...args)
 {

@@ -19,7 +19,7 @@
 // and clears it for the next subset.
 //
 // Backprojector (OSEM2, OSEM.cl:71-105), footprint-staged:
-//   * one CTA owns a pixel tile (32x32 of up to eight slices; 64x64 of one in the batched launches); per
+//   * one CTA owns a pixel tile (32x32 of up to eight slices); per
 //     angle it stages the window of ratio bins its pixels hit (bin coordinates are monotone in X and in
 //     Y, so the tile corners bound the window exactly) into shared memory;
 //   * each thread gathers its pixels' bins per angle, in angle order, evaluating the
@@ -50,17 +50,6 @@ constexpr int kAngChunk = 128;  // most subset angles one forward-projector CTA 
 // lengths inside a tile, so few lanes idle.
 constexpr int kLanesPerRay = 4;
 constexpr int kRaysPerWarp = 32 / kLanesPerRay;
-
-constexpr int kBpTX = 64, kBpTY = 64;  // backprojection tile (pixels)
-// A thread of bp_tile takes 8 pixels of R rows (kBpTY / R apart): R = 4 shares the
-// products Xc*c over four rows (128 threads, 80 registers).
-template <int R>
-struct BpCfg {
-    static constexpr int Threads = (kBpTX / 8) * (kBpTY / R);
-    static constexpr int Stride = kBpTY / R;
-};
-constexpr int kBpW = 96;               // staged bins per angle (>= 63|c| + 63|s| + 3 = 92.1)
-constexpr int kBpChunk = 64;           // angles per staging pass of the backprojector
 
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 
@@ -486,146 +475,22 @@ __global__ void __launch_bounds__(256) fwd_finalize4_kernel(double *acc, const f
     finalize4(acc + ((size_t)z * nrows + k) * g.px + X, meas != nullptr ? meas + o : nullptr, out + o);
 }
 
-// ------------------------------------------------------------------- backprojector
-struct BpShared {
-    float win[kBpChunk * kBpW];
-    float2 scs[kBpChunk];     // (c, s)
-    int slo[kBpChunk];        // first staged bin of the angle's window
-    unsigned soff[kBpChunk];  // byte address of window entry (bits - BIAS - lo)
-};
-
-// The work of one CTA: pixel tile (bx, by) of one slice (image img, ratio rt [pa][px]),
-// angles th = sub + k*ss for k < nang (as OSEM2 loops).  Starts/ends with threads in step.
-template <int kBpRows>
-__device__ __forceinline__ void bp_tile(const KGeom &g, float *__restrict__ img, const float *__restrict__ rt,
-                                        const float2 *__restrict__ trig, int sub, int nang, int bx, int by,
-                                        float ssf, float paf, BpShared &sh)
-{
-    float *win = sh.win;
-    float2 *scs = sh.scs;
-    int *slo = sh.slo;
-    unsigned *soff = sh.soff;
-    const int X0 = bx * kBpTX, Y0 = by * kBpTY;
-    const int X1 = min(X0 + kBpTX, g.nx) - 1, Y1 = min(Y0 + kBpTY, g.ny) - 1;
-    // 8 threads x 8 pixels across, thread tx taking X0 + tx + 8i (the 8 lanes of a row read
-    // neighbouring bins and write neighbouring pixels); thread row ty covers rows
-    // ty + r * (kBpTY / kBpRows)
-    constexpr int kStride = BpCfg<kBpRows>::Stride, kBpThreads = BpCfg<kBpRows>::Threads;
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-    // threads past the image edge of a partial tile gather for the edge pixel (inside the
-    // staged window) and write nothing
-    float Ycr[kBpRows];
-#pragma unroll
-    for (int r = 0; r < kBpRows; ++r) Ycr[r] = (float)min(Y0 + ty + r * kStride, Y1) - g.hy;
-    f2x xcp[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float a = (float)min(X0 + tx + 16 * j, X1) - g.hx;
-        const float b = (float)min(X0 + tx + 16 * j + 8, X1) - g.hx;
-        xcp[j] = f2_pack(a, b);
-    }
-    f2x acc[kBpRows][4];  // pixel pairs of each row, packed adds (each lane an IEEE add)
-#pragma unroll
-    for (int r = 0; r < kBpRows; ++r)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[r][j] = f2_pack(0.0f, 0.0f);
-    const f2x cxp = f2_pack(g.cx, g.cx);
-    const f2x hp = f2_pack(0.5f, 0.5f);
-    const f2x MM = f2_pack(kMagic, kMagic);
-    const unsigned wbase = (unsigned)__cvta_generic_to_shared(win);
-
-    for (int k0 = 0; k0 < nang; k0 += kBpChunk) {
-        const int kn = min(kBpChunk, nang - k0);
-        __syncthreads();  // the previous chunk's gathers are done with the shared arrays
-        for (int k = threadIdx.x; k < kn; k += kBpThreads) {
-            const float2 cs = trig[sub + (k0 + k) * g.ss];
-            scs[k] = cs;
-            // the bin coordinate is monotone in X and in Y: the corners bound the window
-            const float xa = (float)X0 - g.hx, xb = (float)X1 - g.hx;
-            const float yA = (float)Y0 - g.hy, yB = (float)Y1 - g.hy;
-            const float qa = yA * cs.y, qb = yB * cs.y;
-            int lo = xct_floor_bits(xct_bin_coord(xa, cs.x, qa, g.cx));
-            lo = min(lo, xct_floor_bits(xct_bin_coord(xb, cs.x, qa, g.cx)));
-            lo = min(lo, xct_floor_bits(xct_bin_coord(xa, cs.x, qb, g.cx)));
-            lo = min(lo, xct_floor_bits(xct_bin_coord(xb, cs.x, qb, g.cx)));
-            slo[k] = lo - XCT_FLOOR_BIAS;
-            // entry for floor bits fb: wbase + 4*(k*W + fb - lo)  (mod 2^32)
-            soff[k] = wbase + 4u * (unsigned)(k * kBpW) - 4u * (unsigned)lo;
-        }
-        __syncthreads();
-        // element j of angle k holds ratio[th][lo_k + j] (0 off the detector)
-        for (int i = threadIdx.x; i < kn * kBpW; i += kBpThreads) {
-            const int k = i / kBpW, j = i - k * kBpW;
-            const int bin = slo[k] + j;
-            const int th = sub + (k0 + k) * g.ss;
-            win[i] = ((unsigned)bin < (unsigned)g.px) ? ld_global(rt + (size_t)th * g.px + bin) : 0.0f;
-        }
-        __syncthreads();
-        const unsigned wlo = wbase, whi = wbase + 4u * (unsigned)(kn * kBpW - 1);
-        (void)wlo;
-        (void)whi;
-        for (int k = 0; k < kn; ++k) {
-            const float c = scs[k].x, s = scs[k].y;
-            const unsigned off = soff[k];
-            float q[kBpRows];
-#pragma unroll
-            for (int r = 0; r < kBpRows; ++r) q[r] = Ycr[r] * s;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // Xc*c - q in scalar: ptxas contracts a packed multiply feeding a packed
-                // subtract into one fused operation whatever the rounding modifiers, and the
-                // reference rounds the product and the difference separately.  The products
-                // serve every row; the three additions that follow are packed:
-                // ((.) + cx) + 0.5, then floor.
-                float xa, xb;
-                f2_unpack(xcp[j], xa, xb);
-                const float pa_ = xa * c, pb_ = xb * c;
-#pragma unroll
-                for (int r = 0; r < kBpRows; ++r) {
-                    const f2x t = f2_add_rd(f2_add(f2_add(f2_pack(pa_ - q[r], pb_ - q[r]), cxp), hp), MM);
-                    int b0, b1;
-                    f2_unpack_bits(t, b0, b1);
-                    const unsigned ad0 = (unsigned)b0 * 4u + off, ad1 = (unsigned)b1 * 4u + off;
-                    const float v0 = XCT_IN(ad0, wlo, whi, XCT_SITE_BP_WIN) ? lds_f1(ad0) : 0.0f;
-                    const float v1 = XCT_IN(ad1, wlo, whi, XCT_SITE_BP_WIN) ? lds_f1(ad1) : 0.0f;
-                    acc[r][j] = f2_add(acc[r][j], f2_pack(v0, v1));
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < kBpRows; ++r) {
-        const int Y = Y0 + ty + r * kStride;
-        if (Y > Y1) continue;
-        float *row = img + (size_t)Y * g.nx;
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) f2_unpack(acc[r][j], v[2 * j], v[2 * j + 1]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int X = X0 + tx + 8 * i;
-            if (X <= X1) row[X] = xct_update(row[X], v[i], ssf, paf);
-        }
-    }
-    __syncthreads();  // the shared arrays may be restaged by the caller's next tile
-}
-
 // --------------------------------------------- backprojector, one to eight slices per tile
 // For the slices of one OS-EM call (one geometry) a (pixel, angle) pair reads the same bin in
 // all S slices of a group, so the bin expression is evaluated once for S gathers.  A
 // CTA of 256 threads owns a 32 x 32 pixel tile of S slices and stages, per angle and
-// slice, the window of the tile's bins (< 48, bounded exactly by the tile corners as in
-// bp_tile, its start rounded down to a multiple of 4) with asynchronous 16-byte copies
+// slice, the window of the tile's bins (< 48, bounded exactly by the tile corners -- the bin coordinate is
+// monotone in X and in Y -- its start rounded down to a multiple of 4) with asynchronous 16-byte copies
 // (zero-filled off the detector), a chunk of angles at a time.  A thread takes 4 pixels of one row (8
 // apart), a warp 8 adjacent pixels in each of 4 rows: the bins one load instruction touches
 // span fewer than 32 consecutive words, so no load has a bank conflict.  Per pixel and angle:
-// the literal bin expression of bp_tile, one address, S 4-byte loads at constant
+// the reference's bin expression ((Xc*c - Yc*s) + cx) + 0.5, one address, S 4-byte loads at constant
 // offsets (one per slice), packed adds over slice pairs (pixel pairs for one slice) -- in angle order,
-// so each slice's sum is bp_tile's bit for bit -- and the update at the end.
+// so each slice's sum is the same bits in every form -- and the update at the end.
 // Bound: the shared-memory data path from two slices on (4 B per gather and slice), issue for one (5
 // instructions, 7 operations of the FP32 pipe a gather).  The small tiles also spread one slice over the SMs:
-// 2048^2 has 4096 of them against 1024 of bp_tile's 64 x 64 (1.7 waves).  100 angles of one 2048^2 slice:
-// 95 us against 108 with 64 x 64 tiles; three slices of 509 x 487 with 31 angles: 15 against 27.
+// 2048^2 has 4096 of them, and 1024 tiles of 64 x 64 would be 1.7 waves.  100 angles of one 2048^2 slice:
+// 95 us (108 with 64 x 64 tiles); three slices of 509 x 487 with 31 angles: 15 (27).
 constexpr int kMsSlices = 8;  // slices per group of the slice-interleaved kernels
 constexpr int kBpMsT = 32;
 constexpr int kBpMsThreads = 256;
@@ -736,7 +601,9 @@ __device__ __forceinline__ void bp_ms_tile(const KGeom &g, Image image, const fl
             const float q = Yc * s;
 #pragma unroll
             for (int j = 0; j < kBpMsPix / 2; ++j) {
-                // the literal bin expression of bp_tile for pixels 2j and 2j+1
+                // the bin expression for pixels 2j and 2j+1.  Xc*c - q in scalar: ptxas contracts a packed
+                // multiply feeding a packed subtract into one fused operation whatever the rounding
+                // modifiers, and the reference rounds the product and the difference separately
                 const float pa_ = xc[2 * j] * c, pb_ = xc[2 * j + 1] * c;
                 const f2x tt = f2_add_rd(f2_add(f2_add(f2_pack(pa_ - q, pb_ - q), cxp), hp), MM);
                 int b0, b1;
@@ -813,7 +680,10 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
 // of one geometry go in packs of four and of two through the grouped forward projector and the
 // several-slice backprojector, one CTA per (pack, tile) unit; the others one by one on the large tiles in the same
 // way, or on smaller ones through persistent CTAs that take (slice, tile) units from a device queue (an atomic counter) until the units run
-// out.  Units of pack (slice) i are [base[i], base[i+1]); they are independent within a launch, so
+// out.  The single slices' backprojection has one CTA per unit too: what a few of them beside packs take is the
+// time of one CTA over all angles, and on tiles of 64 x 64 that made packs slower than no packs (two
+// geometries of three slices 300 and 320 wide, 240 and 270 angles: 663 us an iteration against 591; on 32 x 32 tiles
+// 363 against 369).  Units of pack (slice) i are [base[i], base[i+1]); they are independent within a launch, so
 // there is no waiting on other CTAs.
 // A pack pays per slice what the forward and backward kernels of several slices save (coordinates,
 // addresses and weights once), and takes the large tiles, one CTA per SM: one iteration of 24 slices, 12
@@ -921,26 +791,6 @@ __global__ void fwd_finalize_batched_kernel(const XctItemDev *__restrict__ items
     }
 }
 
-__global__ void __launch_bounds__(BpCfg<4>::Threads) bp_batched_kernel(const XctItemDev *__restrict__ items,
-                                                              const int *__restrict__ base, int n, int sub,
-                                                              int *queue)
-{
-    __shared__ BpShared sh;
-    __shared__ int s_unit, s_item;
-    const int total = base[n];
-    for (;;) {
-        const int u = queue_take(queue, &s_unit);
-        if (u >= total) break;
-        const int i = unit_item(base, n, u, &s_item);
-        const XctItemDev &it = items[i];
-        const KGeom &g = it.g;
-        const int nang = (g.pa - sub + g.ss - 1) / g.ss;
-        const int t = u - base[i];
-        bp_tile<4>(g, it.img, it.ratio, it.trig, sub, nang, t % it.bp_ntx, t / it.bp_ntx, (float)g.ss, (float)g.pa,
-                sh);
-    }
-}
-
 // grid: one CTA per backprojection unit; a pack's ratio images lie one after the other.
 template <int S>
 __global__ void __launch_bounds__(kBpMsThreads) bp_pack_kernel(const XctItemDev *__restrict__ items,
@@ -1001,18 +851,17 @@ void xct_batched_units(const KGeom &g, int S, int &fwd_ntx, int &fwd_nty, int &f
     const int rows = (g.pa + g.ss - 1) / g.ss;  // the largest subset (cover mode)
     fwd_units = fwd_ntx * fwd_nty * ((rows + g.fwd_chunk - 1) / g.fwd_chunk);
     fin_units = rows;
-    const int tx = S > 1 ? kBpMsT : kBpTX, ty = S > 1 ? kBpMsT : kBpTY;
-    bp_ntx = (g.nx + tx - 1) / tx;
-    bp_units = bp_ntx * ((g.ny + ty - 1) / ty);
+    bp_ntx = (g.nx + kBpMsT - 1) / kBpMsT;
+    bp_units = bp_ntx * ((g.ny + kBpMsT - 1) / kBpMsT);
 }
 
 // Forward tile side of a pack of S slices.
 int xct_pack_tile(int S) { return S == 4 ? FwdGroup<4>::Large : S == 2 ? FwdGroup<2>::Large : FwdGroup<1>::Large; }
 
-// Persistent grids of the single slices' launches; the packs' shared-memory limits.
-int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid)
+// Persistent grid of the single slices' forward launch.
+int xct_batched_grid(int sm_count, int fwd_T, int &fwd_grid)
 {
-    int a = 0, c = 0;
+    int a = 0;
     int rc = with_tile(fwd_T, [&](auto tc) -> int {
         constexpr int T = decltype(tc)::value;
         static std::atomic<bool> done[64];
@@ -1023,9 +872,7 @@ int xct_batched_grids(int sm_count, int fwd_T, int &fwd_grid, int &bp_grid)
         return XCT_OK;
     });
     if (rc) return rc;
-    XCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, bp_batched_kernel, BpCfg<4>::Threads, 0));
     fwd_grid = sm_count * (a > 0 ? a : 1);
-    bp_grid = sm_count * (c > 0 ? c : 1);
     return XCT_OK;
 }
 
@@ -1057,7 +904,7 @@ int launch_fwd_batched(const XctBatchStep &b, int sub, int *queue, cudaStream_t 
 
 // One subset step.  The launches of the pack sizes in use run side by side (sizes beyond the first on
 // side streams, so that one's last CTAs and the next one's first share the SMs).
-int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queues /*[2]*/, cudaStream_t st, const XctBatchSide &side)
+int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queue, cudaStream_t st, const XctBatchSide &side)
 {
     auto parallel = [&](auto &&launch) -> int {
         int used = 0, rc = XCT_OK;
@@ -1079,7 +926,7 @@ int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queues /*[2]*/
     int rc = parallel([&](int q, cudaStream_t on) -> int {
         return q == 0 ? launch_fwd_pack<4>(b, q, sub, on)
                : q == 1 ? launch_fwd_pack<2>(b, q, sub, on)
-                        : launch_fwd_batched(b, sub, queues, on);
+                        : launch_fwd_batched(b, sub, queue, on);
     });
     if (rc) return rc;
     if (b.fin_units > 0) {
@@ -1093,7 +940,7 @@ int launch_osem_step_batched(const XctBatchStep &b, int sub, int *queues /*[2]*/
         else if (q == 1)
             bp_pack_kernel<2><<<b.bp_units[q], kBpMsThreads, 0, on>>>(it, b.bp_base[q], b.packs[q], sub);
         else
-            bp_batched_kernel<<<b.bp_grid, BpCfg<4>::Threads, 0, on>>>(it, b.bp_base[q], b.packs[q], sub, queues + 1);
+            bp_pack_kernel<1><<<b.bp_units[q], kBpMsThreads, 0, on>>>(it, b.bp_base[q], b.packs[q], sub);
         XCT_CUDA_TRY(cudaGetLastError());
         return XCT_OK;  // launches are counted when the captured graph is replayed
     });
