@@ -244,6 +244,7 @@ int xct_osem_plan_create(xct_ctx *ctx, const xct_geom *geom, xct_plan **out)
     p->sub_default.resize(geom->ss);
     xct_subset_order_host(geom->ss, p->sub_default.data());
     KGeom &k = p->kg;
+    k.splits = &p->splits;
     k.nx = geom->nx;
     k.ny = geom->ny;
     k.px = geom->px;

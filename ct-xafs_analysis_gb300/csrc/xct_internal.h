@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <functional>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -11,6 +12,7 @@
 
 // Geometry as the kernels see it (passed by value).  Half sizes are precomputed exactly
 // as the reference's expressions produce them (IMAGESIZE_X*0.5f etc., OSEM.cl:58-59,95).
+struct XctFwdSplits;
 struct KGeom {
     int nx, ny;      // image
     int px, pa;      // sinogram
@@ -27,6 +29,30 @@ struct KGeom {
     int fwd_group = 1;   // forward projection of several slices per CTA (0: one, by hand)
     int fwd_tuned = 0;   // fwd_T and fwd_chunk were measured or set by hand: single slices keep them
     int fwd_direct = 1;  // small problems take the kernels of xct_direct.cu (0: a tile chosen by hand)
+    XctFwdSplits *splits = nullptr;  // (host) the divisions of the forward launches kept so far, or none
+};
+
+// How a forward launch divides groups * ntx * nty tiles (sides tx, ty) x nrows angles among its CTAs.
+// chunk > 0: a CTA per tile and chunk of angles, chunks of all tiles one after the other.  chunk = 0: CTA i
+// takes the run of (tile, angle) units start[i] .. start[i+1]-1 (tile by tile), whatever tile boundaries it
+// crosses.
+constexpr int kMaxRuns = 320;
+struct FwdSplit {
+    int ntx, nty, tx, ty, chunk, ctas;
+    int cap;  // most angles a CTA serves from one staging
+    unsigned start[kMaxRuns + 1];
+};
+// The divisions that one geometry's launches take, found once (see launch_fwd_groups): the last kKept of them.
+struct XctFwdSplits {
+    static constexpr int kKept = 12;
+    struct Entry {
+        int S = 0, groups = 0, nrows = 0, cap = 0;
+        bool large = false;  // ... on the large tiles
+        FwdSplit f;
+    };
+    std::mutex mu;
+    Entry kept[kKept];
+    int next = 0;
 };
 
 // One slice of a batched launch (device-side descriptor).
@@ -108,6 +134,7 @@ struct xct_plan {
     float *d_img2 = nullptr;
     cudaStream_t s_h2d = nullptr, s_d2h = nullptr;
     int acc_rows = 0;
+    XctFwdSplits splits;         // kg.splits
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // OS-EM of a batch runs its two halves on the caller's stream and on s_aux (fork/join by

@@ -132,7 +132,9 @@ extern "C" int xct_osem_run_static(const xct_geom *g, int dN, const float *d_sin
     XCT_CUDA_TRY(cudaMemsetAsync(d_acc, 0, acc_bytes, st));
     XCT_CUDA_TRY(cudaMemsetAsync(d_ratio, 0, ratio_bytes, st));
 
+    XctFwdSplits splits;  // this call's
     KGeom k;
+    k.splits = &splits;
     k.nx = g->nx;
     k.ny = g->ny;
     k.px = g->px;
