@@ -354,7 +354,7 @@ static int xct_osem_split(const xct_plan *p, int dN)
 static int xct_stream_split(const xct_plan *p, int dN)
 {
     const bool one = dN < 4 || fwd_is_small(p->kg, dN, (p->g.pa + p->g.ss - 1) / p->g.ss);
-    return p->g.kernels == XCT_KERNELS_TILED && p->kg.fwd_group && one ? dN : xct_osem_split(p, dN);
+    return p->g.kernels == XCT_KERNELS_TILED && p->kg.fwd_group && !p->kg.fwd_hand && one ? dN : xct_osem_split(p, dN);
 }
 
 // One subset step (OSEM1 then OSEM2) of dN slices with the given plan buffers (ratio

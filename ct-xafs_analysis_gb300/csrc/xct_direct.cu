@@ -138,14 +138,17 @@ __global__ void __launch_bounds__(128) bp_direct_kernel(float *img, const float 
 
 }  // namespace
 
+// a tile or a switch set by hand holds whatever the size
+static bool by_hand(const KGeom &g) { return g.fwd_hand || g.ms_hand; }
+
 bool fwd_is_direct(const KGeom &g, int dN, int nrows)
 {
-    return g.fwd_direct && (long long)g.nx * g.ny * nrows * dN <= kDirectTaps && nrows <= 65535 && dN <= 65535;
+    return !by_hand(g) && (long long)g.nx * g.ny * nrows * dN <= kDirectTaps && nrows <= 65535 && dN <= 65535;
 }
 
 bool bp_is_direct(const KGeom &g, int dN)
 {
-    return g.fwd_direct && (long long)g.nx * g.ny * dN <= kDirectPixels && dN <= 65535;
+    return !by_hand(g) && (long long)g.nx * g.ny * dN <= kDirectPixels && dN <= 65535;
 }
 
 int launch_fwd_direct(const KGeom &g, const float2 *trig, const float *img, const float *meas, float *out, int dN, int sub,

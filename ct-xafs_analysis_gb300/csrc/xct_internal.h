@@ -26,9 +26,10 @@ struct KGeom {
     int fwd_chunk;   // tiled forward projector: subset angles per CTA (1..128)
     int ms_chunk = 0;  // slice-interleaved kernels: most subset angles per forward CTA (1..128);
                        // 0 = off (the backprojectors and the adjoint then work slice by slice)
-    int fwd_group = 1;   // forward projection of several slices per CTA (0: one, by hand)
+    int fwd_group = 1;   // several slices per CTA in the forms that have them (0: one, by hand)
     int fwd_tuned = 0;   // fwd_T and fwd_chunk were measured or set by hand: single slices keep them
-    int fwd_direct = 1;  // small problems take the kernels of xct_direct.cu (0: a tile chosen by hand)
+    int fwd_hand = 0;    // ... set by hand: all slices keep them but whole groups of eight with ms_chunk > 0
+    int ms_hand = 0;     // ms_chunk (and fwd_group with it) was set by hand
     XctFwdSplits *splits = nullptr;  // (host) the divisions of the forward launches kept so far, or none
 };
 

@@ -1146,14 +1146,15 @@ static int launch_fwd_groups(const KGeom &g, const float2 *trig, const float *&i
 bool fwd_is_small(const KGeom &g, int dN, int nrows) { return (long long)g.nx * g.ny * nrows * dN <= 30000000; }
 
 // The forward projection of dN slices into the accumulator: groups of four slices, the rest as one
-// group of five, three, two or one (small batches of five, ten ...: fives); with grouping off or a tuned tile
-// every slice by itself in chunks of angles.
+// group of five, three, two or one (small batches of five, ten ...: fives); with grouping off or a tuned tile and one
+// slice, every slice by itself in chunks of angles.  A tile set by hand serves every slice but, with the eight-slice
+// forms on, whole groups of eight.
 int launch_fwd_tiled_main(const KGeom &g, const float2 *trig, const float *img, double *acc, int dN, int sub, int step,
                           int nrows, cudaStream_t st)
 {
     if (nrows <= 0 || dN <= 0) return XCT_OK;
-    if (g.fwd_group && (dN >= 2 || !g.fwd_tuned)) {
-        int rc = XCT_OK;
+    int rc = XCT_OK;
+    if (g.fwd_group && !g.fwd_hand && (dN >= 2 || !g.fwd_tuned)) {
         if (dN % 5 == 0 && fwd_is_small(g, dN, nrows)) return launch_fwd_groups<5>(g, trig, img, acc, dN, dN / 5, sub, step, nrows, st);
         const bool five = dN > 1 && dN % 4 == 1;
         rc = launch_fwd_groups<4>(g, trig, img, acc, dN, five ? dN / 4 - 1 : dN / 4, sub, step, nrows, st);
@@ -1162,6 +1163,10 @@ int launch_fwd_tiled_main(const KGeom &g, const float2 *trig, const float *img, 
         if (!rc && dN == 2) rc = launch_fwd_groups<2>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
         if (!rc && dN == 1) rc = launch_fwd_groups<1>(g, trig, img, acc, dN, 1, sub, step, nrows, st);
         return rc;
+    }
+    if (g.fwd_group && g.fwd_hand && g.ms_chunk > 0) {
+        rc = launch_fwd_groups<4>(g, trig, img, acc, dN, dN / kMsSlices * 2, sub, step, nrows, st);
+        if (rc || dN == 0) return rc;
     }
     if (g.fwd_chunk <= 0 || g.fwd_chunk > kAngChunk) return xct_fail(XCT_E_INVALID, "forward angle chunk out of range");
     return with_tile(g.fwd_T, [&](auto tc) -> int {

@@ -228,8 +228,7 @@ int xct_plan_set_tuning(xct_plan *p, int fwd_tile, int ang_chunk)
     p->kg.fwd_T = fwd_tile;
     p->kg.fwd_chunk = ang_chunk;
     p->kg.fwd_tuned = 1;
-    p->kg.fwd_direct = 0;  // tiles chosen by hand are used whatever the size and the batch
-    p->kg.fwd_group = 0;
+    p->kg.fwd_hand = 1;
     return XCT_OK;
 }
 
@@ -249,7 +248,7 @@ int xct_plan_set_multislice(xct_plan *p, int ang_chunk)
         return xct_fail(XCT_E_UNSUPPORTED, "xct_plan_set_multislice: the plain kernels have no slice-interleaved form");
     p->kg.ms_chunk = ang_chunk;
     p->kg.fwd_group = ang_chunk > 0;
-    p->kg.fwd_direct = 0;  // a switch set by hand holds whatever the size
+    p->kg.ms_hand = 1;
     return XCT_OK;
 }
 
@@ -266,6 +265,7 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
         p->kg.fwd_T = best.T;
         p->kg.fwd_chunk = best.chunk;
         p->kg.fwd_tuned = !best.runs;
+        p->kg.fwd_hand = 0;
         return XCT_OK;
     }
     XCT_CUDA_TRY(cudaSetDevice(p->ctx->device));
@@ -297,6 +297,7 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
     };
     KGeom k = saved;
     k.fwd_group = 0;  // the choice is the per-slice kernel's
+    k.fwd_hand = 0;
     for (const TuneChoice &c : xct_tune_candidates(rows)) {
         k.fwd_T = c.T;
         k.fwd_chunk = c.chunk;
@@ -320,6 +321,7 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
     p->kg.fwd_T = best.T;
     p->kg.fwd_chunk = best.chunk;
     p->kg.fwd_tuned = !best.runs;
+    p->kg.fwd_hand = 0;
     return xct_tune_store(key, cache_path, best);
 }
 

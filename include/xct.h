@@ -411,7 +411,9 @@ int xct_osem_profile(xct_plan *plan, int dN, const float *d_sino, float *d_img, 
  * group's plan, and one choice for the slices its graph serves (the next xct_batch_run
  * captures its graph again), the large tiles among its candidates; the tile reported is then the
  * best of the others.  The *_tuning calls report
- * the current choice; xct_plan_set_tuning sets one by hand. */
+ * the current choice; xct_plan_set_tuning sets one by hand, for the forward projection of every slice at
+ * any size but of whole groups of eight with the slice-interleaved kernels on (below), until the autotuner
+ * chooses again; the other kernels' grouping of slices stays as it is. */
 #define XCT_TUNE_FORCE 1
 int xct_plan_autotune(xct_plan *plan, int dN, const char *cache_path, int flags, void *stream);
 int xct_plan_tuning(xct_plan *plan, int *fwd_tile, int *ang_chunk);
