@@ -479,6 +479,8 @@ static int osem_loop_maybe_traced(xct_plan *p, int dN, const float *d_sino, floa
     if (rc) return rc;
     std::string line;
     char b[512];
+    // the line counts a tiled plan's timed entries, three per subset step whichever kernels serve it
+    const long long entries = p->g.kernels == XCT_KERNELS_TILED ? (long long)per.size() : n[3];
     snprintf(b, sizeof b,
              "{\"call\": \"%s\", \"device\": %d, \"nx\": %d, \"ny\": %d, \"px\": %d, \"pa\": %d, "
              "\"ss\": %d, \"it\": %d, \"dN\": %d, \"kernels\": \"%s\", \"fwd_tile\": %d, \"ang_chunk\": %d, "
@@ -486,7 +488,7 @@ static int osem_loop_maybe_traced(xct_plan *p, int dN, const float *d_sino, floa
              "\"launches\": %lld, \"slice_iters_per_s\": %.4f, \"subset_ms\": [",
              call, p->ctx->device, p->g.nx, p->g.ny, p->g.px, p->g.pa, p->g.ss, it, dN,
              p->g.kernels == XCT_KERNELS_TILED ? "tiled" : "plain", p->kg.fwd_T, p->kg.fwd_chunk, ms[0], ms[1], ms[2],
-             ms[3], n[3], ms[3] > 0.0f ? dN * it / (ms[3] * 1e-3) : 0.0);
+             ms[3], entries, ms[3] > 0.0f ? dN * it / (ms[3] * 1e-3) : 0.0);
     line = b;
     for (size_t j = 0; j + 2 < per.size(); j += 3) {
         snprintf(b, sizeof b, "%s[%.4f, %.4f, %.4f]", j ? ", " : "", per[j], per[j + 1], per[j + 2]);
@@ -707,7 +709,8 @@ int xct_adj(xct_plan *p, int dN, const float *d_sino, float *d_img, void *stream
 
 // OS-EM of the plan's tiled or plain kernels with a CUDA event pair around every launch
 // (forward, finalize, backprojection per subset); synchronous.  per_launch receives each
-// launch's milliseconds in launch order (the plain kernels' finalize slot stays 0).
+// launch's milliseconds in launch order (a finalize slot without a launch -- the plain kernels', and where the
+// small-problem forward kernel forms the ratio itself -- stays 0).
 static int osem_loop_timed(xct_plan *p, int dN, const float *d_sino, float *d_img, const int *so, int it,
                            cudaStream_t st, float *ms, long long *launches, std::vector<float> *per_launch)
 {
@@ -722,6 +725,7 @@ static int osem_loop_timed(xct_plan *p, int dN, const float *d_sino, float *d_im
             return xct_fail(XCT_E_CUDA, "osem timing: event create");
         }
     int rc = XCT_OK, q = 0;
+    std::vector<char> none(nlaunch, 0);  // slots without a launch
     cudaEventRecord(ev[ev.size() - 2], st);
     for (int i = 0; i < it && rc == 0; ++i)
         for (int k = 0; k < p->g.ss && rc == 0; ++k) {
@@ -729,7 +733,12 @@ static int osem_loop_timed(xct_plan *p, int dN, const float *d_sino, float *d_im
             const int rows = subset_rows(p, s);
             for (int kind = 0; kind < nk && rc == 0; ++kind) {
                 cudaEventRecord(ev[2 * q], st);
-                if (tiled) {
+                const bool direct = tiled && fwd_is_direct(p->kg, dN, rows);
+                if (kind == 1 && (!tiled || direct)) {
+                    none[q] = 1;
+                } else if (kind == 0 && direct) {
+                    rc = launch_fwd_direct(p->kg, p->d_trig, d_img, d_sino, p->d_ratio, dN, s, p->g.ss, rows, st);
+                } else if (tiled) {
                     if (kind == 0) rc = launch_fwd_tiled_main(p->kg, p->d_trig, d_img, p->d_acc, dN, s, p->g.ss, rows, st);
                     else if (kind == 1)
                         rc = launch_fwd_finalize(p->kg, d_sino, p->d_ratio, p->d_acc, dN, s, p->g.ss, rows, st);
@@ -737,7 +746,7 @@ static int osem_loop_timed(xct_plan *p, int dN, const float *d_sino, float *d_im
                 } else {
                     if (kind == 0)
                         rc = launch_fwd_plain(p->kg, p->d_trig, d_img, d_sino, p->d_ratio, dN, s, p->g.ss, rows, st);
-                    else if (kind == 2) rc = launch_bp_update_plain(p->kg, p->d_trig, d_img, p->d_ratio, dN, s, st);
+                    else rc = launch_bp_update_plain(p->kg, p->d_trig, d_img, p->d_ratio, dN, s, st);
                 }
                 cudaEventRecord(ev[2 * q + 1], st);
                 ++q;
@@ -754,10 +763,11 @@ static int osem_loop_timed(xct_plan *p, int dN, const float *d_sino, float *d_im
         if (per_launch) per_launch->assign(q, 0.0f);
         for (int j = 0; j < q; ++j) {
             float t = 0.0f;
+            if (none[j]) continue;
             cudaEventElapsedTime(&t, ev[2 * j], ev[2 * j + 1]);
             ms[j % nk] += t;
             if (per_launch) (*per_launch)[j] = t;
-            if (tiled || j % nk != 1) launches[j % nk] += 1;
+            launches[j % nk] += 1;
         }
         cudaEventElapsedTime(&ms[3], ev[ev.size() - 2], ev[ev.size() - 1]);
         launches[3] = launches[0] + launches[1] + launches[2];

@@ -384,14 +384,17 @@ int xct_check_report(xct_ctx *ctx, long long *count, int *site, long long *index
 /* Tracing by environment: with XCT_TRACE set to a file name (or 1 for stderr) when the
  * library is first used, every xct_osem_run_device / xct_osem_run call of a plan without a
  * sinogram correction runs with CUDA events around each launch, synchronously, and appends
- * one JSON line: shape, dN, iterations, summed milliseconds and launch counts per kernel kind,
- * and [forward, finalize, backprojection] milliseconds per subset step.
+ * one JSON line: shape, dN, iterations, summed milliseconds per kernel kind, the timed entries
+ * ("launches"; three per subset step with the tiled kernels), the plan's xct_plan_tuning, and
+ * [forward, finalize, backprojection] milliseconds per subset step.  A finalize entry is 0 where the
+ * forward kernel forms the ratio (small problems and the plain kernels).
  *
  * Tracing by call: xct_osem_run_device with CUDA events around every launch.  The reference
  * enables CL_QUEUE_PROFILING_ENABLE but never reads the events
  * (share source/OCL_platform_device_class.cpp:175-178).  ms[0..3] = summed device time of
- * the forward-projection launches, of the ratio/finalize launches, of the
- * backprojection launches, and of the whole loop; launches[0..3] = their counts.
+ * the forward-projection launches, of the ratio/finalize launches (none where the forward kernel
+ * forms the ratio), of the backprojection launches, and of the whole loop; launches[0..3] = their
+ * counts, a step's launches of one kind over several slice groups as one.
  * Synchronous. */
 int xct_osem_profile(xct_plan *plan, int dN, const float *d_sino, float *d_img, const int *sub, int it,
                      void *stream, float *ms, long long *launches);
