@@ -63,15 +63,15 @@ __device__ __forceinline__ float cs_select(const float *v, int nx, int ny, int d
 
 // The proximal step alone (x_new from v; First: ISTA3D's floor of 1e-6 and NaN -> 1e-6), for the
 // compressed-sensing OS-EM, whose momentum image and beta never reach an output (FISTA_OSEM_execution
-// feeds its own w back as x_t, GPU.cpp:243-405, and reads neither).  grid: (ceil(nx/32), ceil(ny/8), dN),
-// 256 threads.  The neighbours go through a 12-exchange sorting network; where one of the six or their sum
+// feeds its own w back as x_t, GPU.cpp:243-405, and reads neither).  grid: (ceil(nx/32), ceil(ny/8), slices
+// from z0 on), 256 threads.  The neighbours go through a 12-exchange sorting network; where one of the six or their sum
 // is not finite, through the reference's exchange loop, whose order among NaNs it keeps.  HBM- or L2-bound:
 // 10 slices of 512^2 take 6 us (the general FISTA3D kernel and the copy of its result back took 32).
 template <bool First>
-__global__ void __launch_bounds__(256) prox_kernel(const float *v, float *x_new, int nx, int ny, int dN, float lambda)
+__global__ void __launch_bounds__(256) prox_kernel(const float *v, float *x_new, int nx, int ny, int dN, int z0, float lambda)
 {
     const int X = (int)blockIdx.x * 32 + (int)(threadIdx.x & 31), Y = (int)blockIdx.y * 8 + (int)(threadIdx.x >> 5);
-    const int Z = blockIdx.z;
+    const int Z = z0 + (int)blockIdx.z;
     xct_grid_wait();
     xct_grid_trigger();
     if (X >= nx || Y >= ny) return;
@@ -231,10 +231,13 @@ int launch_ista3d(const float *v, float *x_new, int nx, int ny, int dN, float la
 
 int launch_prox(const float *v, float *x_new, int nx, int ny, int dN, float lambda, bool first, cudaStream_t st)
 {
-    const dim3 grid((nx + 31) / 32, (ny + 7) / 8, dN);
-    if (dN > 65535) return xct_fail(XCT_E_INVALID, "compressed sensing: too many slices in one call");
-    return first ? xct_launch(prox_kernel<true>, grid, 256, 0, st, v, x_new, nx, ny, dN, lambda)
-                 : xct_launch(prox_kernel<false>, grid, 256, 0, st, v, x_new, nx, ny, dN, lambda);
+    int rc = XCT_OK;
+    for (int z = 0; z < dN && !rc; z += kMaxGridZ) {
+        const dim3 grid((nx + 31) / 32, (ny + 7) / 8, std::min(dN - z, kMaxGridZ));
+        rc = first ? xct_launch(prox_kernel<true>, grid, 256, 0, st, v, x_new, nx, ny, dN, z, lambda)
+                   : xct_launch(prox_kernel<false>, grid, 256, 0, st, v, x_new, nx, ny, dN, z, lambda);
+    }
+    return rc;
 }
 
 int launch_fista3d(const float *x_in, float *w, const float *v, float *beta, float *x_new, int nx, int ny, int dN,

@@ -143,12 +143,12 @@ static bool by_hand(const KGeom &g) { return g.fwd_hand || g.ms_hand; }
 
 bool fwd_is_direct(const KGeom &g, int dN, int nrows)
 {
-    return !by_hand(g) && (long long)g.nx * g.ny * nrows * dN <= kDirectTaps && nrows <= 65535 && dN <= 65535;
+    return !by_hand(g) && (long long)g.nx * g.ny * nrows * dN <= kDirectTaps && nrows <= 65535 && dN <= kMaxGridZ;
 }
 
 bool bp_is_direct(const KGeom &g, int dN)
 {
-    return !by_hand(g) && (long long)g.nx * g.ny * dN <= kDirectPixels && dN <= 65535;
+    return !by_hand(g) && (long long)g.nx * g.ny * dN <= kDirectPixels && dN <= kMaxGridZ;
 }
 
 int launch_fwd_direct(const KGeom &g, const float2 *trig, const float *img, const float *meas, float *out, int dN, int sub,

@@ -145,6 +145,9 @@ struct xct_plan {
     float last_ms = 0.0f;
 };
 
+// Most slices (groups) of one launch: a grid's third extent.  More go in several launches.
+constexpr int kMaxGridZ = 65535;
+
 // ---- error handling (per-thread last error) ----
 int xct_fail(int code, const std::string &msg);
 int xct_cuda_fail(cudaError_t e, const char *what);

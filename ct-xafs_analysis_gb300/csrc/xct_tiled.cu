@@ -1183,11 +1183,20 @@ int launch_fwd_finalize(const KGeom &g, const float *meas, float *out, double *a
     if (nrows <= 0 || dN <= 0) return XCT_OK;
     const bool vec = g.px % 4 == 0 && g.fetch == XCT_FETCH_EXACT && (((uintptr_t)meas | (uintptr_t)out) & 15u) == 0 &&
                      ((uintptr_t)acc & 15u) == 0;
-    if (vec)
-        return xct_launch(fwd_finalize4_kernel, dim3((g.px / 4 + 255) / 256, nrows, dN), 256, 0, st, acc, meas, out, g, sub,
-                          step, nrows);
-    return xct_launch(fwd_finalize_kernel, dim3((g.px + 127) / 128, nrows, dN), 128, 0, st, acc, meas, out, g, sub, step,
-                      nrows);
+    int rc = XCT_OK;
+    for (int z = 0; z < dN && !rc; z += kMaxGridZ) {
+        const int n = std::min(dN - z, kMaxGridZ);
+        const size_t nprj = (size_t)g.pa * g.px;
+        double *a = acc + (size_t)z * nrows * g.px;
+        const float *m = meas != nullptr ? meas + z * nprj : nullptr;
+        float *o = out + z * nprj;
+        if (vec)
+            rc = xct_launch(fwd_finalize4_kernel, dim3((g.px / 4 + 255) / 256, nrows, n), 256, 0, st, a, m, o, g, sub, step,
+                            nrows);
+        else
+            rc = xct_launch(fwd_finalize_kernel, dim3((g.px + 127) / 128, nrows, n), 128, 0, st, a, m, o, g, sub, step, nrows);
+    }
+    return rc;
 }
 
 int launch_fwd_tiled(const KGeom &g, const float2 *trig, const float *img, const float *meas, float *out,
@@ -1228,11 +1237,15 @@ int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const
     const long long tiles = (long long)mtx * mty, fill = 4LL * device_sm_count();
     auto run = [&](auto sc, int groups) -> int {
         constexpr int S = decltype(sc)::value;
-        const int rc = xct_launch(bp_ms_kernel<S>, dim3(mtx * mty, 1, groups), kBpMsThreads, 0, st, img, ratio, trig, g, sub,
-                                  nang, mtx, (float)g.ss, (float)g.pa, vec);
-        img += (size_t)groups * S * g.nx * g.ny;
-        ratio += (size_t)groups * S * g.pa * g.px;
-        dN -= groups * S;
+        int rc = XCT_OK;
+        for (int n; groups > 0 && !rc; groups -= n) {
+            n = std::min(groups, kMaxGridZ);
+            rc = xct_launch(bp_ms_kernel<S>, dim3(mtx * mty, 1, n), kBpMsThreads, 0, st, img, ratio, trig, g, sub, nang, mtx,
+                            (float)g.ss, (float)g.pa, vec);
+            img += (size_t)n * S * g.nx * g.ny;
+            ratio += (size_t)n * S * g.pa * g.px;
+            dN -= n * S;
+        }
         return rc;
     };
     int rc = XCT_OK;
