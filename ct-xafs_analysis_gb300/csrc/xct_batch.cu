@@ -41,11 +41,12 @@ struct xct_batch_plan {
     XctBatchStep step;                // the launches of one subset step
     XctBatchSide side;
     int fwd_T = 92, fwd_chunk = 128;  // forward tiles of the single slices
-    bool tuned = false;               // ... from the autotuner or its cache
-    int tuned_runs = 0;               // ... and the large tiles were faster
+    bool tuned = false;               // `choice` is the autotuner's or its cache's, for the slices `tuned_for`
+    TuneChoice choice{92, 128, 0.0f};
+    std::vector<int> tuned_for;
+    std::vector<int> singles;         // the graph's single slices as laid out
     std::vector<int> bases;           // host copy of d_bases
     size_t n_acc = 0;
-    std::string key;                  // tune-cache key of the batch's shapes
     cudaStream_t cap = nullptr;       // capture stream
     cudaGraphExec_t exec = nullptr;
     size_t queue_bytes = 0;
@@ -239,15 +240,35 @@ static TuneChoice default_tiles(const xct_batch_plan *p, const Arrangement &a, c
     return c;
 }
 
+// Tune-cache key of a choice of forward tiles: the single slices it is for (their shapes, in order).
+static std::string singles_key(const xct_batch_plan *p, const std::vector<int> &singles)
+{
+    unsigned long long h = 1469598103934665603ull;  // FNV-1a over the shapes
+    for (int i : singles) {
+        const KGeom &g = p->host[i].g;
+        const int v[6] = {g.nx, g.ny, g.px, g.pa, p->host[i].cover ? 1 : 0, 0};
+        for (int q = 0; q < 6; ++q) {
+            h ^= (unsigned)v[q];
+            h *= 1099511628211ull;
+        }
+    }
+    char kb[96];
+    snprintf(kb, sizeof kb, "batch%d-%016llx", (int)singles.size(), h);
+    return xct_tune_key(p->ctx->name, 0, 0, 0, 0, p->ss, (int)singles.size()) + "|" + kb;
+}
+
 // The graph's slices `want` in descriptor order and the launches of a subset step: work units,
-// prefix sums (uploaded), grids; `tiles`: the single slices' (null: the tuned choice, else the default
-// rule).  A captured graph is dropped (the next run captures again).
+// prefix sums (uploaded), grids; `tiles`: the single slices' (null: the choice tuned for these very slices,
+// else their cached one, else the default rule).  A captured graph is dropped (the next run captures again).
 static int batch_layout(xct_batch_plan *p, const std::vector<int> &want, const TuneChoice *tiles)
 {
     const Arrangement a = arrange(p, want);
-    const TuneChoice c = tiles ? *tiles
-                         : p->tuned ? TuneChoice{p->fwd_T, p->fwd_chunk, 0.0f, 0, p->tuned_runs}
-                                    : default_tiles(p, a, want);
+    if (tiles == nullptr && !(p->tuned && p->tuned_for == a.list[2])) {
+        p->tuned = !a.list[2].empty() && xct_tune_lookup(singles_key(p, a.list[2]), xct_tune_env_path(), p->choice);
+        p->tuned_for = a.list[2];
+    }
+    const TuneChoice c = tiles ? *tiles : p->tuned ? p->choice : default_tiles(p, a, want);
+    p->singles = a.list[2];
     const int T = c.T, chunk = c.chunk;
     const int big = c.runs ? large_chunk(p, a.list[2]) : 0;
     const std::vector<int> *list = a.list;
@@ -355,23 +376,6 @@ static std::vector<int> all_items(int n)
     std::vector<int> v(n);
     for (int i = 0; i < n; ++i) v[i] = i;
     return v;
-}
-
-// Tune-cache key of the graph's slices (their shapes, in order).
-static std::string graph_key(const xct_batch_plan *p)
-{
-    unsigned long long h = 1469598103934665603ull;  // FNV-1a over the shapes
-    for (int i : p->want) {
-        const KGeom &g = p->host[i].g;
-        const int v[6] = {g.nx, g.ny, g.px, g.pa, p->host[i].cover ? 1 : 0, 0};
-        for (int q = 0; q < 6; ++q) {
-            h ^= (unsigned)v[q];
-            h *= 1099511628211ull;
-        }
-    }
-    char kb[96];
-    snprintf(kb, sizeof kb, "batch%d-%016llx", (int)p->want.size(), h);
-    return xct_tune_key(p->ctx->name, 0, 0, 0, 0, p->ss, (int)p->want.size()) + "|" + kb;
 }
 
 extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms, int it, xct_batch_plan **out)
@@ -551,14 +555,9 @@ extern "C" int xct_batch_plan_create(xct_ctx *ctx, int n, const xct_geom *geoms,
     if (scratch > 0 && (e = cudaMalloc(&p->d_gscratch, sizeof(float) * scratch)) != cudaSuccess)
         return fail(e, "cudaMalloc group scratch");
     // the graph's slices with groups in use (every slice when all are grouped: the graph
-    // then serves them only with groups off), its tiles: this list's cached choice, else the
-    // default rule
+    // then serves them only with groups off)
     p->want = p->rest.empty() ? all_items(n) : p->rest;
-    p->key = graph_key(p);
-    TuneChoice c;
-    p->tuned = xct_tune_lookup(p->key, xct_tune_env_path(), c);
-    p->tuned_runs = c.runs;
-    int rc = batch_layout(p, std::vector<int>(p->want), p->tuned ? &c : nullptr);
+    int rc = batch_layout(p, std::vector<int>(p->want), nullptr);
     if (rc) {
         batch_free(p);
         return rc;
@@ -817,7 +816,7 @@ extern "C" int xct_batch_plan_tuning(xct_batch_plan *p, int *fwd_tile, int *ang_
 
 // Time the batched forward launch (subset 0) for every candidate (T, chunk) and keep the
 // fastest; the slices read one scratch image of the largest size (the cost depends on the
-// geometry only).  The choice is cached under the batch's shape key.
+// geometry only).  The choice is cached under the shapes of the slices it is for.
 extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path, int flags, void *stream)
 {
     XCT_RANGE("xct_batch_plan_autotune");
@@ -835,13 +834,16 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
         int rc = batch_layout(p, want, nullptr);
         if (rc) return rc;
     }
-    p->key = graph_key(p);
-    TuneChoice best;
-    if (!(flags & XCT_TUNE_FORCE) && xct_tune_lookup(p->key, cache_path, best)) {
+    if (p->singles.empty()) return XCT_OK;  // packs only: their tiles are fixed
+    const std::string key = singles_key(p, p->singles);
+    auto keep = [&](const TuneChoice &c) {
         p->tuned = true;
-        p->tuned_runs = best.runs;
-        return batch_layout(p, want, &best);
-    }
+        p->choice = c;
+        p->tuned_for = p->singles;
+        return batch_layout(p, want, nullptr);
+    };
+    TuneChoice best;
+    if (!(flags & XCT_TUNE_FORCE) && xct_tune_lookup(key, cache_path, best)) return keep(best);
     XCT_CUDA_TRY(cudaSetDevice(p->ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
     const int m = (int)p->glist.size();
@@ -862,11 +864,10 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
     best = before;
     int rc = cudaMemsetAsync(scratch, 0, sizeof(float) * maxpix, st) == cudaSuccess ? XCT_OK
                                                                                     : xct_fail(XCT_E_CUDA, "memset");
-    if (p->step.packs[2] == 0) best.ms = 0.0f;  // packs only: nothing to choose
     std::vector<TuneChoice> choices = xct_tune_candidates(max_rows);
     choices.push_back(TuneChoice{before.T, before.chunk, 0.0f, 0, 1});  // the large tiles
     for (const TuneChoice &c : choices) {
-        if (rc || p->step.packs[2] == 0) break;
+        if (rc) break;
         if ((rc = batch_layout(p, want, &c))) break;
         for (int j = 0; j < m; ++j) {
             tmp[j] = p->host[p->glist[j]];
@@ -898,9 +899,7 @@ extern "C" int xct_batch_plan_autotune(xct_batch_plan *p, const char *cache_path
         batch_layout(p, want, &before);
         return rc;
     }
-    p->tuned = true;
-    p->tuned_runs = best.runs;
-    rc = batch_layout(p, want, &best);
+    rc = keep(best);
     if (rc) return rc;
-    return xct_tune_store(p->key, cache_path, best);
+    return xct_tune_store(key, cache_path, best);
 }

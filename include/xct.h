@@ -411,9 +411,11 @@ int xct_osem_profile(xct_plan *plan, int dN, const float *d_sino, float *d_img, 
  * fastest, and records it in memory and in cache_path (NULL: XCT_TUNE_CACHE; no file if
  * neither).  A cached entry is reused without timing unless flags has XCT_TUNE_FORCE.
  * Synchronous.  xct_batch_plan_autotune does the same for a batch plan: each geometry
- * group's plan, and one choice for the slices its graph serves (the next xct_batch_run
+ * group's plan, and one choice for the slices its graph serves one by one (the next xct_batch_run
  * captures its graph again), the large tiles among its candidates; the tile reported is then the
- * best of the others.  The *_tuning calls report
+ * best of the others.  The choice is cached under those slices' shapes and holds for them alone: another
+ * setting of the grouping switch has its own, and where every slice is in a pack nothing is timed or
+ * stored.  The *_tuning calls report
  * the current choice; xct_plan_set_tuning sets one by hand, for the forward projection of every slice at
  * any size but of whole groups of eight with the slice-interleaved kernels on (below), until the autotuner
  * chooses again; the other kernels' grouping of slices stays as it is. */
