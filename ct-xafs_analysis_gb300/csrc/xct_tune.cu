@@ -272,7 +272,7 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = (p->g.pa + p->g.ss - 1) / p->g.ss;
     const int nrows = p->g.subset_mode == XCT_SUBSETS_COVER ? rows : p->g.pa / p->g.ss;
-    const size_t acc_bytes = sizeof(double) * (size_t)dN * p->acc_rows * p->g.px;
+    const size_t acc_bytes = sizeof(double) * (size_t)dN * p->acc_rows * p->g.px;  // (dN: at least what is timed)
     cudaEvent_t e0, e1;
     XCT_CUDA_TRY(cudaEventCreate(&e0));
     XCT_CUDA_TRY(cudaEventCreate(&e1));
@@ -295,13 +295,15 @@ int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, vo
         }
         return tmin;
     };
+    // the choice is the per-slice kernel's, which serves one slice, or any number with the grouping off
+    const int slices = saved.fwd_group ? 1 : dN;
     KGeom k = saved;
-    k.fwd_group = 0;  // the choice is the per-slice kernel's
+    k.fwd_group = 0;
     k.fwd_hand = 0;
     for (const TuneChoice &c : xct_tune_candidates(rows)) {
         k.fwd_T = c.T;
         k.fwd_chunk = c.chunk;
-        const float tmin = timed(k, dN);
+        const float tmin = timed(k, slices);
         if (rc) break;
         if (tmin < best.ms) best = TuneChoice{c.T, c.chunk, tmin};
     }

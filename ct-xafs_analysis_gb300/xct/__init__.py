@@ -551,8 +551,9 @@ class OSEMPlan:
 
     # ---- forward-projector tiles --------------------------------------------------------
     def autotune(self, dN=None, cache_path=None, force=False, stream=None):
-        """Time every (tile side, angles per CTA) candidate for dN slices and keep the fastest
-        (cached per shape in memory and in cache_path / $XCT_TUNE_CACHE)."""
+        """Time every (tile side, angles per CTA) candidate -- for one slice, or with the grouping off
+        (set_multislice(0)) for dN -- and keep the fastest (cached per shape and dN in memory and in
+        cache_path / $XCT_TUNE_CACHE)."""
         dN = self.max_batch if dN is None else dN
         cp = None if cache_path is None else str(cache_path).encode()
         _check(self._lib.xct_plan_autotune(self.handle, dN, cp, TUNE_FORCE if force else 0, _stream(stream)))

@@ -406,8 +406,9 @@ int xct_osem_profile(xct_plan *plan, int dN, const float *d_sino, float *d_img, 
  * (device name, nx, ny, px, pa, ss, max_batch) -- in this process, or in the JSON file named by
  * the environment variable XCT_TUNE_CACHE -- or else the tiles of least modelled time; a slice by
  * itself then goes through larger tiles in equal runs of (tile, angle) units, which the autotuner
- * times against its choice.  xct_plan_autotune times every candidate for dN slices on the plan's own
- * geometry (its staging buffers are the input; no caller data is read or written), keeps the
+ * times against its choice.  xct_plan_autotune times every candidate on the plan's own geometry, for one
+ * slice -- slices together go through the grouped forms, whose tiles are fixed -- or with the grouping off
+ * (xct_plan_set_multislice 0) for dN slices (its staging buffers are the input; no caller data is read or written), keeps the
  * fastest, and records it in memory and in cache_path (NULL: XCT_TUNE_CACHE; no file if
  * neither).  A cached entry is reused without timing unless flags has XCT_TUNE_FORCE.
  * Synchronous.  xct_batch_plan_autotune does the same for a batch plan: each geometry
