@@ -252,6 +252,15 @@ int xct_plan_set_multislice(xct_plan *p, int ang_chunk)
     return XCT_OK;
 }
 
+int xct_plan_reset_tuning(xct_plan *p)
+{
+    if (!p) return xct_fail(XCT_E_INVALID, "xct_plan_reset_tuning: plan is null");
+    p->kg.fwd_group = 1;
+    p->kg.fwd_hand = p->kg.ms_hand = 0;
+    xct_plan_default_tuning(p);
+    return XCT_OK;
+}
+
 int xct_plan_autotune(xct_plan *p, int dN, const char *cache_path, int flags, void *stream)
 {
     XCT_RANGE("xct_plan_autotune");

@@ -56,7 +56,7 @@ EXPORTS = (
     "xct_check_report", "xct_reslice_plan_create", "xct_reslice", "xct_reslice_plan_destroy", "xct_reslice_plan_set_wait_limit",
     "xct_denoise_sinogram",
     "xct_cs_osem_run_device", "xct_cs_osem_run", "xct_plan_autotune", "xct_plan_tuning", "xct_plan_set_tuning",
-    "xct_plan_multislice", "xct_plan_set_multislice", "xct_batch_plan_set_cs", "xct_batch_plan_uniform",
+    "xct_plan_multislice", "xct_plan_set_multislice", "xct_plan_reset_tuning", "xct_batch_plan_set_cs", "xct_batch_plan_uniform",
     "xct_batch_plan_groups", "xct_batch_plan_set_grouping",
     "xct_fista_power_iteration", "xct_fista_set_lipschitz", "xct_fista_run_device", "xct_fista_run",
     "xct_batch_plan_autotune", "xct_batch_plan_tuning", "xct_osem_run_volume", "xct_hybrid_cs_run_device",
@@ -165,6 +165,7 @@ def load():
     L.xct_plan_set_tuning.argtypes = [vp, ip, ip]
     L.xct_plan_multislice.argtypes = [vp, ctypes.POINTER(ctypes.c_int)]
     L.xct_plan_set_multislice.argtypes = [vp, ip]
+    L.xct_plan_reset_tuning.argtypes = [vp]
     L.xct_batch_plan_autotune.argtypes = [vp, ctypes.c_char_p, ip, vp]
     L.xct_batch_plan_tuning.argtypes = [vp, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
     L.xct_plan_sync.argtypes = [vp]
@@ -574,9 +575,13 @@ class OSEMPlan:
         return v.value
 
     def set_multislice(self, ang_chunk):
-        """Turn the slice-interleaved forward projector on (subset angles per CTA, 1..128) or
-        off (0) for calls of eight or more slices."""
+        """Turn the slice-interleaved kernels on (most subset angles per forward CTA, 1..128) or every
+        grouping of slices off (0), whatever the size."""
         _check(self._lib.xct_plan_set_multislice(self.handle, int(ang_chunk)))
+
+    def reset_tuning(self):
+        """Take back set_tuning and set_multislice: the plan's own choices again."""
+        _check(self._lib.xct_plan_reset_tuning(self.handle))
 
     def profile(self, d_sino, d_img, dN=None, sub=None, it=-1, stream=None):
         """Run OS-EM with CUDA events around every launch; returns a dict of summed device

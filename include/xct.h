@@ -450,10 +450,15 @@ int xct_batch_plan_tuning(xct_batch_plan *plan, int *fwd_tile, int *ang_chunk);
  * value is the most subset angles a forward CTA serves from one staging of a tile (1..128); 0
  * turns all three off.  Plans start on (128) when max_batch >= 8 and the forward tiles of one group give at
  * least two CTAs per SM, else off (the tile cache and the autotuner leave this switch
- * alone). */
+ * alone).
+ *
+ * A plan that starts with it off still groups up to five slices and, small problems, takes the kernels
+ * made for them; a value set by hand holds whatever the size.  xct_plan_reset_tuning takes back what
+ * xct_plan_set_tuning and xct_plan_set_multislice set: the plan is as it was created. */
 #define XCT_MULTISLICE_SLICES 8
 int xct_plan_multislice(xct_plan *plan, int *ang_chunk);
 int xct_plan_set_multislice(xct_plan *plan, int ang_chunk);
+int xct_plan_reset_tuning(xct_plan *plan);
 
 /* FP32 FMA throughput of a device (TFLOP/s), measured by a dependent-chain-free FMA
  * kernel: the roofline denominator for the projectors. */
