@@ -1229,9 +1229,11 @@ int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const
     if (dN <= 0) return XCT_OK;
     if (bp_is_direct(g, dN)) return launch_bp_update_direct(g, trig, img, ratio, dN, sub, st);
     const int nang = (g.pa - sub + g.ss - 1) / g.ss;  // OSEM2's angle loop (OSEM.cl:93)
-    // With the slice-interleaved kernels on, whole groups of eight slices go through the eight-slice form;
-    // the rest (with grouping on) in fours, pairs and singles -- the larger forms cost less per slice, but
-    // only where their grid still gives every SM four CTAs.
+    // Slices go in eights (with the slice-interleaved kernels on), fours and pairs (with grouping on), the rest one by
+    // one -- the larger forms cost less per slice, but only where their grid still gives every SM four CTAs: a subset
+    // step of 16 slices of 512^2 x 48 angles, in two halves of 256 tiles, takes 194 us in eights and 159 in pairs;
+    // of 768^2 (576 tiles) 322 in eights, 315 in fours; of 1024^2 (1024) 542 and 540.  Eights set by hand hold
+    // whatever the size.
     const int mtx = (g.nx + kBpMsT - 1) / kBpMsT, mty = (g.ny + kBpMsT - 1) / kBpMsT;
     const int vec = g.px % 4 == 0 && ((uintptr_t)ratio & 15u) == 0;
     const long long tiles = (long long)mtx * mty, fill = 4LL * device_sm_count();
@@ -1249,7 +1251,8 @@ int launch_bp_update_tiled(const KGeom &g, const float2 *trig, float *img, const
         return rc;
     };
     int rc = XCT_OK;
-    if (g.ms_chunk > 0 && dN >= kMsSlices) rc = run(std::integral_constant<int, 8>{}, dN / kMsSlices);
+    if (g.ms_chunk > 0 && dN >= kMsSlices && (g.ms_hand || tiles * (dN / kMsSlices) >= fill))
+        rc = run(std::integral_constant<int, 8>{}, dN / kMsSlices);
     if (!rc && g.fwd_group && dN >= 4 && tiles * (dN / 4) >= fill) rc = run(std::integral_constant<int, 4>{}, dN / 4);
     if (!rc && g.fwd_group && dN >= 2 && tiles * (dN / 2) >= fill) rc = run(std::integral_constant<int, 2>{}, dN / 2);
     if (!rc && dN >= 1) rc = run(std::integral_constant<int, 1>{}, dN);
