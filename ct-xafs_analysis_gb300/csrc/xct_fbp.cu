@@ -264,7 +264,9 @@ __global__ void __launch_bounds__(kFbpMsThreads) fbp_bp_ms_kernel(const float *_
     const int z0 = (int)blockIdx.z * S;
     const size_t nprj = (size_t)g.pa * g.px, nimg = (size_t)g.nx * g.ny;
     const float *rz = fprj + (size_t)z0 * nprj;
-    const int bx = (int)blockIdx.x % ntx, by = (int)blockIdx.x / ntx;
+    // rows of tiles from the middle outwards: the last CTAs to start are the rows whose corners have nothing to do
+    const int row = (int)blockIdx.x / ntx, mid = ((int)gridDim.x / ntx - 1) / 2;
+    const int bx = (int)blockIdx.x - row * ntx, by = row & 1 ? mid + (row + 1) / 2 : mid - row / 2;
     const int X0 = bx * kFbpMsT, Y0 = by * kFbpMsT;
     const int X1 = min(X0 + kFbpMsT, g.nx) - 1, Y1 = min(Y0 + kFbpMsT, g.ny) - 1;
     const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
@@ -490,9 +492,25 @@ int launch_fbp_bp(const KGeom &g, const float2 *trig, const float *fprj, float *
         cudaError_t e = cudaMemsetAsync(min_keys, 0x7F, sizeof(int) * dN, st);  // key of a huge float
         if (e != cudaSuccess) return xct_cuda_fail(e, "fbp min reset");
     }
-    // with the slice-interleaved kernels on, groups of eight slices go through the eight-slice form; the
-    // rest (with grouping on) in pairs, and a last single slice alone
+    // Slices go in groups of eight (with the slice-interleaved kernels on), pairs (with grouping on) and singles, as
+    // the modelled time of the launches, one after the other, is least: us an angle of a launch whose SMs get m CTAs
+    // each, a + c m (fits of 64^2 to 2048^2).  The larger forms take less per slice and more per CTA, and each further
+    // launch another a: three slices of 400^2 x 200 angles 69 us as singles and 89 as a pair and one, of 1024^2 x 512
+    // 668 and 578.  Eights set by hand hold whatever the size.
     const int mtx = (g.nx + kFbpMsT - 1) / kFbpMsT, mty = (g.ny + kFbpMsT - 1) / kFbpMsT;
+    const long long tiles = (long long)mtx * mty;
+    const int sms = device_sm_count();
+    auto time = [&](double a, double c, int groups) { return groups > 0 ? a + c * (double)((tiles * groups + sms - 1) / sms) : 0.0; };
+    int eights = 0, pairs = 0;
+    double least = INFINITY;
+    for (int e = 0; e <= (g.ms_chunk > 0 ? dN / kFbpMsSlices : 0); e += std::max(1, dN / kFbpMsSlices)) {
+        if (e == 0 && g.ms_hand && g.ms_chunk > 0 && dN >= kFbpMsSlices) continue;
+        for (int two = 0; two <= (g.fwd_group ? 1 : 0); ++two) {
+            const int rest = dN - e * kFbpMsSlices, p = two ? rest / 2 : 0;
+            const double t = time(0.2, 0.25, e) + time(0.095, 0.085, p) + time(0.07, 0.062, rest - 2 * p);
+            if (t < least) least = t, eights = e, pairs = p;
+        }
+    }
     auto run = [&](auto sc, int groups) -> int {
         constexpr int S = decltype(sc)::value;
         if (groups <= 0) return XCT_OK;
@@ -506,9 +524,8 @@ int launch_fbp_bp(const KGeom &g, const float2 *trig, const float *fprj, float *
         dN -= groups * S;
         return XCT_OK;
     };
-    int rc = XCT_OK;
-    if (g.ms_chunk > 0) rc = run(std::integral_constant<int, kFbpMsSlices>{}, dN / kFbpMsSlices);
-    if (!rc && g.fwd_group) rc = run(std::integral_constant<int, 2>{}, dN / 2);
+    int rc = run(std::integral_constant<int, kFbpMsSlices>{}, eights);
+    if (!rc) rc = run(std::integral_constant<int, 2>{}, pairs);
     if (!rc) rc = run(std::integral_constant<int, 1>{}, dN);
     return rc;
 }
