@@ -669,13 +669,14 @@ int launch_adj_subset(const KGeom &g, const float2 *trig, const float *sino, flo
                                  {2, 32, launch_adj_scatter<2, 32>}, {1, 64, launch_adj_scatter<1, 64>},
                                  {1, 44, launch_adj_scatter<1, 44>}, {1, 32, launch_adj_scatter<1, 32>},
                                  {1, 16, launch_adj_scatter<1, 16>}};
+    const int sms = device_sm_count();
     while (dN > 0) {
         const Form *best = nullptr;
         double cost = 0.0;
         for (const Form &f : forms) {
             if (f.S > dN || (f.S > 1 && !g.fwd_group)) continue;
             const int groups = dN / f.S;
-            const double c = adj_cost(g.nx, g.ny, f.S, f.T, groups, device_sm_count()) / (groups * f.S);
+            const double c = adj_cost(g.nx, g.ny, f.S, f.T, groups, sms) / (groups * f.S);
             if (!best || c < cost) {
                 best = &f;
                 cost = c;
