@@ -214,10 +214,10 @@ static int large_chunk(const xct_batch_plan *p, const std::vector<int> &singles)
 }
 
 // Forward tiles of the single slices when nothing was tuned (of every slice when all are packed).  The large
-// tiles serve them where every SM has at least 32 (tile, angle) units of them to do: one iteration of 12 slices
-// 512 to 2048 wide (500 units) 20.4 ms against 22.3, of five 722 to 1444 wide 3.81 against 4.45, of 21 slices of
-// which 7 single ones 570 to 1140 wide (60 units) 8.33 against 8.70; but of 30 with 10 single ones 327 to 654 wide
-// (25 units) 2.24 against 2.20, and of 8 slices 150 to 300 wide (2 units) 0.69 against 0.61.
+// tiles serve them but where an SM gets less than a quarter of a (tile, angle) unit, which is latency either way:
+// over 57 random stacks with single slices 40 to 1400 wide they took 0.68 to 1.07 of the others' time above that line
+// (an iteration of 12 slices 512 to 2048 wide 19.8 ms against 22.1, of five 722 to 1444 4.38 against 5.19, of
+// eight 150 to 300 0.33 against 0.43) and 1.02 to 1.12 below it (three 71 to 142 wide, 0.1 units: 194 us, 173).
 static TuneChoice default_tiles(const xct_batch_plan *p, const Arrangement &a, const std::vector<int> &want)
 {
     const std::vector<int> &of = a.list[2].empty() ? want : a.list[2];
@@ -236,7 +236,7 @@ static TuneChoice default_tiles(const xct_batch_plan *p, const Arrangement &a, c
         const KGeom &g = p->host[i].g;
         units += (g.nx + 1.0) * (g.ny + 1.0) / (T * T) * (g.pa / g.ss);
     }
-    c.runs = units >= 32.0 * p->ctx->sm_count;
+    c.runs = units >= 0.25 * p->ctx->sm_count;
     return c;
 }
 
