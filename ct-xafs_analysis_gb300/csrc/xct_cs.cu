@@ -65,8 +65,9 @@ __device__ __forceinline__ float cs_select(const float *v, int nx, int ny, int d
 // compressed-sensing OS-EM, whose momentum image and beta never reach an output (FISTA_OSEM_execution
 // feeds its own w back as x_t, GPU.cpp:243-405, and reads neither).  grid: (ceil(nx/32), ceil(ny/8), slices
 // from z0 on), 256 threads.  The neighbours go through a 12-exchange sorting network; where one of the six or their sum
-// is not finite, through the reference's exchange loop, whose order among NaNs it keeps.  HBM- or L2-bound:
-// 10 slices of 512^2 take 6 us (the general FISTA3D kernel and the copy of its result back took 32).
+// is not finite, through the reference's exchange loop, whose order among NaNs it keeps.  Bound by its
+// loads: 10 slices of 512^2 take 15 us from a cold cache (3.1 at the HBM rate; the general FISTA3D kernel and the
+// copy of its result back took 32).
 template <bool First>
 __global__ void __launch_bounds__(256) prox_kernel(const float *v, float *x_new, int nx, int ny, int dN, int z0, float lambda)
 {

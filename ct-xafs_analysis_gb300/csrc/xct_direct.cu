@@ -9,8 +9,8 @@
 //   * bp_direct_kernel: a thread owns one pixel of up to two slices and gathers its bins, in angle
 //     order with the literal bin expression, so the image is the tiled kernel's bit for bit.
 // Both are bound by latency at these sizes: a 256 x 256 slice with 18 angles per subset is 1.2 M
-// samples, 8 per lane with every SM filled.  A subset step of it takes 10.8 us (the two launches
-// overlap by programmatic stream serialization) against 37.4 us with the tiled kernels' three.
+// samples, 8 per lane with every SM filled.  A subset step of it takes 10.4 us (the two launches
+// overlap by programmatic stream serialization); 12.0 with the tiled forward kernel and its finalize (below).
 #include "xct_device.cuh"
 #include "xct_launch.cuh"
 #include "xct_ray.cuh"

@@ -3,9 +3,9 @@
 // Replaces, for CT_reconstruction:
 //   FBP_execution (GPU.cpp:665-819) over the kernels of FBP.cl:
 //     spinFactor .. outputImage (FBP.cl:34-160)  -> fbp_filter_kernel (one launch)
-//     backProjectionFBP (FBP.cl:164-188)          -> fbp_bp_kernel
+//     backProjectionFBP (FBP.cl:164-188)          -> fbp_bp_ms_kernel
 //   hybrid_thread's base-up (GPU.cpp:1538-1566):
-//     findMinimumX/findMinimumY (reconstShare.cl:111-177) -> folded into fbp_bp_kernel
+//     findMinimumX/findMinimumY (reconstShare.cl:111-177) -> folded into fbp_bp_ms_kernel
 //     baseUp (reconstShare.cl:87-109)                     -> base_up_kernel
 //
 // Ramp filter.  The reference zero-pads each sinogram row to ZP_SIZE bins, runs a radix-2
@@ -220,9 +220,9 @@ __device__ __forceinline__ float fkey_decode(int k) { return __int_as_float(k >=
 // A warp whose 32 x 4 pixels all lie outside the field of view (their values are 0 whatever the
 // projections) skips its gathers: 20 % of a square image.
 //
-// Bound: the FP32 pipe for one slice (12 operations a lerp that the reference's rounding fixes), the
-// shared-memory data path for eight (8 B per lerp and slice).  One 2048^2 slice, 1500 angles: 2.51 ms with
-// that pipe 72 % busy (2.88 with 64 x 64 tiles that covered the whole square).
+// Bound: the FP32 pipe for one slice (13 operations a lerp that the reference's rounding fixes), the
+// shared-memory data path for eight (8 B per lerp and slice).  One 2048^2 slice, 1500 angles: 2.49 ms (2.51 with
+// that pipe 72 % busy, rows of tiles from the top down; 2.88 with 64 x 64 tiles that covered the whole square).
 constexpr int kFbpMsT = 32, kFbpMsThreads = 256, kFbpMsW = 52, kFbpMsPix = 4, kFbpMsSlices = 8;
 
 template <int S>

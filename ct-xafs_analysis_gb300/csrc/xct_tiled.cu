@@ -7,7 +7,8 @@
 //     reaches texel 0).  It stages the tile once in shared memory as (t, t[x+1] - t) pairs, so
 //     the x-lerp of a bilinear sample is one FMA and its 2x2 footprint is two 64-bit
 //     loads, and serves its angles from there; a run of (tile, angle) units of equal modelled time per
-//     CTA, so that the grid is one wave whatever the image's size and the angle count;
+//     CTA, so that the grid is one wave (slices of up to 4096 tiles; more, tiles set by hand and the batch
+//     plans take a CTA per tile and chunk of angles);
 //   * a warp takes one angle and 8 consecutive rays, 4 lanes per ray; the exact interval of
 //     sample indices Y whose base texel lies in the tile (the coordinates are monotone in Y)
 //     comes from four boundary searches, one per lane of the ray's group; the 4 lanes then
@@ -676,9 +677,8 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
 // there is no waiting on other CTAs.
 // A pack pays per slice what the forward and backward kernels of several slices save (coordinates,
 // addresses and weights once), and takes the large tiles, one CTA per SM: one iteration of 24 slices, 12
-// geometries 512 to 2048 wide, takes 27.8 ms in packs of two and 43.3 one by one (29.3 with tiles of two CTAs per
-// SM); 21 of seven geometries 570 to 1140 wide, in packs of two and single slices, 8.7 ms (9.3); 6 of
-// three, 200 to 400 wide, 0.33 with either.
+// geometries 512 to 2048 wide, takes 27.8 ms in packs of two and 39.1 one by one; 21 of seven geometries 570 to
+// 1140 wide, in packs of two and single slices, 8.05 ms and 9.65; 6 of three, 200 to 400 wide, 0.33 and 0.44.
 __device__ __forceinline__ int queue_take(int *queue, int *s_unit)
 {
     if (threadIdx.x == 0) *s_unit = atomicAdd(queue, 1);
@@ -963,17 +963,17 @@ static void fwd_split_chunks(const KGeom &g, int T, int nrows, int chunk, int gr
     f.cap = chunk;
 }
 
-// Before runs, a CTA took a tile and a chunk of angles, and the last wave of CTAs was nearly empty at many
-// sizes (three slices of 509 x 487: 64 tiles x 5 chunks on 304 places).  A subset step then and now, with the
-// large tiles: one slice of 2048^2 x 100 angles 464 / 419 us, of 512^2 x 36 28.5 / 25.5; three of 509 x 487 x 31
-// 45.7 / 39.2; ten of 512^2 x 36 107 / 93.
-//
 // Runs of equal modelled time for `blocks` CTAs per SM, on tiles as equal as T allows; returns that time (SM
 // cycles; 0: more units than start[] can count).  A full tile and angle take `angle` cycles of an SM, the
 // staging of a tile `stage`.  The work of a tile whose centre is further from the axis than half the detector
 // is scaled by the share of half a turn in which that centre is projected onto it (a 2048^2 slice on 2048
 // bins: 0.5 in the corners; with equal runs instead, corner CTAs finished early and the launch took 6 %
 // longer).  A run takes the rest of its tile where another staging would cost more than that rest.
+//
+// Against a CTA per tile and chunk of angles, whose last wave is nearly empty at many sizes (three slices of
+// 509 x 487: 64 tiles x 5 chunks on 304 places), a subset step takes, chunks / runs, with the large tiles: one slice
+// of 2048^2 x 100 angles 464 / 419 us, of 512^2 x 36 28.5 / 25.5; three of 509 x 487 x 31 45.7 / 39.2; ten of 512^2 x
+// 36 107 / 93.
 static double fwd_split_runs(const KGeom &g, int T, int blocks, double angle, double stage, int nrows, int groups,
                              FwdSplit &f)
 {

@@ -1,15 +1,15 @@
 // xct_tune.cu -- the forward projector's tile autotuner and its cache.
 //
 // The forward projector divides a launch into runs of (tile, angle) units by itself; a slice alone (or every slice,
-// with grouping off) can instead take a CTA per tile and chunk of angles, which has two launch-shape parameters: the tile side T (44, 60, 76 or
-// 92 base texels; a CTA stages one tile and serves its angles from shared memory) and the
+// with grouping off) can instead take a CTA per tile and chunk of angles, which has two launch-shape
+// parameters: the tile side T (44, 60, 76 or 92 base texels; a CTA stages one tile and serves its angles from shared memory) and the
 // number of subset angles one CTA serves (the chunk, 16..128).  Large values amortise the
 // staging and the per-ray interval search; small values give more CTAs, which small slices
 // and small subsets need to fill 152 SMs.  Four CTAs (48 warps) fit on an SM for T <= 76 and
 // three (36 warps) for T = 92, so the choice changes the occupancy, the grid's granularity and
-// the per-tile overheads -- a trade-off that depends on the slice size, the angles per subset
-// and the slices per call, so it is measured: xct_plan_autotune times every candidate on the plan's
-// own geometry, keeps the fastest and times the runs against it; the choice is cached per (device, shape) in memory and,
+// the per-tile overheads -- a trade-off that depends on the slice size and the angles per subset,
+// so it is measured: xct_plan_autotune times every candidate on the plan's own geometry, for the
+// slices that the choice serves, keeps the fastest and times the runs against it; the choice is cached per (device, shape) in memory and,
 // optionally, in a JSON file that later plans (and processes) read.
 #include <stdio.h>
 #include <stdlib.h>
@@ -162,10 +162,10 @@ const char *xct_tune_env_path()
 }
 
 // ---------------------------------------------------------------- single-shape plans
-// The slice-interleaved forward projector by default: on (all subset angles per CTA) when a
-// plan's full batch holds a group of eight slices whose tiles give at least two waves of
-// CTAs (one per SM); smaller problems keep the per-slice kernel, whose smaller CTAs fill
-// the SMs better.
+// The slice-interleaved kernels' switch by default: on when a plan's full batch holds a group of eight slices of
+// at least 304 (two for every SM) squares of 42 texels.  It admits groups of eight in the backprojectors, which
+// check for themselves whether the grid fills the SMs, and cuts a call's halves at multiples of eight; the
+// forward projector takes its groups of up to five slices either way.
 static int plan_default_ms_chunk(const xct_plan *p)
 {
     const int G = fwd_ms_slices(), T = 42;
@@ -201,8 +201,7 @@ void xct_plan_default_tuning(xct_plan *p)
     const bool cached = xct_tune_lookup(key, xct_tune_env_path(), c);
     if (!cached) c = plan_default_tiles(p);
     p->kg.fwd_tuned = cached && !c.runs;
-    // the cache holds the per-slice kernel's tiles; the slice-interleaved kernels' switch
-    // follows the plan's shape
+    // the cache holds one slice's tiles; the slice-interleaved kernels' switch follows the plan's shape
     c.ms_chunk = plan_default_ms_chunk(p);
     p->kg.fwd_T = c.T;
     p->kg.fwd_chunk = c.chunk;

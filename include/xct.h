@@ -117,8 +117,8 @@ int xct_osem_run_volume(xct_plan *plan, int n, const float *const *sino_host, fl
  * The reference reconstructs dN slices of ONE shape per OSEM_execution call
  * (GPU.cpp:125-240, image2d_array layers).  A batch plan takes n slices of any shapes
  * (each its own xct_geom: size, bins, angle list, centre, modes) that share the subset
- * count; every subset step is three persistent launches whose CTAs take (slice, tile) work
- * units from a device queue, and the whole subset/iteration loop is one CUDA graph,
+ * count; every subset step is three launches over the (slice, tile) work
+ * units of all slices, and the whole subset/iteration loop is one CUDA graph,
  * captured on the first xct_batch_run and replayed after.  d_sino[i] / d_img[i] are slice
  * i's device sinogram [pa_i][px_i] and image [ny_i][nx_i] (initial in, result out); they may
  * change from run to run.  Runs of one plan must not overlap (they share its buffers).
@@ -135,7 +135,7 @@ int xct_osem_run_volume(xct_plan *plan, int n, const float *const *sino_host, fl
  * CT-XAFS stack, the slices of one width at one energy), at least XCT_MULTISLICE_SLICES of
  * them, form a group that runs through a single-shape plan of that geometry, up to 16 slices
  * per xct_osem_run_device call (the slice-interleaved kernels serve such slices faster than
- * the persistent launches): in place when a call's slices are consecutive in one pair of
+ * the graph's launches): in place when a call's slices are consecutive in one pair of
  * arrays ([k][pa][px], [k][ny][nx]), else copied into a contiguous scratch pair of the plan
  * and the images copied back.  The graph serves the other slices, two to seven of one geometry
  * in packs of four and of two (where the modelled time of the whole graph is lower so) and the
@@ -434,23 +434,21 @@ int xct_batch_plan_tuning(xct_batch_plan *plan, int *fwd_tile, int *ang_chunk);
  *    a CTA stages a tile of all slices of a group, and a sample's coordinates, addresses and
  *    weights are found once for all of them.  Results agree with the per-slice kernel to float
  *    rounding of the partial ray sums;
- *  - backprojection + update (OSEM2) in groups of eight, and a pair left over in a two-slice
- *    form: one bin expression per eight (two) gathers; bit-identical to the per-slice kernel;
- *    the FBP backprojection (xct_fbp_backproject, the FBP and hybrid runs) the same way, also
- *    bit-identical;
- *  - the exact adjoint (xct_adj and the FISTA adjoint step) in groups of ten or eight as a
+ *  - backprojection + update (OSEM2) in groups of eight, four and two, where their grid fills the
+ *    GPU: one bin expression for all gathers of a group; bit-identical to the per-slice kernel;
+ *    the FBP backprojection (xct_fbp_backproject, the FBP and hybrid runs) in groups of eight and
+ *    two, also bit-identical;
+ *  - the exact adjoint (xct_adj and the FISTA adjoint step) in groups of ten, eight or four as a
  *    gather: a thread owns one base texel, finds the samples whose base texel it is with the
  *    forward projector's own arithmetic and sums their weighted ray values in registers (no
- *    atomics; float sums in an order fixed by the geometry, so repeatable bit for bit); a
- *    group of four left over in scatter form, each sample's coordinates and weights serving
- *    the four slices.  Both agree with the per-slice kernel to float rounding (the scatter
- *    form exactly where its fixed-point path applies).
- * With it on, a call's slices go in groups through these kernels and the rest through the
- * per-slice ones, and a call that runs as two halves cuts them at a multiple of eight.  The
- * value is the most subset angles a forward CTA serves from one staging of a tile (1..128); 0
- * turns all three off.  Plans start on (128) when max_batch >= 8 and the forward tiles of one group give at
- * least two CTAs per SM, else off (the tile cache and the autotuner leave this switch
- * alone).
+ *    atomics; float sums in an order fixed by the geometry, so repeatable bit for bit); pairs
+ *    and single slices, and any number of small ones, in scatter form (fixed-point sums).  The
+ *    forms agree to float rounding.
+ * Grouping is on in every plan; this switch admits the backprojectors' groups of eight, and a call
+ * that runs as two halves then cuts them at a multiple of eight.  The value is the most subset
+ * angles a forward CTA serves from one staging of a tile (1..128); set to 0 it turns every grouping
+ * off.  Plans start on (128) when max_batch >= 8 and eight slices have at least two squares of 42
+ * pixels for every SM, else off (the tile cache and the autotuner leave this switch alone).
  *
  * A plan that starts with it off still groups up to five slices and, small problems, takes the kernels
  * made for them; a value set by hand holds whatever the size.  xct_plan_reset_tuning takes back what

@@ -3,7 +3,7 @@ angles and the plan's cap on angles a pass; a plan that has served many such cal
 each the ray sums of a plan that serves nothing else (the same samples and partial sums, whose double sums
 meet in any order: 1e-6 rel-L2).  And finding the division is no part of a repeated call: a default plan's
 forward call costs the host at most 1.3 times one with its tile set by hand, which has nothing to find (both
-are two launches; measured 1.2, and 1.7 when every call divided anew)."""
+are two launches; measured 1.0, and 1.7 when every call divided anew)."""
 import time
 
 import numpy as np
