@@ -672,13 +672,13 @@ __global__ void __launch_bounds__(kBpMsThreads) bp_ms_kernel(float *img, const f
 // way, or on smaller ones through persistent CTAs that take (slice, tile) units from a device queue (an atomic counter) until the units run
 // out.  The single slices' backprojection has one CTA per unit too: what a few of them beside packs take is the
 // time of one CTA over all angles, and on tiles of 64 x 64 that made packs slower than no packs (two
-// geometries of three slices 300 and 320 wide, 240 and 270 angles: 663 us an iteration against 591; on 32 x 32 tiles
-// 363 against 369).  Units of pack (slice) i are [base[i], base[i+1]); they are independent within a launch, so
+// geometries of three slices 300 and 320 wide, 240 and 270 angles: 663 us an iteration against 591; now 291
+// against 334).  Units of pack (slice) i are [base[i], base[i+1]); they are independent within a launch, so
 // there is no waiting on other CTAs.
 // A pack pays per slice what the forward and backward kernels of several slices save (coordinates,
 // addresses and weights once), and takes the large tiles, one CTA per SM: one iteration of 24 slices, 12
-// geometries 512 to 2048 wide, takes 27.8 ms in packs of two and 39.1 one by one; 21 of seven geometries 570 to
-// 1140 wide, in packs of two and single slices, 8.05 ms and 9.65; 6 of three, 200 to 400 wide, 0.33 and 0.44.
+// geometries 512 to 2048 wide, takes 27.7 ms in packs of two and 39.0 one by one; 21 of seven geometries 570 to
+// 1140 wide, in packs of two and single slices, 8.02 ms and 9.61; 6 of three, 200 to 400 wide, 0.32 and 0.37.
 __device__ __forceinline__ int queue_take(int *queue, int *s_unit)
 {
     if (threadIdx.x == 0) *s_unit = atomicAdd(queue, 1);

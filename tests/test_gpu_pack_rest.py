@@ -2,7 +2,7 @@
 two packs of two and two single slices.  A leftover slice's kernels run beside the packs', so a third
 slice may not cost a launch the time of one CTA over a large tile and all angles: an iteration of two
 geometries of three stays below 2.3 times that of the same geometries with two (half again the work, and one
-more forward and backprojection kernel side by side with the packs'; measured 1.8 and 1.5, and 3.2 and 2.9
+more forward and backprojection kernel side by side with the packs'; measured 1.4 and 1.3, and 3.2 and 2.9
 with single slices backprojected on tiles of 64 x 64).  And each slice's image is the one it gets alone, to
 the batch plan's bar, 1e-6 rel-L2."""
 import numpy as np
